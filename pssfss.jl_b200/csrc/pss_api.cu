@@ -137,6 +137,7 @@ struct Worker {
   cudaStream_t st = nullptr;
   int cap = 1;  // batch capacity (points)
   DevBuf zb, z64, zr, zi, ipiv, info, bstat, bf, rhs, X, R, D, nonconv, luws, solvews;
+  DevBuf jkws;  // lattice-sum tables of the face integrals
   JKBufs jk, jkx[kJKGroup - 1];  // face integrals of the points whose phasing varies: slots 0..kJKGroup
   SolveWS sws;
   JKDev jk_slot(int q) const { return q == 0 ? jk.jk : jkx[q - 1].jk; }
@@ -403,13 +404,20 @@ bool jk_key_stale(const pss_sheet *sh, double psi1, double psi2, double ulocal) 
          std::fabs((ulocal - sh->jk_u) / sh->jk_u) > 1e-4;
 }
 
-int refresh_jk_cache(pss_sheet *sh, double psi1, double psi2, double ulocal, cudaStream_t st) {
+// Runs on the given worker's stream with its table scratch.
+int refresh_jk_cache(pss_sheet *sh, double psi1, double psi2, double ulocal, Worker &w) {
   if (!jk_key_stale(sh, psi1, psi2, ulocal)) return 0;
+  cudaStream_t st = w.st;
   if (sh->cache.ensure(sh->nufp)) return -3;
+  if (w.jkws.ensure(pss_jktab_bytes(sh->G, ulocal, sh->s1, sh->s2, 1))) return -3;
   DevBuf nc;
   if (nc.ensure(sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemsetAsync(nc.p, 0, sizeof(int), st));
-  pss_filljk(sh->G, ulocal, psi1, psi2, sh->s1, sh->s2, sh->cache.jk, nc.as<int>(), st);
+  if (int rc = pss_filljk(sh->G, ulocal, psi1, psi2, sh->s1, sh->s2, sh->cache.jk, nc.as<int>(), w.jkws.p, w.jkws.n,
+                          st)) {
+    nc.release();
+    return rc;
+  }
   int h = 0;
   PSS_CUDA_TRY(cudaMemcpyAsync(&h, nc.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   PSS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -490,7 +498,7 @@ int pss_ctx_destroy(pss_ctx *c) {
   cudaDeviceSynchronize();
   for (auto &w : c->w) {
     for (DevBuf *b : {&w.zb, &w.z64, &w.zr, &w.zi, &w.ipiv, &w.info, &w.bstat, &w.bf, &w.rhs, &w.X, &w.R, &w.D, &w.nonconv,
-                      &w.luws, &w.solvews})
+                      &w.luws, &w.solvews, &w.jkws})
       b->release();
     w.jk.buf.release();
     for (auto &x : w.jkx) x.buf.release();
@@ -586,6 +594,14 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     hls[3 * f + 2] = std::sqrt(a12x * a12x + a12y * a12y);
     ha48[f] = 48 * std::fabs(0.5 * (a32x * a12y - a32y * a12x));
   }
+  // extents of the vertices in lattice coordinates (the range of every face pair's offset)
+  double lo[2] = {1e300, 1e300}, hi[2] = {-1e300, -1e300};
+  const double cell = s1[0] * s2[1] - s1[1] * s2[0];
+  for (int64_t v = 0; v < nnode; ++v) {
+    const double x = rho[2 * v], y = rho[2 * v + 1];
+    const double a[2] = {(x * s2[1] - y * s2[0]) / cell, (y * s1[0] - x * s1[1]) / cell};
+    for (int d = 0; d < 2; ++d) { lo[d] = std::min(lo[d], a[d]); hi[d] = std::max(hi[d], a[d]); }
+  }
   std::vector<double> hfr(fr, fr + nface);
   int rc = 0;
   rc |= upload(sh->rho, rho, 2 * (size_t)nnode);
@@ -607,6 +623,7 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   G.fr = sh->fr.as<double>(); G.face_ls = sh->ls.as<double>(); G.face_a48 = sh->a48.as<double>();
   G.inc_cnt = sh->inc_cnt.as<int>(); G.inc_face = sh->inc_face.as<int>(); G.inc_loc = sh->inc_loc.as<int>();
   G.inc_sgn = sh->inc_sgn.as<int>(); G.inc_eci = sh->inc_eci.as<int>();
+  G.ext1 = hi[0] - lo[0]; G.ext2 = hi[1] - lo[1];
   *out = sh;
   return 0;
 }
@@ -783,7 +800,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
           PR[p].own_jk = true;
     for (auto &P : PR) {
       if (P.own_jk) continue;
-      if (int rc = refresh_jk_cache(P.sh, P.psi[0], P.psi[1], P.u / P.sh->upm, c->w[0].st)) return rc;
+      if (int rc = refresh_jk_cache(P.sh, P.psi[0], P.psi[1], P.u / P.sh->upm, c->w[0])) return rc;
       if (P.sh->jk_nonconv)
         for (int i = 0; i < P.npts; ++i) hstatus[P.p0 + i] |= PSS_ST_JK_NOCONV;
     }
@@ -843,6 +860,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
   {
     int mufp = 0, mn = 0, mnm = 0, mB = 1;
     bool ojk = false;
+    size_t mtab = 0;  // lattice-sum tables of the sheets whose phasing varies
     for (auto &it : items) {
       for (int b = 0; b < it.cnt; ++b) {
         const Problem &P = PR[it.p[b]];
@@ -854,9 +872,12 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
     for (auto &P : PR) {  // the perturbed sets' pair terms go through the same buffers
       mufp = std::max(mufp, P.sh->nufp);
       ojk = ojk || P.own_jk;
+      if (P.own_jk) mtab = std::max(mtab, pss_jktab_bytes(P.sh->G, P.u / P.sh->upm, P.sh->s1, P.sh->s2, kJKGroup));
     }
-    for (int k = 0; k < nwk; ++k)
+    for (int k = 0; k < nwk; ++k) {
       if (int rc = ensure_worker_dims(c->w[k], mufp, mn, mnm, precision, ojk, mB)) return rc;
+      if (c->w[k].jkws.ensure(mtab)) return -3;
+    }
   }
   // adjoint-stage buffers of every worker: PT, Lam, scratch W (a batch each), R_k and the
   // set's transforms (one point each), the contraction's CTA shares, refinement scratch
@@ -918,7 +939,9 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
           p2[q] = Q.psi[2 * it.i[b + q] + 1];
           jks[q] = w.jk_slot(q);
         }
-        pss_filljk_group(sh->G, P.u / sh->upm, gsz, p1, p2, sh->s1, sh->s2, jks, w.nonconv.as<int>(), st);
+        if (int rc = pss_filljk_group(sh->G, P.u / sh->upm, gsz, p1, p2, sh->s1, sh->s2, jks, w.nonconv.as<int>(),
+                                      w.jkws.p, w.jkws.n, st))
+          return rc;
         for (int q = 0; q < gsz; ++q) {
           pss_count_launch();
           k_nonconv_to_status<<<1, 1, 0, st>>>(w.nonconv.as<int>() + q, dstatus + PR[it.p[b + q]].p0 + it.i[b + q]);
@@ -977,8 +1000,9 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
             jq = Q.sh->cache.jk;
           } else {
             jq = w.jk.jk;
-            pss_filljk(Q.sh->G, Q.u / Q.sh->upm, Q.psi[2 * i], Q.psi[2 * i + 1], Q.sh->s1, Q.sh->s2, jq,
-                       w.nonconv.as<int>(), st);
+            if (int rc = pss_filljk(Q.sh->G, Q.u / Q.sh->upm, Q.psi[2 * i], Q.psi[2 * i + 1], Q.sh->s1, Q.sh->s2, jq,
+                                    w.nonconv.as<int>(), w.jkws.p, w.jkws.n, st))
+              return rc;
             pss_count_launch();
             k_nonconv_to_status<<<1, 1, 0, st>>>(w.nonconv.as<int>(), dstatus + PR[0].p0 + i);
           }
@@ -1184,7 +1208,7 @@ int pss_fill_matrix(pss_sheet *sh, int nl, const double *eps, const double *mu, 
   int rc = build_tables(c, S, c->params.as<PointParams>(), 1, 1e-7, tabs, hs);
   if (rc) return rc;
   Worker &w = c->w[0];
-  if ((rc = refresh_jk_cache(sh, psi1, psi2, u / sh->upm, w.st))) return rc;
+  if ((rc = refresh_jk_cache(sh, psi1, psi2, u / sh->upm, w))) return rc;
   if ((rc = ensure_worker(w, sh, 1, PSS_FP64, false, 1))) return rc;
   pss_fill_pairs(sh->G, c->params.as<PointParams>(), sh->cache.jk, tabs[0].t1, tabs[0].t2, tabs[0].mmax,
                  w.zb.as<cd>(), w.st);
@@ -1232,7 +1256,7 @@ int pss_face_integrals(pss_sheet *sh, double ulocal, double psi1, double psi2, d
   if (!sh) { pss_set_error("null argument"); return -1; }
   if (set_device(sh->ctx)) return -3;
   sh->jk_valid = false;
-  int rc = refresh_jk_cache(sh, psi1, psi2, ulocal, sh->ctx->w[0].st);
+  int rc = refresh_jk_cache(sh, psi1, psi2, ulocal, sh->ctx->w[0]);
   if (rc) return rc;
   const size_t c = (size_t)sh->nufp * sizeof(cd), d = (size_t)sh->nufp * sizeof(double);
   const JKDev &jk = sh->cache.jk;
@@ -1557,7 +1581,7 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
     if ((rc = point_tables(c, S, dP, tb0, t0, hst))) return rc;
     for (int k = 0; k < K; ++k)
       if ((rc = point_tables(c, Sk[k], dP + 1 + k, tbk[k], tk[k], hst))) return rc;
-    if ((rc = refresh_jk_cache(sh, psi[2 * i], psi[2 * i + 1], u / sh->upm, st))) return rc;
+    if ((rc = refresh_jk_cache(sh, psi[2 * i], psi[2 * i + 1], u / sh->upm, w))) return rc;
     if (sh->jk_nonconv) hst |= PSS_ST_JK_NOCONV;
     // Z into slot 0 (and the FP32 planes), fills and transforms of every set
     pss_fill_pairs(sh->G, dP, sh->cache.jk, t0.t1, t0.t2, t0.mmax, w.zb.as<cd>(), st);
@@ -1569,7 +1593,7 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
     for (int k = 0; k < K; ++k) {
       pss_sheet *q = psh[k];
       const double *pp = ppsi + 2 * ((size_t)k * npts + i);
-      if ((rc = refresh_jk_cache(q, pp[0], pp[1], pu[k] / q->upm, st))) return rc;
+      if ((rc = refresh_jk_cache(q, pp[0], pp[1], pu[k] / q->upm, w))) return rc;
       if (q->jk_nonconv) hst |= PSS_ST_JK_NOCONV;
       pss_fill_pairs(q->G, dP + 1 + k, q->cache.jk, tk[k].t1, tk[k].t2, tk[k].mmax, w.zb.as<cd>(), st);
       pss_fill_assemble(q->G, dP + 1 + k, w.zb.as<cd>(), w.z64.as<cd>() + (1 + k) * msz, nullptr, nullptr, ld, ld,

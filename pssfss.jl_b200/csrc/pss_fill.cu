@@ -3,7 +3,8 @@
 // K2 k_filljk   restates Zint.jl:54-179 (filljk!) with PGF.jl:67-106 (jksums): eight
 //               lanes per unique face pair, one lattice sum (quadrature point) per lane in
 //               the reference's ring order, the seven sums gathered by warp shuffles and
-//               accumulated in the 7-point rule's order, FP64.
+//               accumulated in the 7-point rule's order, FP64; larger sheets take the
+//               tabulated form of the same sums (pss_jktab.cu).
 // K3a k_pairs   restates Zint.jl:218-245 (zint) and the per-edge algebra of
 //               FillZY.jl:141-197 / 362-419: one thread per unique face pair computes
 //               the 3x3 unflagged edge-pair terms  zA*(ρc2[iml]·a_isl) - zP*φ.
@@ -15,250 +16,22 @@
 #include <algorithm>
 
 #include "pss_internal.cuh"
+#include "pss_lattice.cuh"
 
 namespace {
 
-// Phase factors of the lattice terms, cis(-m psi1) and cis(-n psi2) for |m|, |n| <= 65 (the
-// ring budget): kPhase entries each, index m + 65.  A term's factor cis(-(m psi1 + n psi2)) is
-// their product, one complex multiply in place of a sincos per summand.
-constexpr int kPhase = 2 * PSS_JKRINGMAX + 1;
-
-// exp(-a), a >= 0, by Tang's table-driven method (P. T. P. Tang, "Table-driven implementation
-// of the exponential function in IEEE floating-point arithmetic", ACM Trans. Math. Softw. 15
-// (1989) 144-157): -a = (256 m + j) ln2/256 + r with |r| <= ln2/512 (k = 256 m + j the nearest
-// integer to -a 256/ln2, found by adding 1.5 * 2^52; ln2/256 in two parts, so r keeps its full
-// precision), exp(-a) = 2^m * 2^(j/256) * p(r) with p the degree-5 Taylor polynomial of e^r
-// (remainder below r^6/720 < 1e-20 relative) and 2^(j/256) from a 256-entry table; 2^m enters
-// through the exponent field.  About ten FP64 operations.  a >= 708 gives 0: such summands are
-// far below the lattice sums' 1e-8 convergence test.
-constexpr double kExpShift = 6755399441055744.0;  // 1.5 * 2^52
-constexpr double kExpInvStep = 0x1.71547652b82fep+8;  // 256 / ln2
-constexpr double kExpStepHi = 0x1.62e42fefa39efp-9;   // ln2 / 256, nearest double
-constexpr double kExpStepLo = 0x1.abc9e3b39803fp-64;  // ln2 / 256 - kExpStepHi
-__device__ __forceinline__ double exp_neg(double a, const double *__restrict__ tab) {
-  if (!(a < 708.0)) return 0.0;
-  const double sh = fma(-a, kExpInvStep, kExpShift);
-  const int k = __double2loint(sh);  // nearest integer to -a 256/ln2, two's complement
-  const double kf = sh - kExpShift;
-  const double r = fma(kf, -kExpStepLo, fma(kf, -kExpStepHi, -a));
-  double p = fma(r, 1.0 / 120, 1.0 / 24);
-  p = fma(p, r, 1.0 / 6);
-  p = fma(p, r, 0.5);
-  p = fma(p, r, 1.0);
-  p = fma(p, r, 1.0);
-  const double t = tab[k & 255] * p;
-  return __hiloint2double(__double2hiint(t) + ((k >> 8) << 20), __double2loint(t));
-}
-
-// jksums (PGF.jl:67-106): the spatial lattice sums J and K at one observation offset, ring by
-// ring in the reference's order (rmin = 5, at most 65 rings, relative change 1e-8), for NP
-// phasings at once.  A summand's distance, exp(-u r) and 1/r do not depend on the phasing, so
-// they are evaluated once and weighted by each phasing's factor; every phasing keeps its own
-// ring partials and stops accumulating at its own convergence ring, so its sums are those of
-// a serial evaluation at that phasing alone, bit for bit.  Slots p >= np are idle.  Returns the
-// mask of converged phasings.
-template <int NP>
-__device__ __forceinline__ unsigned jksums_group(double urx, double ury, int np, bool nophase, double us1x,
-                                                 double us1y, double us2x, double us2y,
-                                                 const cd (*__restrict__ ph1)[kPhase],
-                                                 const cd (*__restrict__ ph2)[kPhase], const double *__restrict__ etab,
-                                                 cd *jout, cd *kout) {
-  const int rmin = 5;
-  const double small = 1e-5, convtest = 1e-8;
-  double arg = sqrt(urx * urx + ury * ury);
-  double rterm = exp_neg(arg, etab);
-  const cd k0 = mkcd(rterm, 0.0);
-  const cd j0 = arg <= small ? mkcd((-arg / 6 + 0.5) * arg - 1, 0.0) : mkcd((rterm - 1) / arg, 0.0);
-  cd jsum[NP], ksum[NP];
-#pragma unroll
-  for (int p = 0; p < NP; ++p) { jsum[p] = j0; ksum[p] = k0; }
-  unsigned live = (1u << np) - 1u, conv = 0;
-  for (int r = 1; r <= PSS_JKRINGMAX && live; ++r) {
-    cd jring[NP], kring[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) { jring[p] = mkcd(0, 0); kring[p] = mkcd(0, 0); }
-    auto summand = [&](int m, int n, double dm, double dn) {
-      double dx = urx - (dm * us1x + dn * us2x);
-      double dy = ury - (dm * us1y + dn * us2y);
-      // one reciprocal square root gives both the distance and the 1/r weight (two FP64
-      // divisions fewer per summand than sqrt then term / r)
-      const double d2 = dx * dx + dy * dy;
-      const double ra = rsqrt(d2);
-      const double a = d2 * ra;
-      double er = exp_neg(a, etab);
-      if (NP == 1 && nophase) {  // real terms: the imaginary parts stay exactly zero
-        jring[0].x = jring[0].x + er * ra;
-        kring[0].x = kring[0].x + er;
-      } else {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const cd f = ph1[p][m + PSS_JKRINGMAX] * ph2[p][n + PSS_JKRINGMAX];
-          const cd term = mkcd(er * f.x, er * f.y);
-          jring[p] = jring[p] + mkcd(term.x * ra, term.y * ra);
-          kring[p] = kring[p] + term;
-        }
-      }
-    };
-    // the ring's 8r lattice points in Ring's order (ring_mn): m = r with n = -r..r, m = -r with
-    // n = -r..r, then n = -r and n = r with m = -r+1..r-1; the indices are also counted in
-    // FP64 (exact integers), so no summand converts one
-    {
-      const double dr = (double)r;
-      double dn = -dr;
-      for (int i = -r; i <= r; ++i, dn += 1.0) summand(r, i, dr, dn);
-      dn = -dr;
-      for (int i = -r; i <= r; ++i, dn += 1.0) summand(-r, i, -dr, dn);
-      double dm = 1.0 - dr;
-      for (int i = 1 - r; i < r; ++i, dm += 1.0) summand(i, -r, dm, -dr);
-      dm = 1.0 - dr;
-      for (int i = 1 - r; i < r; ++i, dm += 1.0) summand(i, r, dm, dr);
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      if (!((live >> p) & 1u)) continue;
-      jsum[p] = jsum[p] + jring[p];
-      ksum[p] = ksum[p] + kring[p];
-      if (r > rmin) {
-        double c1 = cabsd(jring[p] / jsum[p]), c2 = cabsd(kring[p] / ksum[p]);
-        if (fmax(c1, c2) < convtest) { live &= ~(1u << p); conv |= 1u << p; }
-      }
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < NP; ++p) { jout[p] = jsum[p]; kout[p] = ksum[p]; }
-  return conv;
-}
-
-__device__ __forceinline__ void face_vtx(const SheetDev &G, int f, double r[3][2], double scale) {
-  for (int k = 0; k < 3; ++k) {
-    int v = G.fv[3 * f + k];
-    r[k][0] = G.rho[2 * v] * scale;
-    r[k][1] = G.rho[2 * v + 1] * scale;
-  }
-}
-
-// Eight lanes per unique face pair (four pairs per warp): lane q < 7 computes the lattice
-// sums of quadrature point q (jksums, serial in the reference's ring order) for the group's
-// np <= NP phasings; the pair's first lane gathers the seven results with warp shuffles and
-// accumulates them in the 7-point rule's order, so each pair's integrals are those of a
-// serial evaluation bit for bit.  The phasing-free parts (the smooth-term geometry, rho_r and
-// the 1/R integral) are computed once and written to every phasing's slot.
-template <int NP>
-constexpr int jk_threads() { return NP == 1 ? 256 : 128; }
-
+// Direct form: one launch over every face pair of a sheet (pss_jktab.cu holds the tabulated
+// form that larger sheets take, and the rule between the two).
 template <int NP>
 __global__ void __launch_bounds__(jk_threads<NP>(), 3) k_filljk(SheetDev G, double ul, PsiGroup pg, double us1x, double us1y,
                                                 double us2x, double us2y, JKGroup jk, int *nonconv) {
   __shared__ cd ph1[NP][kPhase], ph2[NP][kPhase];
   __shared__ double etab[256];  // 2^(j/256) for exp_neg
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) etab[t] = exp2((double)t / 256.0);
   const int np = NP == 1 ? 1 : pg.n;
-  for (int t = threadIdx.x; t < NP * kPhase; t += blockDim.x) {
-    const int p = t / kPhase;
-    const double k = (double)(t % kPhase - PSS_JKRINGMAX);
-    const double a1 = p < np ? pg.psi1[p] : 0.0, a2 = p < np ? pg.psi2[p] : 0.0;
-    double s1, c1, s2, c2;
-    sincos(-(k * a1), &s1, &c1);
-    sincos(-(k * a2), &s2, &c2);
-    ph1[p][t % kPhase] = mkcd(c1, s1);
-    ph2[p][t % kPhase] = mkcd(c2, s2);
-  }
+  fill_phases<NP>(pg, np, ph1, ph2, etab);
   __syncthreads();
-  const bool nophase = NP == 1 && pg.psi1[0] == 0.0 && pg.psi2[0] == 0.0;
-  const int lane = threadIdx.x & 31, q = lane & 7, grp = lane & ~7;
   const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;  // pair of this group
-  const bool live = gid < G.nufp;
-  const int iu = live ? (int)gid : G.nufp - 1;  // idle groups mirror the last pair, write nothing
-  const int fp = G.ufp_rep[iu];
-  const int ifm = fp % G.nface, ifs = fp / G.nface;
-  double rs[3][2], rm[3][2];
-  face_vtx(G, ifs, rs, 1.0);
-  face_vtx(G, ifm, rm, 1.0);
-  double rs32[2] = {rs[2][0] - rs[1][0], rs[2][1] - rs[1][1]};
-  double rs12[2] = {rs[0][0] - rs[1][0], rs[0][1] - rs[1][1]};
-  double area2 = (-rs32[1]) * rs12[0] + rs32[0] * rs12[1];
-  double unz = 1.0;
-  if (area2 < 0) { area2 = fabs(area2); unz = -1.0; }
-  double rs31[2] = {rs[2][0] - rs[0][0], rs[2][1] - rs[0][1]};
-  double rs21[2] = {-rs12[0], -rs12[1]};
-  double rmc[2] = {((rm[0][0] + rm[1][0]) + rm[2][0]) / 3, ((rm[0][1] + rm[1][1]) + rm[2][1]) / 3};
-  cd js[NP], ks[NP];
-#pragma unroll
-  for (int p = 0; p < NP; ++p) { js[p] = mkcd(0, 0); ks[p] = mkcd(0, 0); }
-  unsigned ok = (1u << np) - 1u;
-  if (q < 7) {
-    double rtx = (rs[0][0] + rs21[0] * c_qxi[q]) + rs31[0] * c_qeta[q];
-    double rty = (rs[0][1] + rs21[1] * c_qxi[q]) + rs31[1] * c_qeta[q];
-    ok = jksums_group<NP>(ul * (rmc[0] - rtx), ul * (rmc[1] - rty), np, nophase, us1x, us1y, us2x, us2y, ph1, ph2,
-                          etab, js, ks);
-  }
-  // phasing-free terms (the pair's first lane only)
-  double rr0 = 0, rr1 = 0, ri = 0;
-  if (q == 0) {
-    const int nxt[3] = {1, 2, 0};
-    for (int i = 0; i < 3; ++i) {
-      int ip1 = nxt[i];
-      double lx = rs[ip1][0] - rs[i][0], ly = rs[ip1][1] - rs[i][1];
-      double ln = sqrt(lx * lx + ly * ly);
-      lx /= ln;
-      ly /= ln;
-      double ux = (-unz) * (-ly), uy = (-unz) * lx;
-      double d0x = rs[i][0] - rmc[0], d0y = rs[i][1] - rmc[1];
-      double d1x = rs[ip1][0] - rmc[0], d1y = rs[ip1][1] - rmc[1];
-      double p0 = ux * d0x + uy * d0y;
-      double p0sq = p0 * p0;
-      double lp = lx * d1x + ly * d1y;
-      double lm = lx * d0x + ly * d0y;
-      double ledge = lp - lm;
-      double pplus = sqrt(p0sq + lp * lp);
-      double pminus = sqrt(p0sq + lm * lm);
-      double factor;
-      if (fabs(p0 / ledge) < 1e-4) {
-        factor = lp * pplus - lm * pminus;
-      } else {
-        factor = p0 * log((pplus + lp) / (pminus + lm));
-        ri += factor;
-        factor = (factor * p0 + pplus * lp) - pminus * lm;
-      }
-      rr0 += ux * factor;
-      rr1 += uy * factor;
-    }
-    rr0 *= 0.5;
-    rr1 *= 0.5;
-    rr0 /= area2;
-    rr1 /= area2;
-    ri /= (area2 * ul);
-  }
-#pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    cd aJ = mkcd(0, 0), aJx = aJ, aJe = aJ, aK = aJ, aKx = aJ, aKe = aJ;
-    int bad = 0;
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {  // every lane takes part in the shuffles; the group's lane 0 keeps the sums
-      cd jv, kv;
-      jv.x = __shfl_sync(0xffffffffu, js[p].x, grp + i);
-      jv.y = __shfl_sync(0xffffffffu, js[p].y, grp + i);
-      kv.x = __shfl_sync(0xffffffffu, ks[p].x, grp + i);
-      kv.y = __shfl_sync(0xffffffffu, ks[p].y, grp + i);
-      bad |= !((__shfl_sync(0xffffffffu, ok, grp + i) >> p) & 1u);
-      cd jw = c_qw[i] * jv;
-      aJx = aJx + c_qxi[i] * jw;
-      aJe = aJe + c_qeta[i] * jw;
-      aJ = aJ + jw;
-      cd kw = c_qw[i] * kv;
-      aKx = aKx + c_qxi[i] * kw;
-      aKe = aKe + c_qeta[i] * kw;
-      aK = aK + kw;
-    }
-    if (q != 0 || !live || p >= np) continue;
-    const JKDev &o = jk.s[p];
-    o.J[iu] = aJ; o.Jxi[iu] = aJx; o.Jeta[iu] = aJe;
-    o.K[iu] = aK; o.Kxi[iu] = aKx; o.Keta[iu] = aKe;
-    o.rho_r[2 * iu] = rr0;
-    o.rho_r[2 * iu + 1] = rr1;
-    o.rinv[iu] = ri;
-    if (bad) atomicAdd(nonconv + p, 1);
-  }
+  filljk_pair<NP>(G, ul, pg, np, us1x, us1y, us2x, us2y, jk, nonconv, gid, gid < G.nufp, ph1, ph2, etab);
 }
 
 // Per-point coefficients that turn the face-pair integrals into Z terms:
@@ -528,9 +301,10 @@ void pss_adj_contract(const SheetDev &G, const PointParams *dP1, const cd *zb, c
   k_adj_reduce<<<nm * nm, 256, 0, st>>>(nblk * kAdjChunks, nm * nm, part, Gout);
 }
 
-void pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi1, const double *psi2,
-                      const double s1[2], const double s2[2], const JKDev *jk, int *nonconv, cudaStream_t st) {
-  if (G.nufp == 0 || np <= 0) return;
+int pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi1, const double *psi2,
+                     const double s1[2], const double s2[2], const JKDev *jk, int *nonconv, void *ws, size_t ws_bytes,
+                     cudaStream_t st) {
+  if (G.nufp == 0 || np <= 0) return 0;
   PsiGroup pg{};
   JKGroup jg{};
   pg.n = std::min(np, kJKGroup);
@@ -540,6 +314,9 @@ void pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *ps
     jg.s[p] = jk[p];
   }
   const double a = ulocal * s1[0], b = ulocal * s1[1], c = ulocal * s2[0], d = ulocal * s2[1];
+  JKTabPlan plan;
+  if (pss_jktab_plan(G, ulocal, s1, s2, pg.n, plan) && ws && ws_bytes >= plan.bytes)
+    return pss_jktab_launch(G, ulocal, pg, s1, s2, jg, nonconv, plan, ws, st);
   const long long lanes = (long long)G.nufp * 8;
   pss_count_launch();
   if (pg.n == 1)
@@ -549,11 +326,13 @@ void pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *ps
   else
     k_filljk<kJKGroup><<<cdiv_u(lanes, jk_threads<kJKGroup>()), jk_threads<kJKGroup>(), 0, st>>>(G, ulocal, pg, a, b,
                                                                                              c, d, jg, nonconv);
+  PSS_CUDA_TRY(cudaGetLastError());
+  return 0;
 }
 
-void pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const double s1[2], const double s2[2],
-                JKDev jk, int *nonconv, cudaStream_t st) {
-  pss_filljk_group(G, ulocal, 1, &psi1, &psi2, s1, s2, &jk, nonconv, st);
+int pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const double s1[2], const double s2[2],
+               JKDev jk, int *nonconv, void *ws, size_t ws_bytes, cudaStream_t st) {
+  return pss_filljk_group(G, ulocal, 1, &psi1, &psi2, s1, s2, &jk, nonconv, ws, ws_bytes, st);
 }
 
 void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const cd *t1, const cd *t2,

@@ -66,6 +66,7 @@ struct SheetDev {
   const int *inc_loc;    // 4*nbf local edge slot 0..2
   const int *inc_sgn;    // 4*nbf +1 plus / -1 minus
   const int *inc_eci;    // 4*nbf edge boundary code 0..4
+  double ext1, ext2;     // extents of the vertices in lattice coordinates (along s1 and s2)
 };
 
 // J/K cache (Zint.jl:54-179), SoA over unique face pairs.
@@ -147,11 +148,24 @@ int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, 
 size_t pss_table_cap(int mmax);  // (mmax+2)^2 entries per padded table
 
 // Face-pair integrals and matrix fill (pss_fill.cu)
-void pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const double s1[2],
-                const double s2[2], JKDev jk, int *nonconv, cudaStream_t st);
+// ws: scratch of pss_jktab_bytes (may be null: every pair's lattice sums then run ring by ring).
+int pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const double s1[2], const double s2[2],
+               JKDev jk, int *nonconv, void *ws, size_t ws_bytes, cudaStream_t st);
 // np <= kJKGroup phasings at once into jk[0..np), non-convergence counts into nonconv[0..np)
-void pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi1, const double *psi2,
-                      const double s1[2], const double s2[2], const JKDev *jk, int *nonconv, cudaStream_t st);
+int pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi1, const double *psi2,
+                     const double s1[2], const double s2[2], const JKDev *jk, int *nonconv, void *ws,
+                     size_t ws_bytes, cudaStream_t st);
+// Tabulated lattice sums (pss_jktab.cu): the panels that cover a sheet's offsets, and the bytes
+// of the tables, maps and the list of pairs left to the direct form for np phasings.
+struct JKTabPlan {
+  int na = 0, nb = 0;  // panels along the two lattice vectors
+  double a0 = 0, b0 = 0, ra = 0, rb = 0;  // first panel's corner; panels per unit lattice coordinate
+  size_t bytes = 0;
+};
+bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np, JKTabPlan &P);
+size_t pss_jktab_bytes(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np);
+int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const double s1[2], const double s2[2],
+                     const JKGroup &jk, int *nonconv, const JKTabPlan &P, void *ws, cudaStream_t st);
 void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const cd *t1, const cd *t2,
                     int mmax, cd *zb, cudaStream_t st);
 // Assemble Z (row-major): z64 with leading dimension ld, the FP32 planes (zr, zi) with ldf.

@@ -1,0 +1,546 @@
+// K2, tabulated form of the face-pair integrals for sheets with many pair classes.
+//
+// jksums (PGF.jl:67-106) adds 168 and more lattice summands at every quadrature point of every
+// pair.  Only the images next to the pair vary fast with the offset; the sum over the images of
+// ring 2 and beyond is smooth (its nearest singularity lies a whole cell away from every offset
+// a sheet can have), so it is tabulated once per phasing and interpolated:
+//   * the offsets, a parallelogram of lattice coordinates, are cut into panels of 8 x 8
+//     Chebyshev nodes.  A panel's half-width is at most 1/48 of the distance D to the nearest
+//     tabulated image: the Bernstein ellipse through that image has radius 96 in both
+//     directions, so the interpolation error is about 96^-8 = 1.4e-16 of the far sum, which is
+//     itself at most a few tenths of the whole;
+//   * the reference stops a sum at its own ring R (relative change below 1e-8), so R is part of
+//     the result.  R depends on the offset alone: a panel stores the far sum through ring R0
+//     and through R0 + 1.  Panels whose nodes all stop at R0, clear of the threshold, are taken
+//     as a whole; the others carry a map of 32 x 32 sub-cells that says R0, R0 + 1 or unknown.
+//     Near a zero of a sum its relative change, and so R, is large: where the values at the
+//     nodes (corners) are not larger than their differences, the panel needs a map (the
+//     sub-cell is unknown);
+//   * pairs with a point in an unknown sub-cell (about 0.3-0.5 % of the points) go to a list
+//     and through the direct form (filljk_pair), bit for bit as before.
+// What bounds it: the direct form issues about 4200 FP64 operations per quadrature point and is
+// bound by the FP64 pipe; this one issues about 400 and reads 64 nodes from L1/L2.  A pair's
+// eight lanes own one column of the panel each, so a node row is one 128-byte line, and a lane
+// keeps its column in registers while consecutive quadrature points stay in the panel.
+// Measured (direct -> tabulated, tables included): 17.6 -> 4.7 ms for the 3.19M classes of the
+// N = 3976 meander at normal incidence, 18.1 -> 6.3 ms for four phasings of a ring of 1168 faces.
+#include <algorithm>
+#include <cmath>
+
+#include "pss_lattice.cuh"
+
+namespace {
+
+constexpr int kND = 8;                  // nodes per panel and direction
+constexpr int kSub = 32;                // sub-cells per panel and direction
+constexpr int kRec = 8;                 // rings 6 .. 6+kRec-1 a panel may stop at
+constexpr int kRMin = 6;                // first ring the reference tests
+constexpr double kConv = 1e-8;          // its threshold
+// How far a node (sub-cell corner) must be from the threshold |ring| = kConv |sum| to speak for
+// its surroundings: a share of |sum| for the slope, and an absolute part for the curvature of the
+// sums, of order 1 in u-scaled lengths (a panel is at most 0.16 wide, a sub-cell 0.005).
+constexpr double kMargin = 0.1, kCurve = 3e-3;
+constexpr double kSubMargin = 1e-4, kSubCurve = 4e-6;
+constexpr int kMaxPanels = 8192;
+constexpr int kMapSmem = 2 * (kSub + 1) * (kSub + 1) * (int)sizeof(cd);  // corner sums of a map's panel
+
+struct TabDev {
+  double iv[4];           // u-scaled offset -> lattice coordinates
+  double a0, b0, ra, rb;
+  int na, nb;
+  double *val[kJKGroup];          // [panel][R0 / R0+1][node a][J, K][node b] (real: one double each)
+  unsigned char *flag[kJKGroup];  // per panel: 0 whole, 1 map, 2 direct
+  unsigned char *r0[kJKGroup];
+  unsigned char *map[kJKGroup];   // [panel][kSub][kSub]
+  int *list, *count;              // pairs left to the direct form, per phasing
+};
+
+// cos((2k+1) pi / 16) and the reciprocals of prod_{m != k} (x_k - x_m)
+__constant__ double c_node[kND] = {0.9807852804032304, 0.8314696123025452, 0.5555702330196023, 0.19509032201612833,
+                                   -0.1950903220161282, -0.555570233019602, -0.8314696123025453, -0.9807852804032304};
+__constant__ double c_nodew[kND] = {3.121445152258054, -8.889123728313642, 13.30351379684073, -15.692564486451692,
+                                    15.692564486451692, -13.303513796840717, 8.889123728313624, -3.121445152258053};
+
+// Sums at one offset, ring by ring as in jksums; the far part (rings >= 2) through each ring r
+// in 6 .. 13 is handed to rec.  Returns the ring the reference stops at (0: beyond the record),
+// whether the test is clear of its threshold there (at) and one ring before (before), and the
+// sums.
+template <bool REAL, class Rec>
+__device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, double us1y, double us2x, double us2y,
+                                          const cd *__restrict__ ph1, const cd *__restrict__ ph2,
+                                          const double *__restrict__ etab, double margin, double curve, bool &at, bool &before,
+                                          cd &jsum, cd &ksum, Rec &&rec) {
+  const double arg = sqrt(urx * urx + ury * ury);
+  const double rterm = exp_neg(arg, etab);
+  ksum = mkcd(rterm, 0.0);
+  jsum = arg <= 1e-5 ? mkcd((-arg / 6 + 0.5) * arg - 1, 0.0) : mkcd((rterm - 1) / arg, 0.0);
+  cd jfar = mkcd(0, 0), kfar = jfar;
+  int R = 0;
+  at = before = true;
+  for (int r = 1; r < kRMin + kRec; ++r) {
+    cd jr = mkcd(0, 0), kr = jr;
+    for (int idx = 0; idx < 8 * r; ++idx) {
+      int m, n;
+      ring_mn(r, idx, m, n);
+      const double dx = urx - ((double)m * us1x + (double)n * us2x), dy = ury - ((double)m * us1y + (double)n * us2y);
+      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
+      if constexpr (REAL) {
+        jr.x += er * ra;
+        kr.x += er;
+      } else {
+        const cd f = ph1[m + PSS_JKRINGMAX] * ph2[n + PSS_JKRINGMAX];
+        jr = jr + mkcd(er * f.x * ra, er * f.y * ra);
+        kr = kr + mkcd(er * f.x, er * f.y);
+      }
+    }
+    if (r >= 2) { jfar = jfar + jr; kfar = kfar + kr; }
+    if (r >= kRMin) rec(r - kRMin, jfar, kfar);
+    if (R) return R;  // one ring past R has been recorded
+    jsum = jsum + jr;
+    ksum = ksum + kr;
+    if (r >= kRMin) {
+      const double aj = cabsd(jsum), ak = cabsd(ksum);
+      const double tj = kConv * aj - cabsd(jr), tk = kConv * ak - cabsd(kr);
+      const double mj = kConv * (margin * aj + curve), mk = kConv * (margin * ak + curve);
+      if (fmax(cabsd(jr / jsum), cabsd(kr / ksum)) < kConv) {
+        R = r;
+        at = tj > mj && tk > mk;
+      } else {
+        before = tj < -mj || tk < -mk;
+      }
+    }
+  }
+  return 0;  // not below the threshold by the last recorded ring, or R + 1 not recorded
+}
+
+// Whether a sum may vanish near v: v is no larger than its distance from one of the corner values.
+__device__ __forceinline__ bool near_zero(cd v, const cd *corner) {
+  bool z = false;
+  const double a = v.x * v.x + v.y * v.y;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double dx = v.x - corner[k].x, dy = v.y - corner[k].y;
+    z = z || a <= dx * dx + dy * dy;
+  }
+  return z;
+}
+
+// One CTA of 64 threads per panel (x) and phasing (y): node (i, j) = (tid / 8, tid % 8).
+template <bool REAL>
+__global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
+                                                    double us2y) {
+  __shared__ cd ph1[1][kPhase], ph2[1][kPhase];
+  __shared__ double etab[256];
+  __shared__ cd rj[kRec][64], rk[kRec][64], corner[2][4];
+  __shared__ int lo, hi;
+  const int p = blockIdx.y, panel = blockIdx.x, tid = threadIdx.x;
+  PsiGroup one{};
+  one.n = 1;
+  one.psi1[0] = pg.psi1[p];
+  one.psi2[0] = pg.psi2[p];
+  fill_phases<1>(one, 1, ph1, ph2, etab);
+  if (tid == 0) { lo = 1000; hi = 0; }
+  for (int r = 0; r < kRec; ++r) rj[r][tid] = rk[r][tid] = mkcd(0, 0);
+  __syncthreads();
+  const int i = tid >> 3, j = tid & 7, ia = panel % T.na, ib = panel / T.na;
+  const double a = T.a0 + (ia + 0.5 * (1.0 + c_node[i])) / T.ra, b = T.b0 + (ib + 0.5 * (1.0 + c_node[j])) / T.rb;
+  bool at, before;
+  cd js, ks;
+  const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0],
+                                 etab, kMargin, kCurve, at, before, js, ks,
+                                 [&](int r, cd jf, cd kf) { rj[r][tid] = jf; rk[r][tid] = kf; });
+  if (tid == 0 || tid == 7 || tid == 56 || tid == 63) {
+    corner[0][(tid & 1) + (tid >> 5) * 2] = js;
+    corner[1][(tid & 1) + (tid >> 5) * 2] = ks;
+  }
+  // the stopping rings that points near this node may have
+  if (R) atomicMin(&lo, R > kRMin && !before ? R - 1 : R);
+  atomicMax(&hi, R == 0 ? 1000 : !at ? R + 1 : R);
+  __syncthreads();
+  if (near_zero(js, corner[0]) || near_zero(ks, corner[1])) atomicMax(&hi, 1000);
+  __syncthreads();
+  const bool direct = lo == 1000;
+  if (tid == 0) {
+    T.flag[p][panel] = direct ? 2 : hi == lo ? 0 : 1;
+    T.r0[p][panel] = (unsigned char)(direct ? kRMin : lo);
+  }
+  const int r0 = direct ? 0 : lo - kRMin;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const cd J = rj[r0 + s][tid], K = rk[r0 + s][tid];
+    if constexpr (REAL) {
+      double2 *v = (double2 *)T.val[p] + (size_t)(panel * 2 + s) * 64;
+      v[i * 8 + j] = make_double2(J.x, K.x);
+    } else {
+      double2 *v = (double2 *)T.val[p] + (size_t)(panel * 2 + s) * 128;
+      v[(i * 2) * 8 + j] = make_double2(J.x, J.y);
+      v[(i * 2 + 1) * 8 + j] = make_double2(K.x, K.y);
+    }
+  }
+}
+
+// Sub-cell maps of the panels that need one: the stopping ring at the 33 x 33 corners.
+template <bool REAL>
+__global__ void __launch_bounds__(256) k_jktab_map(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
+                                                   double us2y) {
+  __shared__ cd ph1[1][kPhase], ph2[1][kPhase];
+  __shared__ double etab[256];
+  constexpr int kCorners = (kSub + 1) * (kSub + 1);
+  __shared__ unsigned char cls[kCorners];
+  extern __shared__ __align__(16) unsigned char map_smem[];
+  cd *cj = (cd *)map_smem, *ck = cj + kCorners;
+  const int p = blockIdx.y, panel = blockIdx.x;
+  if (T.flag[p][panel] != 1) return;
+  PsiGroup one{};
+  one.n = 1;
+  one.psi1[0] = pg.psi1[p];
+  one.psi2[0] = pg.psi2[p];
+  fill_phases<1>(one, 1, ph1, ph2, etab);
+  __syncthreads();
+  const int r0 = T.r0[p][panel], ia = panel % T.na, ib = panel / T.na;
+  for (int e = threadIdx.x; e < (kSub + 1) * (kSub + 1); e += blockDim.x) {
+    const int i = e / (kSub + 1), j = e % (kSub + 1);
+    const double a = T.a0 + (ia + (double)i / kSub) / T.ra, b = T.b0 + (ib + (double)j / kSub) / T.rb;
+    bool at, before;
+    cd js, ks;
+    const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0],
+                                   etab, kSubMargin, kSubCurve, at, before, js, ks, [](int, cd, cd) {});
+    cls[e] = !at || !before || R < r0 || R > r0 + 1 ? 2 : R - r0;
+    cj[e] = js;
+    ck[e] = ks;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < kSub * kSub; e += blockDim.x) {
+    const int e0 = e / kSub * (kSub + 1) + e % kSub;
+    const int c[4] = {e0, e0 + 1, e0 + kSub + 1, e0 + kSub + 2};
+    int v = cls[c[0]];
+    const cd j4[4] = {cj[c[0]], cj[c[1]], cj[c[2]], cj[c[3]]}, k4[4] = {ck[c[0]], ck[c[1]], ck[c[2]], ck[c[3]]};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (cls[c[q]] != v || near_zero(j4[q], j4) || near_zero(k4[q], k4)) v = 2;
+    T.map[p][(size_t)panel * kSub * kSub + e] = (unsigned char)v;
+  }
+}
+
+// Lagrange basis of the panel nodes at t, times s.
+__device__ __forceinline__ void basis8(double t, double s, double *out) {
+  double d[kND], pre[kND];
+#pragma unroll
+  for (int k = 0; k < kND; ++k) d[k] = t - c_node[k];
+  pre[0] = s;
+#pragma unroll
+  for (int k = 1; k < kND; ++k) pre[k] = pre[k - 1] * d[k - 1];
+  double suf = 1.0;
+#pragma unroll
+  for (int k = kND - 1; k >= 0; --k) {
+    out[k] = (pre[k] * suf) * c_nodew[k];
+    suf *= d[k];
+  }
+}
+
+constexpr int kTabThreads = 128;
+constexpr int kBasStride = 7 * 2 * kND + 2;  // doubles per pair: the four pairs of a warp on different banks
+
+// Eight lanes per face pair.  Lane q < 7 owns quadrature point q: its nearest images (rings 0
+// and 1) one by one, its panel, and the Lagrange bases of its position, handed to the pair's
+// lanes through shared memory.  Then every lane j sums its column j of the panel for all seven
+// points into the six moments; a reduce-scatter over the eight lanes leaves moment k in lane k.
+template <int NP, bool REAL>
+__global__ void __launch_bounds__(kTabThreads, 4) k_filljk_tab(SheetDev G, double ul, PsiGroup pg, double us1x,
+                                                               double us1y, double us2x, double us2y, TabDev T,
+                                                               JKGroup jk) {
+  __shared__ cd fnear[NP][9];
+  __shared__ double etab[256];
+  __shared__ __align__(16) double bas[kTabThreads / 8][kBasStride];
+  const int np = NP == 1 ? 1 : pg.n;
+  for (int t = threadIdx.x; t < 256; t += blockDim.x) etab[t] = exp2((double)t / 256.0);
+  for (int t = threadIdx.x; t < NP * 9; t += blockDim.x) {
+    const int p = t / 9, m = t % 9 / 3 - 1, n = t % 3 - 1;
+    double s1, co1, s2, co2;
+    sincos(-((double)m * (p < np ? pg.psi1[p] : 0.0)), &s1, &co1);
+    sincos(-((double)n * (p < np ? pg.psi2[p] : 0.0)), &s2, &co2);
+    fnear[p][t % 9] = mkcd(co1, s1) * mkcd(co2, s2);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, q = lane & 7, grp = lane & ~7;
+  const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
+  const bool live = gid < G.nufp;
+  const int iu = live ? (int)gid : G.nufp - 1;  // idle groups mirror the last pair, write nothing
+  const PairGeo g = pair_geo(G, iu);
+  double ux, uy;
+  quad_offset(g, min(q, 6), ul, ux, uy);
+  // nearest images: the regularised (0, 0) term, then ring 1 in ring order
+  cd js[NP], ks[NP];
+  {
+    const double arg = sqrt(ux * ux + uy * uy);
+    const double rterm = exp_neg(arg, etab);
+    const double j0 = arg <= 1e-5 ? (-arg / 6 + 0.5) * arg - 1 : (rterm - 1) / arg;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) { js[p] = mkcd(0, 0); ks[p] = mkcd(0, 0); }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int m = e < 3 ? 1 : e < 6 ? -1 : 0, n = e < 6 ? e % 3 - 1 : e == 6 ? -1 : 1;
+      const double dx = ux - ((double)m * us1x + (double)n * us2x), dy = uy - ((double)m * us1y + (double)n * us2y);
+      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        if constexpr (REAL) {
+          js[p].x += er * ra;
+          ks[p].x += er;
+        } else {
+          const cd f = fnear[p][(m + 1) * 3 + n + 1];
+          const cd term = mkcd(er * f.x, er * f.y);
+          js[p] = js[p] + mkcd(term.x * ra, term.y * ra);
+          ks[p] = ks[p] + term;
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      js[p].x += j0;
+      ks[p].x += rterm;
+    }
+  }
+  // panel and sub-cell of this point; bases (the quadrature weight goes into the second one)
+  int panel;
+  int sub;
+  {
+    const double fa = (T.iv[0] * ux + T.iv[1] * uy - T.a0) * T.ra, fb = (T.iv[2] * ux + T.iv[3] * uy - T.b0) * T.rb;
+    const int ia = max(0, min(T.na - 1, (int)fa)), ib = max(0, min(T.nb - 1, (int)fb));
+    const double ta = 2.0 * (fa - ia) - 1.0, tb = 2.0 * (fb - ib) - 1.0;
+    panel = ib * T.na + ia;
+    const int ca = max(0, min(kSub - 1, (int)((ta + 1.0) * (0.5 * kSub))));
+    const int cb = max(0, min(kSub - 1, (int)((tb + 1.0) * (0.5 * kSub))));
+    sub = ca * kSub + cb;
+    if (q < 7) {
+      double *o = &bas[threadIdx.x >> 3][q * 2 * kND];
+      basis8(ta, 1.0, o);
+      basis8(tb, c_qw[q], o + kND);
+    }
+  }
+  __syncwarp();
+  double rr0, rr1, ri;
+  edge_terms(g, ul, q, grp, rr0, rr1, ri);
+  const double *mybas = bas[threadIdx.x >> 3];
+  const double qw = q < 7 ? c_qw[q] : 0.0, qx = q < 7 ? c_qxi[q] : 0.0, qe = q < 7 ? c_qeta[q] : 0.0;
+#pragma unroll 1
+  for (int p = 0; p < np; ++p) {
+    // this point's state under phasing p: 0 / 1 the table slot, 2 the direct form
+    int state = T.flag[p][panel];
+    if (state == 1) state = T.map[p][(size_t)panel * kSub * kSub + sub];
+    const unsigned direct = __ballot_sync(0xffffffffu, state == 2 && q < 7) & (0xffu << grp);
+    const int slot = panel * 2 + (state == 1 ? 1 : 0);
+    // near part of the moments: lane q's own point
+    cd jn = mkcd(0, 0), kn = jn;
+#pragma unroll
+    for (int t = 0; t < NP; ++t)
+      if (t == p) { jn = js[t]; kn = ks[t]; }
+    jn = qw * jn;
+    kn = qw * kn;
+    cd acc[6] = {jn, qx * jn, qe * jn, kn, qx * kn, qe * kn};
+    double2 row[REAL ? kND : 2 * kND];
+    int held = -1;
+    const double2 *val = (const double2 *)T.val[p] + q;
+#pragma unroll
+    for (int t = 0; t < 7; ++t) {
+      const int s = __shfl_sync(0xffffffffu, slot, grp + t);
+      if (s != held) {
+        held = s;
+#pragma unroll
+        for (int i = 0; i < (REAL ? kND : 2 * kND); ++i) row[i] = __ldg(val + (size_t)s * (REAL ? 64 : 128) + i * 8);
+      }
+      const double2 *lx = (const double2 *)(mybas + t * 2 * kND);
+      const double ly = mybas[t * 2 * kND + kND + q];
+      if constexpr (REAL) {
+        double jv = 0, kv = 0;
+#pragma unroll
+        for (int i = 0; i < kND; i += 2) {
+          const double2 l = lx[i / 2];
+          jv = fma(l.x, row[i].x, fma(l.y, row[i + 1].x, jv));
+          kv = fma(l.x, row[i].y, fma(l.y, row[i + 1].y, kv));
+        }
+        jv *= ly;
+        kv *= ly;
+        acc[0].x += jv;
+        acc[1].x = fma(c_qxi[t], jv, acc[1].x);
+        acc[2].x = fma(c_qeta[t], jv, acc[2].x);
+        acc[3].x += kv;
+        acc[4].x = fma(c_qxi[t], kv, acc[4].x);
+        acc[5].x = fma(c_qeta[t], kv, acc[5].x);
+      } else {
+        cd jv = mkcd(0, 0), kv = jv;
+#pragma unroll
+        for (int i = 0; i < kND; i += 2) {
+          const double2 l = lx[i / 2];
+          jv.x = fma(l.x, row[2 * i].x, fma(l.y, row[2 * i + 2].x, jv.x));
+          jv.y = fma(l.x, row[2 * i].y, fma(l.y, row[2 * i + 2].y, jv.y));
+          kv.x = fma(l.x, row[2 * i + 1].x, fma(l.y, row[2 * i + 3].x, kv.x));
+          kv.y = fma(l.x, row[2 * i + 1].y, fma(l.y, row[2 * i + 3].y, kv.y));
+        }
+        jv = ly * jv;
+        kv = ly * kv;
+        acc[0] = acc[0] + jv;
+        acc[1] = acc[1] + c_qxi[t] * jv;
+        acc[2] = acc[2] + c_qeta[t] * jv;
+        acc[3] = acc[3] + kv;
+        acc[4] = acc[4] + c_qxi[t] * kv;
+        acc[5] = acc[5] + c_qeta[t] * kv;
+      }
+    }
+    // reduce-scatter over the eight lanes: lane k ends with moment k (lanes 6 and 7 with none)
+    const bool b4 = q & 4, b2 = q & 2, b1 = q & 1;
+    cd h[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const cd keep = b4 ? (k < 2 ? acc[4 + k] : mkcd(0, 0)) : acc[k];
+      const cd send = b4 ? acc[k] : (k < 2 ? acc[4 + k] : mkcd(0, 0));
+      h[k].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 4);
+      h[k].y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 4);
+    }
+    cd h2[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const cd keep = b2 ? h[2 + k] : h[k], send = b2 ? h[k] : h[2 + k];
+      h2[k].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 2);
+      h2[k].y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 2);
+    }
+    cd out;
+    {
+      const cd keep = b1 ? h2[1] : h2[0], send = b1 ? h2[0] : h2[1];
+      out.x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 1);
+      out.y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 1);
+    }
+    if (!live) continue;
+    const JKDev &o = jk.s[p];
+    if (q == 0) o.J[iu] = out;
+    else if (q == 1) o.Jxi[iu] = out;
+    else if (q == 2) o.Jeta[iu] = out;
+    else if (q == 3) o.K[iu] = out;
+    else if (q == 4) o.Kxi[iu] = out;
+    else if (q == 5) o.Keta[iu] = out;
+    else if (q == 6) {
+      o.rho_r[2 * iu] = rr0;
+      o.rho_r[2 * iu + 1] = rr1;
+    } else {
+      o.rinv[iu] = ri;
+      if (direct) T.list[(size_t)p * G.nufp + atomicAdd(T.count + p, 1)] = iu;
+    }
+  }
+}
+
+// The listed pairs of phasing blockIdx.y by the direct form, over the values just written.
+__global__ void __launch_bounds__(jk_threads<1>(), 3) k_filljk_list(SheetDev G, double ul, PsiGroup pg, double us1x,
+                                                                    double us1y, double us2x, double us2y, TabDev T,
+                                                                    JKGroup jk, int *nonconv) {
+  __shared__ cd ph1[1][kPhase], ph2[1][kPhase];
+  __shared__ double etab[256];
+  const int p = blockIdx.y, cnt = T.count[p];
+  const int per = blockDim.x >> 3;  // pairs of a CTA
+  if ((long long)blockIdx.x * per >= cnt) return;
+  PsiGroup one{};
+  one.n = 1;
+  one.psi1[0] = pg.psi1[p];
+  one.psi2[0] = pg.psi2[p];
+  JKGroup oj{};
+  oj.s[0] = jk.s[p];
+  fill_phases<1>(one, 1, ph1, ph2, etab);
+  __syncthreads();
+  const int *list = T.list + (size_t)p * G.nufp;
+  const int n = (cnt + 3) & ~3;  // whole warps: four pairs each
+  for (int e = blockIdx.x * per + (threadIdx.x >> 3); e < n; e += gridDim.x * per) {
+    const bool live = e < cnt;
+    filljk_pair<1>(G, ul, one, 1, us1x, us1y, us2x, us2y, oj, nonconv + p, list[live ? e : cnt - 1], live, ph1, ph2,
+                   etab);
+  }
+}
+
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+}  // namespace
+
+// The panels of a sheet, or false where the direct form is taken:
+//   * an image of ring 2 lies inside the parallelogram of offsets (a sheet that reaches over
+//     more than a cell), or would need more than 8192 panels;
+//   * fewer than 55 pair classes per panel: seven direct evaluations per class then cost less
+//     than six per table node, which is what the tables cost with their maps.
+bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np, JKTabPlan &P) {
+  P = JKTabPlan{};
+  if (G.nufp < 4096 || !(ulocal > 0) || !(G.ext1 > 0) || !(G.ext2 > 0) || !(G.ext1 < 1.5) || !(G.ext2 < 1.5)) return false;
+  const double e1[2] = {ulocal * s1[0], ulocal * s1[1]}, e2[2] = {ulocal * s2[0], ulocal * s2[1]};
+  const double W1 = G.ext1, W2 = G.ext2;  // |offset| in lattice coordinates (panel indices are clamped)
+  // distance from the parallelogram [-W1, W1] x [-W2, W2] to the nearest image of ring >= 2
+  double dmin = 1e300;
+  for (int m = -5; m <= 5; ++m)
+    for (int n = -5; n <= 5; ++n) {
+      if (std::max(std::abs(m), std::abs(n)) < 2) continue;
+      if (std::fabs(m) <= W1 && std::fabs(n) <= W2) return false;
+      for (int e = 0; e < 4; ++e) {  // edges a = +-W1, b = +-W2
+        const double sgn = e & 1 ? 1 : -1;
+        const double *t = e < 2 ? e2 : e1;                      // edge direction
+        const double fa = e < 2 ? sgn * W1 : 0, fb = e < 2 ? 0 : sgn * W2, half = e < 2 ? W2 : W1;
+        const double px = (m - fa) * e1[0] + (n - fb) * e2[0], py = (m - fa) * e1[1] + (n - fb) * e2[1];
+        const double tt = t[0] * t[0] + t[1] * t[1];
+        const double s = std::max(-half, std::min(half, (px * t[0] + py * t[1]) / tt));
+        dmin = std::min(dmin, std::hypot(px - s * t[0], py - s * t[1]));
+      }
+    }
+  const double h = std::min(dmin / 48.0, 0.15);  // panel half-width (u-scaled; exp(-R) varies on the scale 1)
+  if (!(h > 0)) return false;
+  const double ca = std::ceil(W1 * std::hypot(e1[0], e1[1]) / h), cb = std::ceil(W2 * std::hypot(e2[0], e2[1]) / h);
+  if (!(ca * cb <= kMaxPanels)) return false;
+  P.na = std::max(1, (int)ca);
+  P.nb = std::max(1, (int)cb);
+  const size_t panels = (size_t)P.na * P.nb;
+  if ((size_t)G.nufp < 55 * panels) return false;
+  P.a0 = -W1;
+  P.b0 = -W2;
+  P.ra = P.na / (2 * W1);
+  P.rb = P.nb / (2 * W2);
+  const size_t per = align256(panels * 2 * 64 * 4 * sizeof(double)) + 2 * align256(panels) + align256(panels * kSub * kSub);
+  P.bytes = (size_t)np * (per + (size_t)G.nufp * sizeof(int)) + 512;
+  return true;
+}
+
+size_t pss_jktab_bytes(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np) {
+  JKTabPlan P;
+  return pss_jktab_plan(G, ulocal, s1, s2, np, P) ? P.bytes : 0;
+}
+
+int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const double s1[2], const double s2[2],
+                     const JKGroup &jk, int *nonconv, const JKTabPlan &P, void *ws, cudaStream_t st) {
+  const double a = ulocal * s1[0], b = ulocal * s1[1], c = ulocal * s2[0], d = ulocal * s2[1];
+  const double det = a * d - b * c;
+  const int np = pg.n;
+  const size_t panels = (size_t)P.na * P.nb;
+  TabDev T{};
+  T.iv[0] = d / det; T.iv[1] = -c / det; T.iv[2] = -b / det; T.iv[3] = a / det;
+  T.a0 = P.a0; T.b0 = P.b0; T.ra = P.ra; T.rb = P.rb; T.na = P.na; T.nb = P.nb;
+  char *w = (char *)(((uintptr_t)ws + 255) & ~(uintptr_t)255);
+  for (int p = 0; p < np; ++p) {
+    T.val[p] = (double *)w; w += align256(panels * 2 * 64 * 4 * sizeof(double));
+    T.flag[p] = (unsigned char *)w; w += align256(panels);
+    T.r0[p] = (unsigned char *)w; w += align256(panels);
+    T.map[p] = (unsigned char *)w; w += align256(panels * kSub * kSub);
+  }
+  T.count = (int *)w; w += 64;
+  T.list = (int *)w;
+  PSS_CUDA_TRY(cudaMemsetAsync(T.count, 0, kJKGroup * sizeof(int), st));
+  const bool real = np == 1 && pg.psi1[0] == 0.0 && pg.psi2[0] == 0.0;
+  const dim3 gp((unsigned)panels, np);
+  const unsigned gt = cdiv_u((long long)G.nufp * 8, kTabThreads);
+  for (int k = 0; k < 4; ++k) pss_count_launch();
+  if (real) {
+    k_jktab_nodes<true><<<gp, 64, 0, st>>>(T, pg, a, b, c, d);
+    k_jktab_map<true><<<gp, 256, kMapSmem, st>>>(T, pg, a, b, c, d);
+    k_filljk_tab<1, true><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
+  } else {
+    k_jktab_nodes<false><<<gp, 64, 0, st>>>(T, pg, a, b, c, d);
+    k_jktab_map<false><<<gp, 256, kMapSmem, st>>>(T, pg, a, b, c, d);
+    if (np == 1) k_filljk_tab<1, false><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
+    else if (np == 2) k_filljk_tab<2, false><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
+    else k_filljk_tab<kJKGroup, false><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
+  }
+  k_filljk_list<<<dim3(148, np), jk_threads<1>(), 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk, nonconv);
+  PSS_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
