@@ -12,7 +12,7 @@
 //     (a sparse map of the <= 2W moved positions), CTA 0 writes ipiv and a compact
 //     interchange list, and the rows are copied to their final positions.
 //   * k_laswp applies that list to all other columns in one launch.
-//   * k_trsm_small: the W-row block-row solve L11^{-1} X, one column per thread.
+//   * k_rowsolve: the block-row solve L11^{-1} X of an outer block (or of one panel inside it).
 //   * the Schur complement A22 -= L21 U12: k_gemm64 (FP64 matrix pipe), and in FP32 mode
 //     k_gemm32 for the skinny updates inside an outer block and the tcgen05 3xTF32 kernel
 //     (pss_gemm_tc.cu) for the trailing update of each outer block.
@@ -331,43 +331,134 @@ __global__ void __launch_bounds__(kSwpThreads) k_laswp(Mat<F32> M0, long long ms
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncol - w) return;
   const int c = t < skip0 ? t : t + w;
-  for (int q = 0; q < m; ++q) stage[q][threadIdx.x] = M.get(src[q], c);
+  for (int q0 = 0; q0 < m; q0 += 8) {  // eight loads in flight
+    E t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t[u] = q0 + u < m ? M.get(src[q0 + u], c) : E{0, 0};
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (q0 + u < m) stage[q0 + u][threadIdx.x] = t[u];
+  }
+#pragma unroll 4
   for (int q = 0; q < m; ++q) M.put(dst[q], c, stage[q][threadIdx.x]);
 }
 
-// Rows k0..k0+w-1 of columns [c0, c1): X = L11^{-1} X, L11 the w x w unit-lower block at
-// (k0, k0) in shared memory; one column per thread, its w entries in shared memory too.
-// Runtime loops keep the code small: each instruction of a fully unrolled triangle would
-// run once per launch and miss the instruction cache.
-template <bool F32, int W>
-__global__ void __launch_bounds__(128) k_trsm_small(Mat<F32> M0, long long ms, int k0, int w, int c0, int c1) {
+// Block-row solve: rows k0..k0+jb-1 of columns [c0, c1) become X = L11^{-1} X, L11 the jb x jb
+// unit-lower block at (k0, k0), jb <= NB; COLS columns per CTA, all jb rows of them in shared
+// memory.  32 rows at a time: the 32 columns of L below and on the diagonal go to shared memory;
+// 256 / COLS lanes hold one column of the diagonal solve (rows interleaved, the finished entry
+// broadcast by a shuffle); then the remaining rows take their rank-32 update from shared memory.
+// One launch per outer block replaces four 32-row solves and three updates of the rows between
+// them (with their operand splits): about 10 ms of launches, each too short to fill the chip, per
+// batch of 12 at N = 3976, now 4.1 ms (172 us at the first outer block).
+template <bool F32>
+struct RowSolve {
+  static constexpr int NB = F32 ? 128 : 64, COLS = F32 ? 64 : 32, S = 32, LP = S + 1;
+  static constexpr int LANES = 256 / COLS, NI = S / LANES, CQ = COLS / 16, RQ = (NB - S) / 16;
+  static constexpr int SMEM = (NB * COLS + NB * LP) * (int)sizeof(typename Prec<F32>::E);
+};
+template <bool F32>
+__global__ void __launch_bounds__(256) k_rowsolve(Mat<F32> M0, long long ms, int k0, int jb, int c0, int c1) {
+  using T = RowSolve<F32>;
   using E = typename Prec<F32>::E;
   const Mat<F32> M = M0.at(blockIdx.y, ms);
-  __shared__ E L[W][W];
-  __shared__ E xs[W][128];
-  for (int e = threadIdx.x; e < W * W; e += blockDim.x) {
-    const int i = e / W, t = e % W;
-    L[i][t] = (i < w && t < i) ? M.get(k0 + i, k0 + t) : E{0, 0};
-  }
-  const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ok = c < c1;
-  const int tx = threadIdx.x;
-#pragma unroll 8
-  for (int i = 0; i < w; ++i) xs[i][tx] = ok ? M.get(k0 + i, c) : E{0, 0};
-  __syncthreads();
-  for (int i = 1; i < w; ++i) {
-    E v0 = xs[i][tx], v1{0, 0};  // two partial sums halve the dependency chain
-    int t = 0;
-    for (; t + 1 < i; t += 2) {
-      v0 = csubE(v0, cmulE(L[i][t], xs[t][tx]));
-      v1 = caddE(v1, cmulE(L[i][t + 1], xs[t + 1][tx]));
+  extern __shared__ __align__(16) unsigned char rs_smem[];
+  E *X = (E *)rs_smem;          // [jb][COLS]
+  E *L = X + T::NB * T::COLS;   // [jb - b0][LP]
+  const int tid = threadIdx.x, cb = c0 + blockIdx.x * T::COLS;
+  {
+    const int c = tid % T::COLS, rstep = 256 / T::COLS;
+    const bool ok = cb + c < c1;
+    for (int r0 = tid / T::COLS; r0 < jb; r0 += 8 * rstep) {  // eight loads in flight
+      E t[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int r = r0 + u * rstep;
+        t[u] = (ok && r < jb) ? M.get(k0 + r, cb + c) : E{0, 0};
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + u * rstep < jb) X[(r0 + u * rstep) * T::COLS + c] = t[u];
     }
-    if (t < i) v0 = csubE(v0, cmulE(L[i][t], xs[t][tx]));
-    xs[i][tx] = csubE(v0, v1);
   }
-  if (ok) {
+  for (int b0 = 0; b0 < jb; b0 += T::S) {
+    __syncthreads();  // X rows written, L of the previous step read
+    const int nr = jb - b0, nc = min(T::S, nr);
+    for (int r0 = tid >> 5; r0 < nr; r0 += 64) {
+      E t[8];
+      const int k = tid & 31;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) t[u] = (r0 + 8 * u < nr && k < nc) ? M.get(k0 + b0 + r0 + 8 * u, k0 + b0 + k) : E{0, 0};
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + 8 * u < nr) L[(r0 + 8 * u) * T::LP + k] = t[u];
+    }
+    __syncthreads();
+    {
+      const int c = tid / T::LANES, p = tid % T::LANES;
+      E x[T::NI];
+#pragma unroll
+      for (int i = 0; i < T::NI; ++i) {
+        const int r = p + T::LANES * i;
+        x[i] = r < nc ? X[(b0 + r) * T::COLS + c] : E{0, 0};
+      }
+#pragma unroll
+      for (int j = 0; j < T::S - 1; ++j) {
+        E xj;
+        xj.x = __shfl_sync(0xffffffffu, x[j / T::LANES].x, j % T::LANES, T::LANES);
+        xj.y = __shfl_sync(0xffffffffu, x[j / T::LANES].y, j % T::LANES, T::LANES);
+#pragma unroll
+        for (int i = j / T::LANES; i < T::NI; ++i) {
+          const int r = p + T::LANES * i;
+          if (r > j && r < nc) x[i] = csubE(x[i], cmulE(L[r * T::LP + j], xj));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < T::NI; ++i) {
+        const int r = p + T::LANES * i;
+        if (r < nc) X[(b0 + r) * T::COLS + c] = x[i];
+      }
+    }
+    if (b0 + T::S >= jb) break;
+    __syncthreads();
+    // rows b0 + 32 .. jb - 1: rank-32 update; thread (ty, tx) rows ty + 16 i, columns tx + 16 q
+    const int tx = tid & 15, ty = tid >> 4, rem = jb - b0 - T::S;
+    E acc[T::RQ][T::CQ];
+#pragma unroll
+    for (int i = 0; i < T::RQ; ++i)
+#pragma unroll
+      for (int q = 0; q < T::CQ; ++q) acc[i][q] = E{0, 0};
+    const int ni = (rem + 15) / 16;
+#pragma unroll 4
+    for (int k = 0; k < T::S; ++k) {
+      E xv[T::CQ];
+#pragma unroll
+      for (int q = 0; q < T::CQ; ++q) xv[q] = X[(b0 + k) * T::COLS + tx + 16 * q];
+#pragma unroll
+      for (int i = 0; i < T::RQ; ++i) {
+        if (i >= ni) break;
+        const E l = L[min(T::S + ty + 16 * i, T::S + rem - 1) * T::LP + k];
+#pragma unroll
+        for (int q = 0; q < T::CQ; ++q) acc[i][q] = caddE(acc[i][q], cmulE(l, xv[q]));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < T::RQ; ++i) {
+      const int r = ty + 16 * i;
+      if (r >= rem) break;
+#pragma unroll
+      for (int q = 0; q < T::CQ; ++q) {
+        E &z = X[(b0 + T::S + r) * T::COLS + tx + 16 * q];
+        z = csubE(z, acc[i][q]);
+      }
+    }
+  }
+  __syncthreads();
+  {
+    const int c = tid % T::COLS, rstep = 256 / T::COLS;
+    if (cb + c < c1)
 #pragma unroll 8
-    for (int i = 0; i < w; ++i) M.put(k0 + i, c, xs[i][tx]);
+      for (int r = tid / T::COLS; r < jb; r += rstep) M.put(k0 + r, cb + c, X[r * T::COLS + c]);
   }
 }
 
@@ -603,16 +694,18 @@ void launch_laswp(Mat<F32> M, const LuBatch &bt, int nb, int n, int k0, int w, c
 }
 
 template <bool F32>
-void launch_trsm(Mat<F32> M, long long ms, int nb, int k0, int w, int c0, int c1, cudaStream_t st) {
-  if (c1 <= c0) return;
+int launch_rowsolve(Mat<F32> M, long long ms, int nb, int k0, int jb, int c0, int c1, cudaStream_t st) {
+  if (c1 <= c0) return 0;
+  using T = RowSolve<F32>;
+  static DeviceOnce once;
+  if (int rc = device_once(once, [&] {
+        PSS_CUDA_TRY(cudaFuncSetAttribute(k_rowsolve<F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
+        return 0;
+      }))
+    return rc;
   pss_count_launch();
-  const dim3 grid(cdiv_u(c1 - c0, 128), nb);
-  if constexpr (F32) {
-    if (w <= 16) k_trsm_small<true, 16><<<grid, 128, 0, st>>>(M, ms, k0, w, c0, c1);
-    else k_trsm_small<true, 32><<<grid, 128, 0, st>>>(M, ms, k0, w, c0, c1);
-  } else {  // FP64 panels are at most 16 wide
-    k_trsm_small<false, 16><<<grid, 128, 0, st>>>(M, ms, k0, w, c0, c1);
-  }
+  k_rowsolve<F32><<<dim3(cdiv_u(c1 - c0, T::COLS), nb), 256, T::SMEM, st>>>(M, ms, k0, jb, c0, c1);
+  return 0;
 }
 
 int launch_gemm(Mat<false> M, long long ms, int nb, int r0, int r1, int c0, int c1, int k0, int kb,
@@ -668,7 +761,7 @@ int launch_update(Mat<true> M, const LuBatch &bt, int nb, int r0, int r1, int c0
 //   1. each inner panel: factor, its interchanges on every other column, the W-row
 //      triangular solve and Schur update restricted to the outer block's own columns;
 //   2. once all interchanges of the outer block are applied, the block row of the
-//      trailing columns, U12 = L11^{-1} A12, as W-row solves plus block-row updates;
+//      trailing columns, U12 = L11^{-1} A12, in one launch;
 //   3. the trailing matrix A22 -= L21 U12, one GEMM with K = NB.
 // All nb matrices of the batch advance together, one launch per step.
 template <bool F32>
@@ -682,16 +775,12 @@ int lu_blocked(int n, int nb, Mat<F32> M, const LuBatch &bt, int NB, int W, cons
       if ((rc = launch_panel<F32>(M, bt, nb, k0, n - k0, k0, w, st))) return rc;
       launch_laswp<F32>(M, bt, nb, n, k0, w, st);
       if (k0 + w < E) {
-        launch_trsm<F32>(M, bt.ms, nb, k0, w, k0 + w, E, st);
+        if ((rc = launch_rowsolve<F32>(M, bt.ms, nb, k0, w, k0 + w, E, st))) return rc;
         if ((rc = launch_update(M, bt, nb, k0 + w, n, k0 + w, E, k0, w, tc, st))) return rc;
       }
     }
     if (E < n) {
-      for (int k0 = K0; k0 < E; k0 += W) {
-        const int w = min(W, E - k0);
-        launch_trsm<F32>(M, bt.ms, nb, k0, w, E, n, st);
-        if (k0 + w < E && (rc = launch_update(M, bt, nb, k0 + w, E, E, n, k0, w, tc, st))) return rc;
-      }
+      if ((rc = launch_rowsolve<F32>(M, bt.ms, nb, K0, JB, E, n, st))) return rc;
       if ((rc = launch_update(M, bt, nb, E, n, E, n, K0, JB, tc, st))) return rc;
     }
   }
