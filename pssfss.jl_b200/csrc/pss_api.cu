@@ -240,7 +240,7 @@ struct pss_sheet {
   double upm = 1.0;
   double s1[2], s2[2], b1[2], b2[2];
   int nnode = 0, nface = 0, nbf = 0, nufp = 0;
-  DevBuf rho, fv, ufpm, rep, fr, ls, a48, inc_cnt, inc_face, inc_loc, inc_sgn, inc_eci;
+  DevBuf rho, fv, ufpm, rep, fr, ls, a48, inc_cnt, inc_face, inc_loc, inc_sgn, inc_eci, face_m, pfaces, inc;
   SheetDev G{};
   JKBufs cache;
   bool jk_valid = false;
@@ -327,6 +327,22 @@ void make_params(int magnetic, const StackParams &S, const double b1m[2], const 
   P.ff[0] = P.ff[1] = P.ff[3] = mkcd(1, 0);
   P.ff[2] = hcis(-psi1);
   P.ff[4] = hcis(-psi2);
+  const double eps0 = 1.0 / (PSS_MU0 * (PSS_C0 * PSS_C0)), w = P.omega;
+  if (!magnetic) {
+    P.cI1 = mkcd(PSS_FOURPI, 0);
+    P.cK = P.c3 / u;
+    P.cI2 = mkcd(PSS_FOURPI, 0);
+    P.cKP = P.d3 / u;
+    P.zA = mkcd(0.0, w) * ((PSS_MU0 / PSS_FOURPI) * P.mutilde);
+    P.zP = (mkcd(0.0, 1.0) / P.epsbar) * mkcd(1.0 / (PSS_TWOPI * w * eps0), 0.0);
+  } else {
+    P.cI1 = P.I1fact;
+    P.cK = P.KFfact;
+    P.cI2 = P.I2fact;
+    P.cKP = P.KPfact;
+    P.zA = mkcd(0.0, -w) * ((-eps0 / PSS_PI) * P.epsbar);
+    P.zP = mkcd(0.0, 2.0) / ((PSS_PI * w * PSS_MU0) * P.mutilde);
+  }
 }
 
 // Tables of npts points (params already on the device at dP).  Fills tabs[i] and ORs
@@ -378,20 +394,18 @@ int build_tables(pss_ctx *c, const StackParams &S, const PointParams *dP, int np
         size_t cap = pss_table_cap(mmax);
         if (c->bigtables[i].ensure(2 * cap * sizeof(cd))) return -3;
         if (c->stage.ensure(2 * (size_t)mmax * mmax * sizeof(cd))) return -3;
-        tabs[i].t1 = c->bigtables[i].as<cd>();
-        tabs[i].t2 = tabs[i].t1 + cap;
+        tabs[i].t = c->bigtables[i].as<cd>();
         tabs[i].mmax = mmax;
-        int rc = pss_tables_finish(c->bigdense.as<cd>(), R1, mmax, dP + il, c->stage.as<cd>(), tabs[i].t1,
-                                   tabs[i].t2, st);
+        int rc = pss_tables_finish(c->bigdense.as<cd>(), R1, mmax, dP + il, c->stage.as<cd>(), tabs[i].t,
+                                   st);
         if (rc) return rc;
         continue;
       }
       if (flag == 1) hstatus[i] |= PSS_ST_TABLE_NOCONV;
-      tabs[i].t1 = c->tables.as<cd>() + (size_t)i * 2 * cap0;
-      tabs[i].t2 = tabs[i].t1 + cap0;
+      tabs[i].t = c->tables.as<cd>() + (size_t)i * 2 * cap0;
       tabs[i].mmax = mmax;
       int rc = pss_tables_finish(c->dense.as<cd>() + (size_t)q * pstride, R0, mmax, dP + il, c->stage.as<cd>(),
-                                 tabs[i].t1, tabs[i].t2, st);
+                                 tabs[i].t, st);
       if (rc) return rc;
     }
   }
@@ -550,10 +564,12 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     if (ufpm[i] < 1 || ufpm[i] > nufp) { pss_set_error("ufpm entry out of range"); delete sh; return -1; }
     hufpm[i] = (int)(ufpm[i] - 1);
   }
-  std::vector<int> hrep(nufp);
+  std::vector<int> hrep(nufp), hpf(2 * nufp);
   for (int64_t i = 0; i < nufp; ++i) {
     if (ufp_rep[i] < 1 || ufp_rep[i] > nface * nface) { pss_set_error("ufp_rep out of range"); delete sh; return -1; }
     hrep[i] = (int)(ufp_rep[i] - 1);
+    hpf[2 * i] = (int)((ufp_rep[i] - 1) % nface);
+    hpf[2 * i + 1] = (int)((ufp_rep[i] - 1) / nface);
   }
   // basis-function incidences: (face, local edge, sign, edge code), fixed order
   std::vector<int> icnt(nbf, 0), iface(4 * nbf, 0), iloc(4 * nbf, 0), isgn(4 * nbf, 0), ieci(4 * nbf, 0);
@@ -578,14 +594,18 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
       ++cnt;
     }
   // per-face edge lengths (m) and 48|area| (m^2) for the surface-resistance terms
-  std::vector<double> hls(3 * nface), ha48(nface);
+  std::vector<double> hls(3 * nface), ha48(nface), hfm(8 * nface);
   for (int64_t f = 0; f < nface; ++f) {
     double r[3][2];
     for (int k = 0; k < 3; ++k) {
       int64_t v = fv[3 * f + k] - 1;
       r[k][0] = rho[2 * v] / units_per_meter;
       r[k][1] = rho[2 * v + 1] / units_per_meter;
+      hfm[8 * f + 2 * k] = r[k][0];
+      hfm[8 * f + 2 * k + 1] = r[k][1];
     }
+    hfm[8 * f + 6] = ((r[0][0] + r[1][0]) + r[2][0]) / 3;
+    hfm[8 * f + 7] = ((r[0][1] + r[1][1]) + r[2][1]) / 3;
     double a32x = r[2][0] - r[1][0], a32y = r[2][1] - r[1][1];
     double a12x = r[0][0] - r[1][0], a12y = r[0][1] - r[1][1];
     double a13x = r[0][0] - r[2][0], a13y = r[0][1] - r[2][1];
@@ -602,6 +622,12 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     const double a[2] = {(x * s2[1] - y * s2[0]) / cell, (y * s1[0] - x * s1[1]) / cell};
     for (int d = 0; d < 2; ++d) { lo[d] = std::min(lo[d], a[d]); hi[d] = std::max(hi[d], a[d]); }
   }
+  std::vector<int> hinc(4 * nbf, 0);
+  for (int64_t b = 0; b < nbf; ++b)
+    for (int q = 0; q < icnt[b]; ++q) {
+      const int64_t o = 4 * b + q;
+      hinc[o] = iface[o] << 8 | iloc[o] << 4 | (isgn[o] < 0 ? 8 : 0) | ieci[o];
+    }
   std::vector<double> hfr(fr, fr + nface);
   int rc = 0;
   rc |= upload(sh->rho, rho, 2 * (size_t)nnode);
@@ -616,6 +642,9 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   rc |= upload(sh->inc_loc, iloc.data(), iloc.size());
   rc |= upload(sh->inc_sgn, isgn.data(), isgn.size());
   rc |= upload(sh->inc_eci, ieci.data(), ieci.size());
+  rc |= upload(sh->face_m, hfm.data(), hfm.size());
+  rc |= upload(sh->pfaces, hpf.data(), hpf.size());
+  rc |= upload(sh->inc, hinc.data(), hinc.size());
   if (rc) { delete sh; return -3; }
   SheetDev &G = sh->G;
   G.nface = sh->nface; G.nbf = sh->nbf; G.nufp = sh->nufp; G.nnode = sh->nnode; G.upm = units_per_meter;
@@ -623,6 +652,8 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   G.fr = sh->fr.as<double>(); G.face_ls = sh->ls.as<double>(); G.face_a48 = sh->a48.as<double>();
   G.inc_cnt = sh->inc_cnt.as<int>(); G.inc_face = sh->inc_face.as<int>(); G.inc_loc = sh->inc_loc.as<int>();
   G.inc_sgn = sh->inc_sgn.as<int>(); G.inc_eci = sh->inc_eci.as<int>();
+  G.face_m = sh->face_m.as<double>(); G.pair_faces = sh->pfaces.as<int2>(); G.inc = sh->inc.as<int4>();
+  G.has_res = std::any_of(hfr.begin(), hfr.end(), [](double r) { return r != 0.0; }) ? 1 : 0;
   G.ext1 = hi[0] - lo[0]; G.ext2 = hi[1] - lo[1];
   *out = sh;
   return 0;
@@ -633,7 +664,7 @@ int pss_sheet_destroy(pss_sheet *sh) {
   cudaSetDevice(sh->ctx->device);
   cudaDeviceSynchronize();
   for (DevBuf *b : {&sh->rho, &sh->fv, &sh->ufpm, &sh->rep, &sh->fr, &sh->ls, &sh->a48, &sh->inc_cnt,
-                    &sh->inc_face, &sh->inc_loc, &sh->inc_sgn, &sh->inc_eci})
+                    &sh->inc_face, &sh->inc_loc, &sh->inc_sgn, &sh->inc_eci, &sh->face_m, &sh->pfaces, &sh->inc})
     b->release();
   sh->cache.buf.release();
   delete sh;
@@ -952,7 +983,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
       for (int q = 0; q < gsz; ++q, ++b) {
         const int g = PR[it.p[b]].p0 + it.i[b];
         const PointParams *Pi = dP + g;
-        pss_fill_pairs(sh->G, Pi, jks[q], tabs[g].t1, tabs[g].t2, tabs[g].mmax, w.zb.as<cd>(), st);
+        pss_fill_pairs(sh->G, Pi, jks[q], tabs[g], w.zb.as<cd>(), st);
         pss_fill_assemble(sh->G, Pi, w.zb.as<cd>(), w.z64.as<cd>() + b * msz, zr ? zr + b * msf : nullptr,
                           zi ? zi + b * msf : nullptr, ld, ldf, st);
       }
@@ -1006,7 +1037,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
             pss_count_launch();
             k_nonconv_to_status<<<1, 1, 0, st>>>(w.nonconv.as<int>(), dstatus + PR[0].p0 + i);
           }
-          pss_fill_pairs(Q.sh->G, dP + gq, jq, tabs[gq].t1, tabs[gq].t2, tabs[gq].mmax, w.zb.as<cd>(), st);
+          pss_fill_pairs(Q.sh->G, dP + gq, jq, tabs[gq], w.zb.as<cd>(), st);
           pss_bfft(Q.sh->G, nm, dkv + Q.kb + (size_t)i * nm * 2, Q.psi[2 * i], Q.psi[2 * i + 1], bfk, st);
           pss_rhs(n, nm, bfk, dsrc + Q.sb + (size_t)i * nm * 2, Rk, st);
           const size_t o = ((size_t)k * np0 + i) * nm2;
@@ -1210,7 +1241,7 @@ int pss_fill_matrix(pss_sheet *sh, int nl, const double *eps, const double *mu, 
   Worker &w = c->w[0];
   if ((rc = refresh_jk_cache(sh, psi1, psi2, u / sh->upm, w))) return rc;
   if ((rc = ensure_worker(w, sh, 1, PSS_FP64, false, 1))) return rc;
-  pss_fill_pairs(sh->G, c->params.as<PointParams>(), sh->cache.jk, tabs[0].t1, tabs[0].t2, tabs[0].mmax,
+  pss_fill_pairs(sh->G, c->params.as<PointParams>(), sh->cache.jk, tabs[0],
                  w.zb.as<cd>(), w.st);
   pss_fill_assemble(sh->G, c->params.as<PointParams>(), w.zb.as<cd>(), w.z64.as<cd>(), nullptr, nullptr, sh->nbf, sh->nbf,
                     w.st);
@@ -1245,8 +1276,12 @@ int pss_modal_tables(pss_ctx *c, int magnetic, int nl, const double *eps, const 
   *mmax_out = tabs[0].mmax;
   if (status) *status = hs[0];
   if ((int64_t)need > cap) { pss_set_error("table capacity %lld < %zu", (long long)cap, need); return -2; }
-  PSS_CUDA_TRY(cudaMemcpy(t1, tabs[0].t1, need * sizeof(cd), cudaMemcpyDeviceToHost));
-  PSS_CUDA_TRY(cudaMemcpy(t2, tabs[0].t2, need * sizeof(cd), cudaMemcpyDeviceToHost));
+  std::vector<cd> both(2 * need);  // the device keeps both tables of a node side by side
+  PSS_CUDA_TRY(cudaMemcpy(both.data(), tabs[0].t, 2 * need * sizeof(cd), cudaMemcpyDeviceToHost));
+  for (size_t e = 0; e < need; ++e) {
+    ((cd *)t1)[e] = both[2 * e];
+    ((cd *)t2)[e] = both[2 * e + 1];
+  }
   return 0;
 }
 
@@ -1461,10 +1496,8 @@ int point_tables(pss_ctx *c, const StackParams &S, const PointParams *dP, DevBuf
   const size_t used = (size_t)(tabs[0].mmax + 2) * (tabs[0].mmax + 2);
   if (own.ensure(2 * used * sizeof(cd))) return -3;
   cudaStream_t st = c->w[0].st;
-  PSS_CUDA_TRY(cudaMemcpyAsync(own.p, tabs[0].t1, used * sizeof(cd), cudaMemcpyDeviceToDevice, st));
-  PSS_CUDA_TRY(cudaMemcpyAsync(own.as<cd>() + used, tabs[0].t2, used * sizeof(cd), cudaMemcpyDeviceToDevice, st));
-  t.t1 = own.as<cd>();
-  t.t2 = own.as<cd>() + used;
+  PSS_CUDA_TRY(cudaMemcpyAsync(own.p, tabs[0].t, 2 * used * sizeof(cd), cudaMemcpyDeviceToDevice, st));
+  t.t = own.as<cd>();
   t.mmax = tabs[0].mmax;
   hstat |= hs[0];
   return 0;
@@ -1584,7 +1617,7 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
     if ((rc = refresh_jk_cache(sh, psi[2 * i], psi[2 * i + 1], u / sh->upm, w))) return rc;
     if (sh->jk_nonconv) hst |= PSS_ST_JK_NOCONV;
     // Z into slot 0 (and the FP32 planes), fills and transforms of every set
-    pss_fill_pairs(sh->G, dP, sh->cache.jk, t0.t1, t0.t2, t0.mmax, w.zb.as<cd>(), st);
+    pss_fill_pairs(sh->G, dP, sh->cache.jk, t0, w.zb.as<cd>(), st);
     pss_fill_assemble(sh->G, dP, w.zb.as<cd>(), w.z64.as<cd>(), zr, zi, ld, Worker::ld32(n), st);
     cd *bf = w.bf.as<cd>();
     const size_t bfs = (size_t)nm * n * 2;
@@ -1595,7 +1628,7 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
       const double *pp = ppsi + 2 * ((size_t)k * npts + i);
       if ((rc = refresh_jk_cache(q, pp[0], pp[1], pu[k] / q->upm, w))) return rc;
       if (q->jk_nonconv) hst |= PSS_ST_JK_NOCONV;
-      pss_fill_pairs(q->G, dP + 1 + k, q->cache.jk, tk[k].t1, tk[k].t2, tk[k].mmax, w.zb.as<cd>(), st);
+      pss_fill_pairs(q->G, dP + 1 + k, q->cache.jk, tk[k], w.zb.as<cd>(), st);
       pss_fill_assemble(q->G, dP + 1 + k, w.zb.as<cd>(), w.z64.as<cd>() + (1 + k) * msz, nullptr, nullptr, ld, ld,
                         st);
       pss_bfft(q->G, nm, kv_of(1 + k), pp[0], pp[1], bf + (1 + k) * bfs, st);

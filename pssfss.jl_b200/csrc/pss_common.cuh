@@ -45,6 +45,17 @@ __host__ __device__ __forceinline__ cd conjd(cd a) { return cd{a.x, -a.y}; }
 // Real - Complex keeping the sign of a zero imaginary part: Complex(x - re, -im).
 __host__ __device__ __forceinline__ cd rsubc(double x, cd z) { return cd{x - z.x, -z.y}; }
 
+// acc + a * b and acc - a * b, four fused multiply-adds each (written as operators, the product
+// is rounded before the sum: six operations).
+template <class C>
+__host__ __device__ __forceinline__ C cmac(C acc, C a, C b) {
+  return C{fma(a.x, b.x, fma(-a.y, b.y, acc.x)), fma(a.x, b.y, fma(a.y, b.x, acc.y))};
+}
+template <class C>
+__host__ __device__ __forceinline__ C cmsub(C acc, C a, C b) {
+  return C{fma(-a.x, b.x, fma(a.y, b.y, acc.x)), fma(-a.x, b.y, fma(-a.y, b.x, acc.y))};
+}
+
 // Smith's complex division with scaling.
 __host__ __device__ __forceinline__ cd operator/(cd a, cd b) {
   if (fabs(b.y) <= fabs(b.x)) {

@@ -34,138 +34,155 @@ __global__ void __launch_bounds__(jk_threads<NP>(), 3) k_filljk(SheetDev G, doub
   filljk_pair<NP>(G, ul, pg, np, us1x, us1y, us2x, us2y, jk, nonconv, gid, gid < G.nufp, ph1, ph2, etab);
 }
 
-// Per-point coefficients that turn the face-pair integrals into Z terms:
-//   a_isl = cI1*I1_i + sing + u*J_i + cK*K_i,   φ = cI2*I2 + u*(rinv + J) + cKP*K,
-//   term(isl, iml) = zA*(ρc2[iml]·a_isl) - zP*φ.
-struct PairCoef {
-  cd cI1, cK, cI2, cKP, zA, zP;
-};
-
-__device__ __forceinline__ PairCoef pair_coef(const PointParams &P) {
-  PairCoef c;
-  const double eps0 = 1.0 / (PSS_MU0 * (PSS_C0 * PSS_C0));
-  const double u = P.u, w = P.omega;
-  if (!P.magnetic) {
-    c.cI1 = mkcd(PSS_FOURPI, 0);
-    c.cK = P.c3 / u;
-    c.cI2 = mkcd(PSS_FOURPI, 0);
-    c.cKP = P.d3 / u;
-    c.zA = mkcd(0.0, w) * ((PSS_MU0 / PSS_FOURPI) * P.mutilde);
-    c.zP = (mkcd(0.0, 1.0) / P.epsbar) * mkcd(1.0 / (PSS_TWOPI * w * eps0), 0.0);
-  } else {
-    c.cI1 = P.I1fact;
-    c.cK = P.KFfact;
-    c.cI2 = P.I2fact;
-    c.cKP = P.KPfact;
-    c.zA = mkcd(0.0, -w) * ((-eps0 / PSS_PI) * P.epsbar);
-    c.zP = mkcd(0.0, 2.0) / ((PSS_PI * w * PSS_MU0) * P.mutilde);
-  }
-  return c;
+__device__ __forceinline__ cd ld_cd(const cd *p) {  // one 16-byte load
+  const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+  return mkcd(v.x, v.y);
 }
 
-__global__ void __launch_bounds__(128, 5) k_pairs(SheetDev G, const PointParams *__restrict__ Pp, JKDev jk,
-                                               const cd *__restrict__ t1, const cd *__restrict__ t2, int mmax,
-                                               cd *__restrict__ zb) {
-  int iu = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per class.  Bound by its FP64 operations (about 1200) and the gathers of its 42
+// table nodes; what does not belong to the pair is prepared elsewhere: the point's coefficients
+// on the host, vertices in metres and centroids per face at the upload, the cell-shift phases
+// per CTA, both tables of a node in one 32-byte load.  613 -> 310 us for the 3.19M classes of the
+// N = 3976 meander.
+__global__ void __launch_bounds__(128, 4) k_pairs(SheetDev G, const PointParams *__restrict__ Pp, JKDev jk,
+                                               const cd *__restrict__ tab, int mmax, cd *__restrict__ zb) {
+  __shared__ PointParams P;
+  __shared__ cd ph[9];
+  for (int e = threadIdx.x; e < (int)(sizeof(PointParams) / sizeof(double)); e += blockDim.x)
+    ((double *)&P)[e] = ((const double *)Pp)[e];
+  __syncthreads();
+  if (threadIdx.x < 9) ph[threadIdx.x] = cisd(-((double)((int)threadIdx.x / 3 - 1) * P.psi1 + (double)((int)threadIdx.x % 3 - 1) * P.psi2));
+  __syncthreads();
+  const int iu = blockIdx.x * blockDim.x + threadIdx.x;
   if (iu >= G.nufp) return;
-  const PointParams &P = *Pp;
-  const PairCoef C = pair_coef(P);
-  int fp = G.ufp_rep[iu];
-  int ifm = fp % G.nface, ifs = fp / G.nface;
-  const double inv = 1.0 / G.upm;
-  double rs[3][2], rm[3][2];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    int vs = G.fv[3 * ifs + k], vm = G.fv[3 * ifm + k];
-    rs[k][0] = G.rho[2 * vs] / G.upm;
-    rs[k][1] = G.rho[2 * vs + 1] / G.upm;
-    rm[k][0] = G.rho[2 * vm] / G.upm;
-    rm[k][1] = G.rho[2 * vm + 1] / G.upm;
-  }
-  (void)inv;
-  double rmc[2] = {((rm[0][0] + rm[1][0]) + rm[2][0]) / 3, ((rm[0][1] + rm[1][1]) + rm[2][1]) / 3};
+  const cd *phase = P.psi1 == 0.0 && P.psi2 == 0.0 ? nullptr : ph;
+  const int2 pf = __ldg(G.pair_faces + iu);
+  const double2 *fm = reinterpret_cast<const double2 *>(G.face_m);
+  const double2 rs0 = __ldg(fm + 4 * pf.y), rs1 = __ldg(fm + 4 * pf.y + 1), rs2 = __ldg(fm + 4 * pf.y + 2);
+  const double2 rc = __ldg(fm + 4 * pf.x + 3);
+  const double2 e1 = make_double2(rs1.x - rs0.x, rs1.y - rs0.y), e2 = make_double2(rs2.x - rs0.x, rs2.y - rs0.y);
   cd I1 = mkcd(0, 0), I1x = I1, I1e = I1, I2 = I1;
+#pragma unroll 1
   for (int i = 0; i < 7; ++i) {
-    double rtx = (rs[0][0] + (rs[1][0] - rs[0][0]) * c_qxi[i]) + (rs[2][0] - rs[0][0]) * c_qeta[i];
-    double rty = (rs[0][1] + (rs[1][1] - rs[0][1]) * c_qxi[i]) + (rs[2][1] - rs[0][1]) * c_qeta[i];
-    double dx = rmc[0] - rtx, dy = rmc[1] - rty;
-    cd g1 = sigma_interp(t1, mmax, P, dx, dy);
-    cd g2 = sigma_interp(t2, mmax, P, dx, dy);
-    cd g1w = c_qw[i] * g1;
-    I1x = I1x + c_qxi[i] * g1w;
-    I1e = I1e + c_qeta[i] * g1w;
-    I1 = I1 + g1w;
-    I2 = I2 + c_qw[i] * g2;
+    const double xi = c_qxi[i], eta = c_qeta[i], w = c_qw[i];
+    const double rtx = (rs0.x + e1.x * xi) + e2.x * eta, rty = (rs0.y + e1.y * xi) + e2.y * eta;
+    cd g1, g2;
+    sigma_interp(tab, mmax, P, rc.x - rtx, rc.y - rty, phase, g1, g2);
+    g1 = w * g1;
+    I1x = mkcd(fma(xi, g1.x, I1x.x), fma(xi, g1.y, I1x.y));
+    I1e = mkcd(fma(eta, g1.x, I1e.x), fma(eta, g1.y, I1e.y));
+    I1 = I1 + g1;
+    I2 = mkcd(fma(w, g2.x, I2.x), fma(w, g2.y, I2.y));
   }
-  cd J = jk.J[iu], Jx = jk.Jxi[iu], Je = jk.Jeta[iu];
-  cd K = jk.K[iu], Kx = jk.Kxi[iu], Ke = jk.Keta[iu];
-  double rinv = jk.rinv[iu], rr0 = jk.rho_r[2 * iu], rr1 = jk.rho_r[2 * iu + 1];
-  cd I1z = (I1 - I1x) - I1e, Jz = (J - Jx) - Je, Kz = (K - Kx) - Ke;
   const double u = P.u;
-  cd phi = (C.cI2 * I2 + u * (mkcd(rinv, 0) + J)) + C.cKP * K;
-  cd zphi = C.zP * phi;
-  double rc2[3][2];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    rc2[i][0] = 0.5 * (rmc[0] - rm[i][0]);
-    rc2[i][1] = 0.5 * (rmc[1] - rm[i][1]);
-  }
-  cd *out = zb + iu;  // plane q at out[q * nufp]: consecutive classes, coalesced stores
+  const double rinv = jk.rinv[iu];
+  const double2 rr = __ldg(reinterpret_cast<const double2 *>(jk.rho_r) + iu);
+  // cI1*I1 + u*J + cK*K and its xi, eta moments; the third barycentric moment is the rest
+  const cd J = ld_cd(jk.J + iu), K = ld_cd(jk.K + iu);
+  const cd zphi = P.zP * cmac(cmac(u * mkcd(rinv + J.x, J.y), P.cI2, I2), P.cKP, K);
+  const cd A0 = cmac(cmac(u * J, P.cI1, I1), P.cK, K);
+  const cd Ax = cmac(cmac(u * ld_cd(jk.Jxi + iu), P.cI1, I1x), P.cK, ld_cd(jk.Kxi + iu));
+  const cd Ae = cmac(cmac(u * ld_cd(jk.Jeta + iu), P.cI1, I1e), P.cK, ld_cd(jk.Keta + iu));
+  const cd Az = (A0 - Ax) - Ae;
+  const double2 rm0 = __ldg(fm + 4 * pf.x), rm1 = __ldg(fm + 4 * pf.x + 1), rm2 = __ldg(fm + 4 * pf.x + 2);
+  // rho - r_isl integrated: the moments weighted by the vertices' offsets from vertex isl
+  double2 *out = reinterpret_cast<double2 *>(zb) + iu;  // plane q at out[q * nufp]: coalesced stores
 #pragma unroll
   for (int isl = 0; isl < 3; ++isl) {
-    double sing0 = rr0 + (u * rinv) * (rmc[0] - rs[isl][0]);
-    double sing1 = rr1 + (u * rinv) * (rmc[1] - rs[isl][1]);
+    const double2 ri = isl == 0 ? rs0 : isl == 1 ? rs1 : rs2;
     cd av[2];
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
-      cd Ii = ((rs[0][d] * I1x + rs[1][d] * I1e) + rs[2][d] * I1z) - rs[isl][d] * I1;
-      cd Ji = ((rs[0][d] * Jx + rs[1][d] * Je) + rs[2][d] * Jz) - rs[isl][d] * J;
-      cd Ki = ((rs[0][d] * Kx + rs[1][d] * Ke) + rs[2][d] * Kz) - rs[isl][d] * K;
-      double sg = d == 0 ? sing0 : sing1;
-      av[d] = ((C.cI1 * Ii + mkcd(sg, 0)) + u * Ji) + C.cK * Ki;
+      const double o = d ? ri.y : ri.x;
+      const double d0 = (d ? rs0.y : rs0.x) - o, d1 = (d ? rs1.y : rs1.x) - o, d2 = (d ? rs2.y : rs2.x) - o;
+      const double sg = (d ? rr.y : rr.x) + (u * rinv) * ((d ? rc.y : rc.x) - o);
+      av[d] = mkcd(fma(d0, Ax.x, fma(d1, Ae.x, fma(d2, Az.x, sg))), fma(d0, Ax.y, fma(d1, Ae.y, d2 * Az.y)));
+      av[d] = P.zA * av[d];
     }
 #pragma unroll
     for (int iml = 0; iml < 3; ++iml) {
-      cd dp = rc2[iml][0] * av[0] + rc2[iml][1] * av[1];
-      out[(size_t)(3 * isl + iml) * G.nufp] = C.zA * dp - zphi;
+      const double2 rm = iml == 0 ? rm0 : iml == 1 ? rm1 : rm2;
+      const double cx = 0.5 * (rc.x - rm.x), cy = 0.5 * (rc.y - rm.y);
+      out[(size_t)(3 * isl + iml) * G.nufp] =
+          make_double2(fma(cx, av[0].x, fma(cy, av[1].x, -zphi.x)), fma(cx, av[0].y, fma(cy, av[1].y, -zphi.y)));
     }
   }
+}
+
+// The incidences of a test basis function, unpacked once per thread: face, slot and conjugated
+// signed Floquet factor of each (unused ones repeat the first with factor 0).
+struct RowInc {
+  int cnt, face[4], loc[4];
+  cd flag[4];
+};
+__device__ __forceinline__ void unpack_inc(int4 v, const cd *ff, int cnt, bool conj, RowInc &r) {
+  const int q[4] = {v.x, v.y, v.z, v.w};
+  r.cnt = cnt;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int e = a < cnt ? q[a] : q[0];
+    r.face[a] = e >> 8;
+    r.loc[a] = (e >> 4) & 3;
+    cd f = ff[e & 7];
+    if (conj) f = conjd(f);
+    r.flag[a] = a < cnt ? (e & 8 ? -f : f) : mkcd(0, 0);
+  }
+}
+
+// Surface-resistance term of incidences (fa, ka) x (fa, kb) of one face (Eqs. 7-34/7-35,
+// FillZY.jl:221-230).
+__device__ __noinline__ cd resistance_term(const SheetDev &G, int fa, int ka, int kb, cd mflag, cd sflag) {
+  const double fr = G.fr[fa];
+  if (fr == 0.0) return mkcd(0, 0);
+  const double *ls = G.face_ls + 3 * fa;
+  const double g = fr / G.face_a48[fa];
+  if (ka == kb) {  // the other two edges of the face: next and previous slot
+    const double l1 = ls[(kb + 1) % 3], l2 = ls[(kb + 2) % 3], l0 = ls[kb];
+    return mkcd(g * (3 * (l1 * l1 + l2 * l2) - l0 * l0), 0.0);
+  }
+  const double lt = ls[3 - ka - kb];  // the third edge
+  const double geo = ls[kb] * ls[kb] + ls[ka] * ls[ka] - 3 * (lt * lt);
+  return geo * ((g * sflag) * mflag);
 }
 
 // Z[m, n] (m = test / match basis function, n = source) from the pair terms zb: the <= 4 x 4
 // face incidences of the two basis functions in a fixed order, with the Floquet / sign flags
-// and the surface-resistance terms of Eqs. 7-34/7-35 (FillZY.jl:221-230).
-__device__ __forceinline__ cd assemble_entry(const SheetDev &G, const PointParams &P, const cd *__restrict__ zb,
-                                             int m, int n) {
+// and the surface-resistance terms.  Two by two, the case of every interior edge and of every
+// edge pair across the cell boundary, runs without branches so that its loads overlap.
+__device__ __forceinline__ cd assemble_entry(const SheetDev &G, const cd *ff, bool res, const cd *__restrict__ zb,
+                                             const RowInc &M, int n) {
+  const int cn = __ldg(G.inc_cnt + n);
+  RowInc S;
+  unpack_inc(__ldg(G.inc + n), ff, cn, false, S);
   cd acc = mkcd(0, 0);
-  const int cm = G.inc_cnt[m], cn = G.inc_cnt[n];
-  for (int a = 0; a < cm; ++a) {
-    const int fa = G.inc_face[4 * m + a], ka = G.inc_loc[4 * m + a];
-    const cd ffa = P.ff[G.inc_eci[4 * m + a]];
-    const cd mflag = G.inc_sgn[4 * m + a] > 0 ? conjd(ffa) : -conjd(ffa);
-    for (int b = 0; b < cn; ++b) {
-      const int fb = G.inc_face[4 * n + b], kb = G.inc_loc[4 * n + b];
-      const cd ffb = P.ff[G.inc_eci[4 * n + b]];
-      const cd sflag = G.inc_sgn[4 * n + b] > 0 ? ffb : -ffb;
-      const int iu = G.ufpm[(size_t)fa + (size_t)fb * G.nface];
-      const cd v = zb[(size_t)(3 * kb + ka) * G.nufp + iu];
-      acc = acc + (mflag * sflag) * v;
-      if (!P.magnetic && fa == fb) {
-        const double fr = G.fr[fa];
-        if (fr != 0.0) {
-          const double *ls = G.face_ls + 3 * fa;
-          const double g = fr / G.face_a48[fa];
-          if (ka == kb) {  // the other two edges of the face: next and previous slot
-            double l1 = ls[(kb + 1) % 3], l2 = ls[(kb + 2) % 3], l0 = ls[kb];
-            acc = acc + mkcd(g * (3 * (l1 * l1 + l2 * l2) - l0 * l0), 0.0);
-          } else {
-            double lt = ls[3 - ka - kb];  // the third edge
-            double geo = ls[kb] * ls[kb] + ls[ka] * ls[ka] - 3 * (lt * lt);
-            acc = acc + geo * ((g * sflag) * mflag);
-          }
-        }
+  if (M.cnt <= 2 && cn <= 2) {
+    int iu[4];
+    cd v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      iu[t] = __ldg(G.ufpm + (size_t)M.face[t >> 1] + (size_t)S.face[t & 1] * G.nface);
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      v[t] = ld_cd(zb + (size_t)(3 * S.loc[t & 1] + M.loc[t >> 1]) * G.nufp + iu[t]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc = cmac(acc, M.flag[t >> 1] * S.flag[t & 1], v[t]);
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        if (a >= M.cnt || b >= cn) continue;
+        const int iu = __ldg(G.ufpm + (size_t)M.face[a] + (size_t)S.face[b] * G.nface);
+        acc = cmac(acc, M.flag[a] * S.flag[b], ld_cd(zb + (size_t)(3 * S.loc[b] + M.loc[a]) * G.nufp + iu));
       }
-    }
+  }
+  if (res) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (a < M.cnt && b < cn && M.face[a] == S.face[b])
+          acc = acc + resistance_term(G, M.face[a], M.loc[a], S.loc[b], M.flag[a], S.flag[b]);
   }
   return acc;
 }
@@ -174,21 +191,28 @@ __device__ __forceinline__ cd assemble_entry(const SheetDev &G, const PointParam
 // tile per CTA of 32 x 8 threads.  The gathers run with a warp along the 32 rows of a tile
 // column (consecutive match basis functions against one source basis function: consecutive
 // match faces, so the class look-ups and most pair-term loads of a warp are contiguous); each
-// thread takes 8 columns (independent gathers in flight); the tile then goes out through
-// shared memory row by row, 64 consecutive entries per row.
+// thread keeps its row's incidences and takes 8 columns (independent gathers in flight); the
+// tile then goes out through shared memory row by row, 64 consecutive entries per row.  Bound by
+// the gathers (4 class numbers and 4 pair terms per entry): 460 -> 369 us at N = 3976.
 __global__ void __launch_bounds__(256) k_assemble(SheetDev G, const PointParams *__restrict__ Pp,
                                                   const cd *__restrict__ zb, cd *__restrict__ z64,
                                                   float *__restrict__ zr, float *__restrict__ zi, long long ld,
                                                   long long ldf) {
-  __shared__ cd tile[32][65];
+  __shared__ __align__(16) cd tile[32][65];
+  __shared__ cd ff[8];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 64;
-  const int m = m0 + tx;
-  const PointParams &P = *Pp;
+  if (ty == 0 && tx < 5) ff[tx] = Pp->ff[tx];
+  __syncthreads();
+  const int m = min(m0 + tx, G.nbf - 1);  // rows past the end repeat the last, written nowhere
+  const bool res = G.has_res && !Pp->magnetic;
+  RowInc M;
+  unpack_inc(__ldg(G.inc + m), ff, __ldg(G.inc_cnt + m), true, M);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const int c = ty + 8 * k, n = n0 + c;
-    tile[tx][c] = (m < G.nbf && n < G.nbf) ? assemble_entry(G, P, zb, m, n) : mkcd(0, 0);
+    const int c = ty + 8 * k;
+    const cd v = assemble_entry(G, ff, res, zb, M, min(n0 + c, G.nbf - 1));
+    *reinterpret_cast<double2 *>(&tile[tx][c]) = make_double2(v.x, v.y);
   }
   __syncthreads();
 #pragma unroll
@@ -199,8 +223,8 @@ __global__ void __launch_bounds__(256) k_assemble(SheetDev G, const PointParams 
     for (int h = 0; h < 2; ++h) {
       const int c = tx + 32 * h, n = n0 + c;
       if (n >= G.nbf) continue;
-      const cd v = tile[r][c];
-      if (z64) z64[(size_t)mm * ld + n] = v;
+      const double2 v = *reinterpret_cast<const double2 *>(&tile[r][c]);
+      if (z64) *reinterpret_cast<double2 *>(z64 + (size_t)mm * ld + n) = v;
       if (zr) {
         zr[(size_t)mm * ldf + n] = (float)v.x;
         zi[(size_t)mm * ldf + n] = (float)v.y;
@@ -233,16 +257,23 @@ __global__ void __launch_bounds__(256) k_adj_contract(SheetDev G, const PointPar
   const int csz = (nbf + gridDim.y - 1) / gridDim.y, c0 = blockIdx.y * csz, c1 = min(nbf, c0 + csz);
   __shared__ cd red[8][32][kAdjNB];
   __shared__ cd yrow[32][kAdjNB];
+  __shared__ cd ff[8];
   cd acc[kAdjNB];
 #pragma unroll
   for (int b = 0; b < kAdjNB; ++b) acc[b] = mkcd(0, 0);
-  if (m < nbf) {
-    const PointParams &P = *Pp;
+  if (ty == 0 && tx < 5) ff[tx] = Pp->ff[tx];
+  __syncthreads();
+  {
+    const bool res = G.has_res && !Pp->magnetic;
+    const int mc = min(m, nbf - 1);  // rows past the end repeat the last and are dropped below
+    RowInc M;
+    unpack_inc(__ldg(G.inc + mc), ff, __ldg(G.inc_cnt + mc), true, M);
+#pragma unroll 2
     for (int n = c0 + ty; n < c1; n += 8) {
-      const cd z = assemble_entry(G, P, zb, m, n);
+      const cd z = assemble_entry(G, ff, res, zb, M, n);
 #pragma unroll
       for (int b = 0; b < kAdjNB; ++b)
-        if (b < nb) acc[b] = acc[b] + z * X[(size_t)(b0 + b) * nbf + n];
+        if (b < nb) acc[b] = cmac(acc[b], z, X[(size_t)(b0 + b) * nbf + n]);
     }
   }
 #pragma unroll
@@ -335,11 +366,11 @@ int pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const
   return pss_filljk_group(G, ulocal, 1, &psi1, &psi2, s1, s2, &jk, nonconv, ws, ws_bytes, st);
 }
 
-void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const cd *t1, const cd *t2,
-                    int mmax, cd *zb, cudaStream_t st) {
+void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const TableDev &tab, cd *zb,
+                    cudaStream_t st) {
   if (G.nufp == 0) return;
   pss_count_launch();
-  k_pairs<<<cdiv_u(G.nufp, 128), 128, 0, st>>>(G, dP1, jk, t1, t2, mmax, zb);
+  k_pairs<<<cdiv_u(G.nufp, 128), 128, 0, st>>>(G, dP1, jk, tab.t, tab.mmax, zb);
 }
 
 void pss_fill_assemble(const SheetDev &G, const PointParams *dP1, const cd *zb, cd *z64, float *zr, float *zi,

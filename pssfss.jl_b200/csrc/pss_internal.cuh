@@ -45,6 +45,9 @@ struct PointParams {
   cd f1, f3, p1, p3;                // magnetic summand factors (PGF.jl:496-499)
   cd I1fact, KFfact, I2fact, KPfact;  // filly factors (FillZY.jl:319-322)
   cd ff[5];                         // Floquet factors by edge code (FillZY.jl:72-77)
+  // coefficients of the pair terms (k_pairs): a_isl = cI1*I1_i + sing + u*J_i + cK*K_i,
+  // phi = cI2*I2 + u*(rinv + J) + cKP*K, term(isl, iml) = zA*(rc2[iml] . a_isl) - zP*phi
+  cd cI1, cK, cI2, cKP, zA, zP;
   int magnetic;
 };
 
@@ -66,6 +69,10 @@ struct SheetDev {
   const int *inc_loc;    // 4*nbf local edge slot 0..2
   const int *inc_sgn;    // 4*nbf +1 plus / -1 minus
   const int *inc_eci;    // 4*nbf edge boundary code 0..4
+  const double *face_m;  // 8 per face, metres: the three vertices and the centroid (k_pairs)
+  const int2 *pair_faces;// nufp: (match face, source face) of the class representative
+  const int4 *inc;       // nbf: packed incidences, face << 8 | slot << 4 | minus << 3 | edge code
+  int has_res;           // some face has a surface resistance
   double ext1, ext2;     // extents of the vertices in lattice coordinates (along s1 and s2)
 };
 
@@ -87,43 +94,74 @@ struct JKGroup {
   JKDev s[kJKGroup];
 };
 
-// Modal tables of one point: padded (mmax+2)^2 column-major, index (m,n) in -1..mmax.
+// Modal tables of one point: padded (mmax+2)^2 column-major, index (m,n) in -1..mmax, both
+// tables of a node side by side (entry e: t[2e] and t[2e + 1], one 32-byte sector).
 struct TableDev {
-  cd *t1, *t2;
+  cd *t;
   int mmax;
 };
 
-// Six-point interpolation of a padded table (PGF.jl:396-441).
-__device__ __forceinline__ cd sigma_interp(const cd *__restrict__ T, int mmax, const PointParams &P,
-                                           double rx, double ry) {
-  double x1o = (P.b1[0] * rx + P.b1[1] * ry) / PSS_TWOPI;
+// Both tables of one node by one 32-byte load.
+__device__ __forceinline__ void ld_node(const cd *p, double (&v)[4]) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
+// a / 2 pi, correctly rounded: quotient estimate and one fused correction with the correctly
+// rounded reciprocal (P. W. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119).  The rounding matters: the stencil
+// below is not continuous across its cells, and mesh offsets fall on cell boundaries.
+__device__ __forceinline__ double over_twopi(double a) {
+  constexpr double y = 1.0 / PSS_TWOPI;
+  const double q = a * y;
+  return fma(fma(-q, PSS_TWOPI, a), y, q);
+}
+
+// Six-point interpolation of both padded tables (PGF.jl:396-441) at offset (rx, ry); ph: the
+// phase factors cis(-(ms psi1 + ns psi2)) for ms, ns in -1..1 (null: no phasing).
+__device__ __forceinline__ void sigma_interp(const cd *__restrict__ T, int mmax, const PointParams &P, double rx,
+                                             double ry, const cd *__restrict__ ph, cd &s1, cd &s2) {
+  double x1o = over_twopi(P.b1[0] * rx + P.b1[1] * ry);
   if (fabs(x1o) < 1e-8) x1o = 0.0;
-  double x2o = (P.b2[0] * rx + P.b2[1] * ry) / PSS_TWOPI;
+  double x2o = over_twopi(P.b2[0] * rx + P.b2[1] * ry);
   if (fabs(x2o) < 1e-8) x2o = 0.0;
-  // Julia's mod(x, 1) in [0, 1]: x - floor(x) rounds once, exactly as fmod(x, 1) (exact)
-  // followed by + 1 for negative x, so the result is bit-identical and avoids fmod
-  const double x1 = x1o - floor(x1o), x2 = x2o - floor(x2o);
-  double ms = rint(x1o - x1), ns = rint(x2o - x2);
-  int m = (int)trunc(mmax * x1);
-  double p = mmax * x1 - m;
-  int n = (int)trunc(mmax * x2);
-  double q = mmax * x2 - n;
-  // x < 1 always, but mmax*x can round up to mmax; the stencil then must stay inside
-  // the padded table (same point, one cell to the left).
-  if (m >= mmax) { m = mmax - 1; p = mmax * x1 - m; }
-  if (n >= mmax) { n = mmax - 1; q = mmax * x2 - n; }
-  double p2 = p * p, q2 = q * q, pq = p * q;
+  // Julia's mod(x, 1) in [0, 1] is x - floor(x); the cell shift is floor(x)
+  const double ms = floor(x1o), ns = floor(x2o);
+  const double x1 = x1o - ms, x2 = x2o - ns;
+  int m = (int)(mmax * x1);
+  int n = (int)(mmax * x2);
+  // x <= 1, and mmax*x can round up to mmax; the stencil then must stay inside the padded
+  // table (same point, one cell to the left).
+  if (m >= mmax) m = mmax - 1;
+  if (n >= mmax) n = mmax - 1;
+  const double p = mmax * x1 - m, q = mmax * x2 - n;
+  const double p2 = p * p, q2 = q * q, pq = p * q;
   const int L = mmax + 2;
-#define TX(a, b) T[(size_t)((a) + 1) + (size_t)((b) + 1) * L]
-  cd s = (0.5 * (q2 - q)) * TX(m, n - 1);
-  s = s + (0.5 * (p2 - p)) * TX(m - 1, n);
-  s = s + (((1.0 + pq) - p2) - q2) * TX(m, n);
-  s = s + (0.5 * ((p2 - 2.0 * pq) + p)) * TX(m + 1, n);
-  s = s + (0.5 * ((q2 - 2.0 * pq) + q)) * TX(m, n + 1);
-  s = s + pq * TX(m + 1, n + 1);
-#undef TX
-  if (ms != 0.0 || ns != 0.0) s = s * cisd(-(ms * P.psi1 + ns * P.psi2));
-  return s;
+  const cd *c = T + 2 * ((size_t)(m + 1) + (size_t)(n + 1) * L);
+  const double w[6] = {0.5 * (q2 - q),  0.5 * (p2 - p),              ((1.0 + pq) - p2) - q2,
+                       0.5 * ((p2 - 2.0 * pq) + p), 0.5 * ((q2 - 2.0 * pq) + q), pq};
+  double v[6][4];
+  ld_node(c - 2 * L, v[0]);
+  ld_node(c - 2, v[1]);
+  ld_node(c, v[2]);
+  ld_node(c + 2, v[3]);
+  ld_node(c + 2 * L, v[4]);
+  ld_node(c + 2 * L + 2, v[5]);
+  double s[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    s[e] = w[0] * v[0][e];
+#pragma unroll
+    for (int k = 1; k < 6; ++k) s[e] = fma(w[k], v[k][e], s[e]);
+  }
+  s1 = mkcd(s[0], s[1]);
+  s2 = mkcd(s[2], s[3]);
+  if (ph) {
+    cd f;
+    if (fabs(ms) <= 1.0 && fabs(ns) <= 1.0) f = ph[((int)ms + 1) * 3 + (int)ns + 1];
+    else f = cisd(-(ms * P.psi1 + ns * P.psi2));
+    s1 = s1 * f;
+    s2 = s2 * f;
+  }
 }
 
 // The device a context runs on (0, or -1 for a null context with a message).
@@ -143,8 +181,7 @@ void pss_tables_ring_fill(const StackParams &S, const PointParams *dP, int npts,
 void pss_tables_ring_sums(const PointParams *dP, int npts, int R, const cd *dense, size_t point_stride,
                           double convtest, unsigned char *conv, cudaStream_t st);
 void pss_tables_find_mmax(int npts, int R, const unsigned char *conv, int *mmax, int *flag, cudaStream_t st);
-int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t1, cd *t2,
-                      cudaStream_t st);
+int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t, cudaStream_t st);
 size_t pss_table_cap(int mmax);  // (mmax+2)^2 entries per padded table
 
 // Face-pair integrals and matrix fill (pss_fill.cu)
@@ -166,8 +203,8 @@ bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const 
 size_t pss_jktab_bytes(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np);
 int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const double s1[2], const double s2[2],
                      const JKGroup &jk, int *nonconv, const JKTabPlan &P, void *ws, cudaStream_t st);
-void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const cd *t1, const cd *t2,
-                    int mmax, cd *zb, cudaStream_t st);
+void pss_fill_pairs(const SheetDev &G, const PointParams *dP1, const JKDev &jk, const TableDev &tab, cd *zb,
+                    cudaStream_t st);
 // Assemble Z (row-major): z64 with leading dimension ld, the FP32 planes (zr, zi) with ldf.
 // z64 and/or (zr, zi) may be null.
 void pss_fill_assemble(const SheetDev &G, const PointParams *dP1, const cd *zb, cd *z64, float *zr, float *zi,

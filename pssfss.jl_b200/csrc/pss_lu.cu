@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kPanelRows / RPT) k_panel(Mat<F32> M0, LuBatch
       const E p = prow[c];
 #pragma unroll
       for (int q = 0; q < RPT; ++q)
-        if (act[q]) R[c * kPanelRows + tid + q * T] = csubE(R[c * kPanelRows + tid + q * T], cmulE(l[q], p));
+        if (act[q]) R[c * kPanelRows + tid + q * T] = cmsub(R[c * kPanelRows + tid + q * T], l[q], p);
     }
   }
 #pragma unroll
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kSwpThreads) k_laswp(Mat<F32> M0, long long ms
 // broadcast by a shuffle); then the remaining rows take their rank-32 update from shared memory.
 // One launch per outer block replaces four 32-row solves and three updates of the rows between
 // them (with their operand splits): about 10 ms of launches, each too short to fill the chip, per
-// batch of 12 at N = 3976, now 4.1 ms (172 us at the first outer block).
+// batch of 12 at N = 3976, now 3.4 ms (143 us at the first outer block).
 template <bool F32>
 struct RowSolve {
   static constexpr int NB = F32 ? 128 : 64, COLS = F32 ? 64 : 32, S = 32, LP = S + 1;
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(256) k_rowsolve(Mat<F32> M0, long long ms, int
 #pragma unroll
         for (int i = j / T::LANES; i < T::NI; ++i) {
           const int r = p + T::LANES * i;
-          if (r > j && r < nc) x[i] = csubE(x[i], cmulE(L[r * T::LP + j], xj));
+          if (r > j && r < nc) x[i] = cmsub(x[i], L[r * T::LP + j], xj);
         }
       }
 #pragma unroll
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(256) k_rowsolve(Mat<F32> M0, long long ms, int
         if (i >= ni) break;
         const E l = L[min(T::S + ty + 16 * i, T::S + rem - 1) * T::LP + k];
 #pragma unroll
-        for (int q = 0; q < T::CQ; ++q) acc[i][q] = caddE(acc[i][q], cmulE(l, xv[q]));
+        for (int q = 0; q < T::CQ; ++q) acc[i][q] = cmac(acc[i][q], l, xv[q]);
       }
     }
 #pragma unroll

@@ -284,16 +284,16 @@ __device__ __forceinline__ cd pad_value(const cd *__restrict__ A, int mmax, cons
 }
 
 __global__ void k_phase_pad(const cd *__restrict__ a1, const cd *__restrict__ a2, int mmax,
-                            const PointParams *__restrict__ Pp, cd *__restrict__ t1, cd *__restrict__ t2) {
+                            const PointParams *__restrict__ Pp, cd *__restrict__ tab) {
   const int L = mmax + 2;
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)L * L) return;
   int a = (int)(t % L) - 1, b = (int)(t / L) - 1;
-  if (a == mmax && b == -1) { t1[t] = mkcd(0, 0); t2[t] = mkcd(0, 0); return; }  // unused corner
+  if (a == mmax && b == -1) { tab[2 * t] = tab[2 * t + 1] = mkcd(0, 0); return; }  // unused corner
   const PointParams &P = *Pp;
   double scale = P.magnetic ? P.area : 2.0 * P.area;
-  t1[t] = pad_value(a1, mmax, P, scale, a, b);
-  t2[t] = pad_value(a2, mmax, P, scale, a, b);
+  tab[2 * t] = pad_value(a1, mmax, P, scale, a, b);
+  tab[2 * t + 1] = pad_value(a2, mmax, P, scale, a, b);
 }
 
 // Radix sequence for n = 2^a 3^b 5^c: radix-4 stages first, then 5, 3 and a last 2.
@@ -343,8 +343,8 @@ void pss_tables_find_mmax(int npts, int R, const unsigned char *conv, int *mmax,
   k_find_mmax<<<cdiv_u(npts, 64), 64, 0, st>>>(npts, R, conv, mmax, flag);
 }
 
-// dense: this point's (2R+1)^2 x 2 tables; stage: >= 2*mmax^2 entries; t1/t2: (mmax+2)^2 each.
-int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t1, cd *t2,
+// dense: this point's (2R+1)^2 x 2 tables; stage: >= 2*mmax^2 entries; t: 2*(mmax+2)^2.
+int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t,
                       cudaStream_t st) {
   static DeviceOnce once;
   if (int rc = device_once(once, [] {
@@ -365,7 +365,7 @@ int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, 
   }
   long long L2 = (long long)(mmax + 2) * (mmax + 2);
   pss_count_launch();
-  k_phase_pad<<<cdiv_u(L2, 256), 256, 0, st>>>(a1, a2, mmax, dP1, t1, t2);
+  k_phase_pad<<<cdiv_u(L2, 256), 256, 0, st>>>(a1, a2, mmax, dP1, t);
   PSS_CUDA_TRY(cudaGetLastError());
   return 0;
 }

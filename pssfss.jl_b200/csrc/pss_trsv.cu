@@ -139,9 +139,7 @@ struct SolveT<true> {
   __device__ static C from(cd v) { return cf{(float)v.x, (float)v.y}; }
   __device__ static cd to(C v) { return mkcd(v.x, v.y); }
 };
-__device__ __forceinline__ cf operator+(cf a, cf b) { return cf{a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ cf operator-(cf a, cf b) { return cf{a.x - b.x, a.y - b.y}; }
-__device__ __forceinline__ cf operator*(cf a, cf b) { return cf{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
 template <class C>
 __device__ __forceinline__ C czero() { return C{0, 0}; }
 
@@ -244,7 +242,7 @@ __global__ void __launch_bounds__(256, F32 ? 2 : 1) k_trsv(Fac F0, int n, const 
 #pragma unroll
         for (int rr = 0; rr < 8; ++rr)
 #pragma unroll
-          for (int j = 0; j < NJ; ++j) a8[rr][j] = a8[rr][j] + lv[rr][h] * xv[h][j];
+          for (int j = 0; j < NJ; ++j) a8[rr][j] = cmac(a8[rr][j], lv[rr][h], xv[h][j]);
     }
 #pragma unroll
     for (int rr = 0; rr < 8; ++rr)
@@ -288,7 +286,7 @@ __global__ void __launch_bounds__(256, F32 ? 2 : 1) k_trsv(Fac F0, int n, const 
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[j] = acc[j] + lv[q] * xs[p * 16 + q][j];
+      for (int j = 0; j < NJ; ++j) acc[j] = cmac(acc[j], lv[q], xs[p * 16 + q][j]);
     }
   }
 #pragma unroll
@@ -312,7 +310,7 @@ __global__ void __launch_bounds__(256, F32 ? 2 : 1) k_trsv(Fac F0, int n, const 
     if (e < nr * nj) {
 #pragma unroll 4
       for (int k = part * 16; k < part * 16 + 16; ++k)
-        if (k < nr) s = s + Ds[r * BS + k] * y[k][j];
+        if (k < nr) s = cmac(s, Ds[r * BS + k], y[k][j]);
     }
     for (int o = 1; o < 4; o <<= 1) {
       s.x += __shfl_xor_sync(0xffffffff, s.x, o);
@@ -348,7 +346,7 @@ __global__ void __launch_bounds__(256) k_resid(int n, const cd *__restrict__ A0,
       for (int t = lane; t < n; t += 32) {
         cd av = a[t];
         if (j0 == 0) rs += cabs1(av);
-        for (int j = 0; j < nj; ++j) acc[j] = acc[j] + av * X[(size_t)(j0 + j) * n + t];
+        for (int j = 0; j < nj; ++j) acc[j] = cmac(acc[j], av, X[(size_t)(j0 + j) * n + t]);
       }
       for (int j = 0; j < nj; ++j)
         for (int o = 16; o > 0; o >>= 1) {
@@ -430,7 +428,7 @@ __global__ void __launch_bounds__(256) k_resid4(int n, const cd *__restrict__ A0
       for (int i = 0; i < kResRows; ++i) {
         rs[i] += cabs1(av[i]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = acc[i][j] + av[i] * xv[j];
+        for (int j = 0; j < 4; ++j) acc[i][j] = cmac(acc[i][j], av[i], xv[j]);
       }
     }
   }
