@@ -42,9 +42,9 @@ __device__ __forceinline__ cd ld_cd(const cd *p) {  // one 16-byte load
 // One thread per class.  Bound by its FP64 operations (about 1200) and the gathers of its 42
 // table nodes; what does not belong to the pair is prepared elsewhere: the point's coefficients
 // on the host, vertices in metres and centroids per face at the upload, the cell-shift phases
-// per CTA, both tables of a node in one 32-byte load.  613 -> 310 us for the 3.19M classes of the
+// per CTA, both tables of a node in one 32-byte load.  613 -> 291 us for the 3.19M classes of the
 // N = 3976 meander.
-__global__ void __launch_bounds__(128, 4) k_pairs(SheetDev G, const PointParams *__restrict__ Pp, JKDev jk,
+__global__ void __launch_bounds__(128, 5) k_pairs(SheetDev G, const PointParams *__restrict__ Pp, JKDev jk,
                                                const cd *__restrict__ tab, int mmax, cd *__restrict__ zb) {
   __shared__ PointParams P;
   __shared__ cd ph[9];
@@ -193,8 +193,8 @@ __device__ __forceinline__ cd assemble_entry(const SheetDev &G, const cd *ff, bo
 // match faces, so the class look-ups and most pair-term loads of a warp are contiguous); each
 // thread keeps its row's incidences and takes 8 columns (independent gathers in flight); the
 // tile then goes out through shared memory row by row, 64 consecutive entries per row.  Bound by
-// the gathers (4 class numbers and 4 pair terms per entry): 460 -> 369 us at N = 3976.
-__global__ void __launch_bounds__(256) k_assemble(SheetDev G, const PointParams *__restrict__ Pp,
+// the gathers (4 class numbers and 4 pair terms per entry): 460 -> 336 us at N = 3976.
+__global__ void __launch_bounds__(256, 3) k_assemble(SheetDev G, const PointParams *__restrict__ Pp,
                                                   const cd *__restrict__ zb, cd *__restrict__ z64,
                                                   float *__restrict__ zr, float *__restrict__ zi, long long ld,
                                                   long long ldf) {

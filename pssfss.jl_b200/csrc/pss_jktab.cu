@@ -22,8 +22,8 @@
 // bound by the FP64 pipe; this one issues about 400 and reads 64 nodes from L1/L2.  A pair's
 // eight lanes own one column of the panel each, so a node row is one 128-byte line, and a lane
 // keeps its column in registers while consecutive quadrature points stay in the panel.
-// Measured (direct -> tabulated, tables included): 17.6 -> 4.7 ms for the 3.19M classes of the
-// N = 3976 meander at normal incidence, 18.1 -> 6.3 ms for four phasings of a ring of 1168 faces.
+// Measured (direct -> tabulated, tables included): 17.6 -> 3.2 ms for the 3.19M classes of the
+// N = 3976 meander at normal incidence, 18.1 -> 4.7 ms for four phasings of a ring of 1168 faces.
 #include <algorithm>
 #include <cmath>
 
@@ -33,8 +33,8 @@ namespace {
 
 constexpr int kND = 8;                  // nodes per panel and direction
 constexpr int kSub = 32;                // sub-cells per panel and direction
-constexpr int kRec = 8;                 // rings 6 .. 6+kRec-1 a panel may stop at
 constexpr int kRMin = 6;                // first ring the reference tests
+constexpr int kRec = 9;                 // far sums recorded at a node: through rings kRMin - 1 .. 13
 constexpr double kConv = 1e-8;          // its threshold
 // How far a node (sub-cell corner) must be from the threshold |ring| = kConv |sum| to speak for
 // its surroundings: a share of |sum| for the slope, and an absolute part for the curvature of the
@@ -42,13 +42,13 @@ constexpr double kConv = 1e-8;          // its threshold
 constexpr double kMargin = 0.1, kCurve = 3e-3;
 constexpr double kSubMargin = 1e-4, kSubCurve = 4e-6;
 constexpr int kMaxPanels = 8192;
-constexpr int kMapSmem = 2 * (kSub + 1) * (kSub + 1) * (int)sizeof(cd);  // corner sums of a map's panel
 
 struct TabDev {
   double iv[4];           // u-scaled offset -> lattice coordinates
   double a0, b0, ra, rb;
   int na, nb;
   double *val[kJKGroup];          // [panel][R0 / R0+1][node a][J, K][node b] (real: one double each)
+  double *ring[kJKGroup];         // ring R0 alone at the nodes, laid out like one slot of val
   unsigned char *flag[kJKGroup];  // per panel: 0 whole, 1 map, 2 direct
   unsigned char *r0[kJKGroup];
   unsigned char *map[kJKGroup];   // [panel][kSub][kSub]
@@ -62,14 +62,18 @@ __constant__ double c_nodew[kND] = {3.121445152258054, -8.889123728313642, 13.30
                                     15.692564486451692, -13.303513796840717, 8.889123728313624, -3.121445152258053};
 
 // Sums at one offset, ring by ring as in jksums; the far part (rings >= 2) through each ring r
-// in 6 .. 13 is handed to rec.  Returns the ring the reference stops at (0: beyond the record),
+// in 5 .. 13 is handed to rec.  Returns the ring the reference stops at (0: beyond the record),
 // whether the test is clear of its threshold there (at) and one ring before (before), and the
 // sums.
+__device__ __forceinline__ bool clear_of(double ring, double sum, double margin, double curve, bool below) {
+  const double t = kConv * sum - ring, m = kConv * (margin * sum + curve);
+  return below ? t > m : t < -m;
+}
 template <bool REAL, class Rec>
 __device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, double us1y, double us2x, double us2y,
                                           const cd *__restrict__ ph1, const cd *__restrict__ ph2,
-                                          const double *__restrict__ etab, double margin, double curve, bool &at, bool &before,
-                                          cd &jsum, cd &ksum, Rec &&rec) {
+                                          const double *__restrict__ etab, bool &at, bool &before, cd &jsum, cd &ksum,
+                                          Rec &&rec) {
   const double arg = sqrt(urx * urx + ury * ury);
   const double rterm = exp_neg(arg, etab);
   ksum = mkcd(rterm, 0.0);
@@ -77,12 +81,10 @@ __device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, d
   cd jfar = mkcd(0, 0), kfar = jfar;
   int R = 0;
   at = before = true;
-  for (int r = 1; r < kRMin + kRec; ++r) {
+  for (int r = 1; r < kRMin - 1 + kRec; ++r) {
     cd jr = mkcd(0, 0), kr = jr;
-    for (int idx = 0; idx < 8 * r; ++idx) {
-      int m, n;
-      ring_mn(r, idx, m, n);
-      const double dx = urx - ((double)m * us1x + (double)n * us2x), dy = ury - ((double)m * us1y + (double)n * us2y);
+    auto summand = [&](int m, int n, double dm, double dn) {
+      const double dx = urx - (dm * us1x + dn * us2x), dy = ury - (dm * us1y + dn * us2y);
       const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
       if constexpr (REAL) {
         jr.x += er * ra;
@@ -92,21 +94,32 @@ __device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, d
         jr = jr + mkcd(er * f.x * ra, er * f.y * ra);
         kr = kr + mkcd(er * f.x, er * f.y);
       }
+    };
+    const double dr = (double)r;
+    double d = -dr;
+    for (int i = -r; i <= r; ++i, d += 1.0) {
+      summand(r, i, dr, d);
+      summand(-r, i, -dr, d);
+    }
+    d = 1.0 - dr;
+    for (int i = 1 - r; i < r; ++i, d += 1.0) {
+      summand(i, -r, d, -dr);
+      summand(i, r, d, dr);
     }
     if (r >= 2) { jfar = jfar + jr; kfar = kfar + kr; }
-    if (r >= kRMin) rec(r - kRMin, jfar, kfar);
+    if (r >= kRMin - 1) rec(r - (kRMin - 1), jfar, kfar);
     if (R) return R;  // one ring past R has been recorded
     jsum = jsum + jr;
     ksum = ksum + kr;
     if (r >= kRMin) {
-      const double aj = cabsd(jsum), ak = cabsd(ksum);
-      const double tj = kConv * aj - cabsd(jr), tk = kConv * ak - cabsd(kr);
-      const double mj = kConv * (margin * aj + curve), mk = kConv * (margin * ak + curve);
-      if (fmax(cabsd(jr / jsum), cabsd(kr / ksum)) < kConv) {
+      const double aj = cabsd(jsum), ak = cabsd(ksum), rj = cabsd(jr), rk = cabsd(kr);
+      const bool stop = fmax(cabsd(jr / jsum), cabsd(kr / ksum)) < kConv;
+      const bool cj = clear_of(rj, aj, kMargin, kCurve, stop), ck = clear_of(rk, ak, kMargin, kCurve, stop);
+      if (stop) {
         R = r;
-        at = tj > mj && tk > mk;
+        at = cj && ck;
       } else {
-        before = tj < -mj || tk < -mk;
+        before = cj || ck;
       }
     }
   }
@@ -147,8 +160,7 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
   bool at, before;
   cd js, ks;
   const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0],
-                                 etab, kMargin, kCurve, at, before, js, ks,
-                                 [&](int r, cd jf, cd kf) { rj[r][tid] = jf; rk[r][tid] = kf; });
+                                 etab, at, before, js, ks, [&](int r, cd jf, cd kf) { rj[r][tid] = jf; rk[r][tid] = kf; });
   if (tid == 0 || tid == 7 || tid == 56 || tid == 63) {
     corner[0][(tid & 1) + (tid >> 5) * 2] = js;
     corner[1][(tid & 1) + (tid >> 5) * 2] = ks;
@@ -164,7 +176,7 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
     T.flag[p][panel] = direct ? 2 : hi == lo ? 0 : 1;
     T.r0[p][panel] = (unsigned char)(direct ? kRMin : lo);
   }
-  const int r0 = direct ? 0 : lo - kRMin;
+  const int r0 = direct ? 1 : lo - (kRMin - 1);
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const cd J = rj[r0 + s][tid], K = rk[r0 + s][tid];
@@ -177,48 +189,14 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
       v[(i * 2 + 1) * 8 + j] = make_double2(K.x, K.y);
     }
   }
-}
-
-// Sub-cell maps of the panels that need one: the stopping ring at the 33 x 33 corners.
-template <bool REAL>
-__global__ void __launch_bounds__(256) k_jktab_map(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
-                                                   double us2y) {
-  __shared__ cd ph1[1][kPhase], ph2[1][kPhase];
-  __shared__ double etab[256];
-  constexpr int kCorners = (kSub + 1) * (kSub + 1);
-  __shared__ unsigned char cls[kCorners];
-  extern __shared__ __align__(16) unsigned char map_smem[];
-  cd *cj = (cd *)map_smem, *ck = cj + kCorners;
-  const int p = blockIdx.y, panel = blockIdx.x;
-  if (T.flag[p][panel] != 1) return;
-  PsiGroup one{};
-  one.n = 1;
-  one.psi1[0] = pg.psi1[p];
-  one.psi2[0] = pg.psi2[p];
-  fill_phases<1>(one, 1, ph1, ph2, etab);
-  __syncthreads();
-  const int r0 = T.r0[p][panel], ia = panel % T.na, ib = panel / T.na;
-  for (int e = threadIdx.x; e < (kSub + 1) * (kSub + 1); e += blockDim.x) {
-    const int i = e / (kSub + 1), j = e % (kSub + 1);
-    const double a = T.a0 + (ia + (double)i / kSub) / T.ra, b = T.b0 + (ib + (double)j / kSub) / T.rb;
-    bool at, before;
-    cd js, ks;
-    const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0],
-                                   etab, kSubMargin, kSubCurve, at, before, js, ks, [](int, cd, cd) {});
-    cls[e] = !at || !before || R < r0 || R > r0 + 1 ? 2 : R - r0;
-    cj[e] = js;
-    ck[e] = ks;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kSub * kSub; e += blockDim.x) {
-    const int e0 = e / kSub * (kSub + 1) + e % kSub;
-    const int c[4] = {e0, e0 + 1, e0 + kSub + 1, e0 + kSub + 2};
-    int v = cls[c[0]];
-    const cd j4[4] = {cj[c[0]], cj[c[1]], cj[c[2]], cj[c[3]]}, k4[4] = {ck[c[0]], ck[c[1]], ck[c[2]], ck[c[3]]};
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (cls[c[q]] != v || near_zero(j4[q], j4) || near_zero(k4[q], k4)) v = 2;
-    T.map[p][(size_t)panel * kSub * kSub + e] = (unsigned char)v;
+  // ring R0 itself, for the map
+  const cd J = rj[r0][tid] - rj[r0 - 1][tid], K = rk[r0][tid] - rk[r0 - 1][tid];
+  double2 *v = (double2 *)T.ring[p] + (size_t)panel * (REAL ? 64 : 128);
+  if constexpr (REAL) {
+    v[i * 8 + j] = make_double2(J.x, K.x);
+  } else {
+    v[(i * 2) * 8 + j] = make_double2(J.x, J.y);
+    v[(i * 2 + 1) * 8 + j] = make_double2(K.x, K.y);
   }
 }
 
@@ -238,7 +216,104 @@ __device__ __forceinline__ void basis8(double t, double s, double *out) {
   }
 }
 
+// Sub-cell maps of the panels that need one: the stopping ring at the 33 x 33 corners, from the
+// nearest images and the panel's own interpolants of the far sums (through R0 and R0 + 1) and of
+// ring R0: about 400 operations per corner, where summing the rings anew would take 5000.
+constexpr int kC = kSub + 1, kCorners = kC * kC;
+template <bool REAL>
+__global__ void __launch_bounds__(256) k_jktab_map(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
+                                                   double us2y) {
+  constexpr int W = REAL ? 6 : 12;  // reals per node: far R0 (J, K), far R0 + 1, ring R0
+  __shared__ double etab[256];
+  __shared__ cd fnear[9];
+  __shared__ double lag[kC][kND];
+  __shared__ double node[64][W];
+  __shared__ unsigned char cls[kCorners];
+  extern __shared__ __align__(16) unsigned char map_smem[];
+  cd *cj = (cd *)map_smem, *ck = cj + kCorners;
+  double *half = (double *)(ck + kCorners);  // [corner i][node j][W]
+  const int p = blockIdx.y, panel = blockIdx.x, tid = threadIdx.x;
+  if (T.flag[p][panel] != 1) return;
+  etab[tid] = exp2((double)tid / 256.0);
+  if (tid < 9) {
+    double s1, c1, s2, c2;
+    sincos(-((double)(tid / 3 - 1) * pg.psi1[p]), &s1, &c1);
+    sincos(-((double)(tid % 3 - 1) * pg.psi2[p]), &s2, &c2);
+    fnear[tid] = mkcd(c1, s1) * mkcd(c2, s2);
+  }
+  if (tid < kC) basis8(2.0 * tid / kSub - 1.0, 1.0, lag[tid]);
+  for (int e = tid; e < 64 * W; e += 256) {
+    // value w of node k = 8 i + j: slot w / (W / 3), then J and K (real and imaginary)
+    const int k = e / W, w = e % W, sl = w / (W / 3), c = w % (W / 3);
+    const double *v = sl < 2 ? T.val[p] + (size_t)(panel * 2 + sl) * 64 * (W / 3) : T.ring[p] + (size_t)panel * 64 * (W / 3);
+    node[k][w] = REAL ? v[k * 2 + c] : v[((k / 8 * 2 + c / 2) * 8 + k % 8) * 2 + c % 2];
+  }
+  __syncthreads();
+  for (int e = tid; e < kC * kND * W; e += 256) {
+    const int i = e / (kND * W), j = e / W % kND, w = e % W;
+    double s = 0;
+#pragma unroll
+    for (int k = 0; k < kND; ++k) s = fma(lag[i][k], node[k * 8 + j][w], s);
+    half[e] = s;
+  }
+  __syncthreads();
+  const int ia = panel % T.na, ib = panel / T.na;
+  for (int e = tid; e < kCorners; e += 256) {
+    const int i = e / kC, j = e % kC;
+    double v[12];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      double s = 0;
+#pragma unroll
+      for (int k = 0; k < kND; ++k) s = fma(lag[j][k], half[(i * kND + k) * W + w], s);
+      v[w] = s;
+    }
+    const double a = T.a0 + (ia + (double)i / kSub) / T.ra, b = T.b0 + (ib + (double)j / kSub) / T.rb;
+    const double ux = a * us1x + b * us2x, uy = a * us1y + b * us2y;
+    const double arg = sqrt(ux * ux + uy * uy), rterm = exp_neg(arg, etab);
+    cd js = mkcd(arg <= 1e-5 ? (-arg / 6 + 0.5) * arg - 1 : (rterm - 1) / arg, 0.0), ks = mkcd(rterm, 0.0);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      if (q == 4) continue;
+      const double m = q / 3 - 1, n = q % 3 - 1;
+      const double dx = ux - (m * us1x + n * us2x), dy = uy - (m * us1y + n * us2y);
+      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
+      const cd f = fnear[q];
+      js = js + mkcd(er * f.x * ra, er * f.y * ra);
+      ks = ks + mkcd(er * f.x, er * f.y);
+    }
+    auto val = [&](int k) { return REAL ? mkcd(v[k], 0.0) : mkcd(v[2 * k], v[2 * k + 1]); };  // (slot, J / K)
+    const cd j0 = js + val(0), k0 = ks + val(1), j1 = js + val(2), k1 = ks + val(3);
+    const double a0 = cabsd(j0), b0 = cabsd(k0), r0 = cabsd(val(4)), s0 = cabsd(val(5));
+    int c = 2;
+    if (clear_of(r0, a0, kSubMargin, kSubCurve, true) && clear_of(s0, b0, kSubMargin, kSubCurve, true)) {
+      c = 0;
+    } else if (clear_of(r0, a0, kSubMargin, kSubCurve, false) || clear_of(s0, b0, kSubMargin, kSubCurve, false)) {
+      const double r1 = cabsd(val(2) - val(0)), s1 = cabsd(val(3) - val(1));
+      if (clear_of(r1, cabsd(j1), kSubMargin, kSubCurve, true) && clear_of(s1, cabsd(k1), kSubMargin, kSubCurve, true)) c = 1;
+    }
+    cls[e] = (unsigned char)c;
+    cj[e] = c == 0 ? j0 : j1;
+    ck[e] = c == 0 ? k0 : k1;
+  }
+  __syncthreads();
+  for (int e = tid; e < kSub * kSub; e += 256) {
+    const int e0 = e / kSub * kC + e % kSub;
+    const int c[4] = {e0, e0 + 1, e0 + kC, e0 + kC + 1};
+    int v = cls[c[0]];
+    const cd j4[4] = {cj[c[0]], cj[c[1]], cj[c[2]], cj[c[3]]}, k4[4] = {ck[c[0]], ck[c[1]], ck[c[2]], ck[c[3]]};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (cls[c[q]] != v || near_zero(j4[q], j4) || near_zero(k4[q], k4)) v = 2;
+    T.map[p][(size_t)panel * kSub * kSub + e] = (unsigned char)v;
+  }
+}
+constexpr int kMapSmem = 2 * kCorners * (int)sizeof(cd) + kC * kND * 12 * (int)sizeof(double);
+
 constexpr int kTabThreads = 128;
+// The seven points in a walk around the triangle (vertex, midpoint, ..., centroid): neighbours
+// share a panel more often than in the rule's order.
+__host__ __device__ constexpr int walk(int t) { return t == 0 ? 3 : t == 1 ? 4 : t == 2 ? 2 : t == 3 ? 6 : t == 4 ? 1 : t == 5 ? 5 : 0; }
 constexpr int kBasStride = 7 * 2 * kND + 2;  // doubles per pair: the four pairs of a warp on different banks
 
 // Eight lanes per face pair.  Lane q < 7 owns quadrature point q: its nearest images (rings 0
@@ -246,12 +321,15 @@ constexpr int kBasStride = 7 * 2 * kND + 2;  // doubles per pair: the four pairs
 // lanes through shared memory.  Then every lane j sums its column j of the panel for all seven
 // points into the six moments; a reduce-scatter over the eight lanes leaves moment k in lane k.
 template <int NP, bool REAL>
-__global__ void __launch_bounds__(kTabThreads, 4) k_filljk_tab(SheetDev G, double ul, PsiGroup pg, double us1x,
+__global__ void __launch_bounds__(kTabThreads, REAL ? 8 : 4) k_filljk_tab(SheetDev G, double ul, PsiGroup pg, double us1x,
                                                                double us1y, double us2x, double us2y, TabDev T,
                                                                JKGroup jk) {
   __shared__ cd fnear[NP][9];
   __shared__ double etab[256];
   __shared__ __align__(16) double bas[kTabThreads / 8][kBasStride];
+  // a group's near sums wait in shared memory for their phasing's turn (registers limit the CTAs
+  // per SM)
+  __shared__ double2 near_sum[NP == 1 ? 1 : NP][2][NP == 1 ? 1 : kTabThreads];
   const int np = NP == 1 ? 1 : pg.n;
   for (int t = threadIdx.x; t < 256; t += blockDim.x) etab[t] = exp2((double)t / 256.0);
   for (int t = threadIdx.x; t < NP * 9; t += blockDim.x) {
@@ -299,6 +377,10 @@ __global__ void __launch_bounds__(kTabThreads, 4) k_filljk_tab(SheetDev G, doubl
     for (int p = 0; p < NP; ++p) {
       js[p].x += j0;
       ks[p].x += rterm;
+      if constexpr (NP > 1) {
+        near_sum[p][0][threadIdx.x] = make_double2(js[p].x, js[p].y);
+        near_sum[p][1][threadIdx.x] = make_double2(ks[p].x, ks[p].y);
+      }
     }
   }
   // panel and sub-cell of this point; bases (the quadrature weight goes into the second one)
@@ -331,27 +413,33 @@ __global__ void __launch_bounds__(kTabThreads, 4) k_filljk_tab(SheetDev G, doubl
     const unsigned direct = __ballot_sync(0xffffffffu, state == 2 && q < 7) & (0xffu << grp);
     const int slot = panel * 2 + (state == 1 ? 1 : 0);
     // near part of the moments: lane q's own point
-    cd jn = mkcd(0, 0), kn = jn;
+    cd jn, kn;
+    if constexpr (NP == 1) {
+      jn = js[0];
+      kn = ks[0];
+    } else {
+      const double2 a = near_sum[p][0][threadIdx.x], b = near_sum[p][1][threadIdx.x];
+      jn = mkcd(a.x, a.y);
+      kn = mkcd(b.x, b.y);
+    }
+    const JKDev &o = jk.s[p];
+    if constexpr (REAL) {
+      // J and K together: one double2 per node
+      double acc[6] = {qw * jn.x, qx * (qw * jn.x), qe * (qw * jn.x), qw * kn.x, qx * (qw * kn.x), qe * (qw * kn.x)};
+      double2 row[kND];
+      int held = -1;
+      const double2 *val = (const double2 *)T.val[p] + q;
 #pragma unroll
-    for (int t = 0; t < NP; ++t)
-      if (t == p) { jn = js[t]; kn = ks[t]; }
-    jn = qw * jn;
-    kn = qw * kn;
-    cd acc[6] = {jn, qx * jn, qe * jn, kn, qx * kn, qe * kn};
-    double2 row[REAL ? kND : 2 * kND];
-    int held = -1;
-    const double2 *val = (const double2 *)T.val[p] + q;
+      for (int w = 0; w < 7; ++w) {
+        const int t = walk(w);
+        const int s = __shfl_sync(0xffffffffu, slot, grp + t);
+        if (s != held) {
+          held = s;
 #pragma unroll
-    for (int t = 0; t < 7; ++t) {
-      const int s = __shfl_sync(0xffffffffu, slot, grp + t);
-      if (s != held) {
-        held = s;
-#pragma unroll
-        for (int i = 0; i < (REAL ? kND : 2 * kND); ++i) row[i] = __ldg(val + (size_t)s * (REAL ? 64 : 128) + i * 8);
-      }
-      const double2 *lx = (const double2 *)(mybas + t * 2 * kND);
-      const double ly = mybas[t * 2 * kND + kND + q];
-      if constexpr (REAL) {
+          for (int i = 0; i < kND; ++i) row[i] = __ldg(val + (size_t)s * 64 + i * 8);
+        }
+        const double2 *lx = (const double2 *)(mybas + t * 2 * kND);
+        const double ly = mybas[t * 2 * kND + kND + q];
         double jv = 0, kv = 0;
 #pragma unroll
         for (int i = 0; i < kND; i += 2) {
@@ -361,67 +449,88 @@ __global__ void __launch_bounds__(kTabThreads, 4) k_filljk_tab(SheetDev G, doubl
         }
         jv *= ly;
         kv *= ly;
-        acc[0].x += jv;
-        acc[1].x = fma(c_qxi[t], jv, acc[1].x);
-        acc[2].x = fma(c_qeta[t], jv, acc[2].x);
-        acc[3].x += kv;
-        acc[4].x = fma(c_qxi[t], kv, acc[4].x);
-        acc[5].x = fma(c_qeta[t], kv, acc[5].x);
-      } else {
-        cd jv = mkcd(0, 0), kv = jv;
+        acc[0] += jv;
+        acc[1] = fma(c_qxi[t], jv, acc[1]);
+        acc[2] = fma(c_qeta[t], jv, acc[2]);
+        acc[3] += kv;
+        acc[4] = fma(c_qxi[t], kv, acc[4]);
+        acc[5] = fma(c_qeta[t], kv, acc[5]);
+      }
+      // reduce-scatter over the eight lanes: lane k ends with moment k (lanes 6 and 7 with none)
+      const bool b4 = q & 4, b2 = q & 2, b1 = q & 1;
+      double h[4], h2[2];
 #pragma unroll
-        for (int i = 0; i < kND; i += 2) {
-          const double2 l = lx[i / 2];
-          jv.x = fma(l.x, row[2 * i].x, fma(l.y, row[2 * i + 2].x, jv.x));
-          jv.y = fma(l.x, row[2 * i].y, fma(l.y, row[2 * i + 2].y, jv.y));
-          kv.x = fma(l.x, row[2 * i + 1].x, fma(l.y, row[2 * i + 3].x, kv.x));
-          kv.y = fma(l.x, row[2 * i + 1].y, fma(l.y, row[2 * i + 3].y, kv.y));
+      for (int k = 0; k < 4; ++k) {
+        const double hi = k < 2 ? acc[4 + k] : 0.0;
+        h[k] = (b4 ? hi : acc[k]) + __shfl_xor_sync(0xffffffffu, b4 ? acc[k] : hi, 4);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        h2[k] = (b2 ? h[2 + k] : h[k]) + __shfl_xor_sync(0xffffffffu, b2 ? h[k] : h[2 + k], 2);
+      const cd out = mkcd((b1 ? h2[1] : h2[0]) + __shfl_xor_sync(0xffffffffu, b1 ? h2[0] : h2[1], 1), 0.0);
+      if (live) {
+        if (q == 0) o.J[iu] = out;
+        else if (q == 1) o.Jxi[iu] = out;
+        else if (q == 2) o.Jeta[iu] = out;
+        else if (q == 3) o.K[iu] = out;
+        else if (q == 4) o.Kxi[iu] = out;
+        else if (q == 5) o.Keta[iu] = out;
+      }
+    } else {
+      // J, then K: half the registers of both at once
+#pragma unroll 1
+      for (int hk = 0; hk < 2; ++hk) {
+        const cd own = qw * (hk ? kn : jn);
+        cd acc[3] = {own, qx * own, qe * own};
+        double2 row[kND];
+        int held = -1;
+        const double2 *val = (const double2 *)T.val[p] + hk * 8 + q;
+#pragma unroll
+        for (int w = 0; w < 7; ++w) {
+          const int t = walk(w);
+          const int s = __shfl_sync(0xffffffffu, slot, grp + t);
+          if (s != held) {
+            held = s;
+#pragma unroll
+            for (int i = 0; i < kND; ++i) row[i] = __ldg(val + (size_t)s * 128 + i * 16);
+          }
+          const double2 *lx = (const double2 *)(mybas + t * 2 * kND);
+          const double ly = mybas[t * 2 * kND + kND + q];
+          cd v = mkcd(0, 0);
+#pragma unroll
+          for (int i = 0; i < kND; i += 2) {
+            const double2 l = lx[i / 2];
+            v.x = fma(l.x, row[i].x, fma(l.y, row[i + 1].x, v.x));
+            v.y = fma(l.x, row[i].y, fma(l.y, row[i + 1].y, v.y));
+          }
+          v = ly * v;
+          acc[0] = acc[0] + v;
+          acc[1] = mkcd(fma(c_qxi[t], v.x, acc[1].x), fma(c_qxi[t], v.y, acc[1].y));
+          acc[2] = mkcd(fma(c_qeta[t], v.x, acc[2].x), fma(c_qeta[t], v.y, acc[2].y));
         }
-        jv = ly * jv;
-        kv = ly * kv;
-        acc[0] = acc[0] + jv;
-        acc[1] = acc[1] + c_qxi[t] * jv;
-        acc[2] = acc[2] + c_qeta[t] * jv;
-        acc[3] = acc[3] + kv;
-        acc[4] = acc[4] + c_qxi[t] * kv;
-        acc[5] = acc[5] + c_qeta[t] * kv;
+        // reduce-scatter: lanes 0, 2 and 4 end with moments 0, 1 and 2
+        const bool b4 = q & 4, b2 = q & 2;
+        cd h[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const cd hi = k == 0 ? acc[2] : mkcd(0, 0), keep = b4 ? hi : acc[k], send = b4 ? acc[k] : hi;
+          h[k] = mkcd(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 4), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 4));
+        }
+        const cd keep = b2 ? h[1] : h[0], send = b2 ? h[0] : h[1];
+        cd out = mkcd(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 2), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 2));
+        out = mkcd(out.x + __shfl_xor_sync(0xffffffffu, out.x, 1), out.y + __shfl_xor_sync(0xffffffffu, out.y, 1));
+        if (live) {
+          if (q == 0) (hk ? o.K : o.J)[iu] = out;
+          else if (q == 2) (hk ? o.Kxi : o.Jxi)[iu] = out;
+          else if (q == 4) (hk ? o.Keta : o.Jeta)[iu] = out;
+        }
       }
     }
-    // reduce-scatter over the eight lanes: lane k ends with moment k (lanes 6 and 7 with none)
-    const bool b4 = q & 4, b2 = q & 2, b1 = q & 1;
-    cd h[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const cd keep = b4 ? (k < 2 ? acc[4 + k] : mkcd(0, 0)) : acc[k];
-      const cd send = b4 ? acc[k] : (k < 2 ? acc[4 + k] : mkcd(0, 0));
-      h[k].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 4);
-      h[k].y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 4);
-    }
-    cd h2[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const cd keep = b2 ? h[2 + k] : h[k], send = b2 ? h[k] : h[2 + k];
-      h2[k].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 2);
-      h2[k].y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 2);
-    }
-    cd out;
-    {
-      const cd keep = b1 ? h2[1] : h2[0], send = b1 ? h2[0] : h2[1];
-      out.x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 1);
-      out.y = REAL ? 0.0 : keep.y + __shfl_xor_sync(0xffffffffu, send.y, 1);
-    }
     if (!live) continue;
-    const JKDev &o = jk.s[p];
-    if (q == 0) o.J[iu] = out;
-    else if (q == 1) o.Jxi[iu] = out;
-    else if (q == 2) o.Jeta[iu] = out;
-    else if (q == 3) o.K[iu] = out;
-    else if (q == 4) o.Kxi[iu] = out;
-    else if (q == 5) o.Keta[iu] = out;
-    else if (q == 6) {
+    if (q == 6) {
       o.rho_r[2 * iu] = rr0;
       o.rho_r[2 * iu + 1] = rr1;
-    } else {
+    } else if (q == 7) {
       o.rinv[iu] = ri;
       if (direct) T.list[(size_t)p * G.nufp + atomicAdd(T.count + p, 1)] = iu;
     }
@@ -496,7 +605,7 @@ bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const 
   P.b0 = -W2;
   P.ra = P.na / (2 * W1);
   P.rb = P.nb / (2 * W2);
-  const size_t per = align256(panels * 2 * 64 * 4 * sizeof(double)) + 2 * align256(panels) + align256(panels * kSub * kSub);
+  const size_t per = align256(panels * 3 * 64 * 4 * sizeof(double)) + 2 * align256(panels) + align256(panels * kSub * kSub);
   P.bytes = (size_t)np * (per + (size_t)G.nufp * sizeof(int)) + 512;
   return true;
 }
@@ -517,7 +626,9 @@ int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const
   T.a0 = P.a0; T.b0 = P.b0; T.ra = P.ra; T.rb = P.rb; T.na = P.na; T.nb = P.nb;
   char *w = (char *)(((uintptr_t)ws + 255) & ~(uintptr_t)255);
   for (int p = 0; p < np; ++p) {
-    T.val[p] = (double *)w; w += align256(panels * 2 * 64 * 4 * sizeof(double));
+    T.val[p] = (double *)w;
+    T.ring[p] = T.val[p] + panels * 2 * 64 * 4;
+    w += align256(panels * 3 * 64 * 4 * sizeof(double));
     T.flag[p] = (unsigned char *)w; w += align256(panels);
     T.r0[p] = (unsigned char *)w; w += align256(panels);
     T.map[p] = (unsigned char *)w; w += align256(panels * kSub * kSub);
@@ -528,6 +639,13 @@ int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const
   const bool real = np == 1 && pg.psi1[0] == 0.0 && pg.psi2[0] == 0.0;
   const dim3 gp((unsigned)panels, np);
   const unsigned gt = cdiv_u((long long)G.nufp * 8, kTabThreads);
+  static DeviceOnce once;
+  if (int rc = device_once(once, [] {
+        PSS_CUDA_TRY(cudaFuncSetAttribute(k_jktab_map<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMapSmem));
+        PSS_CUDA_TRY(cudaFuncSetAttribute(k_jktab_map<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMapSmem));
+        return 0;
+      }))
+    return rc;
   for (int k = 0; k < 4; ++k) pss_count_launch();
   if (real) {
     k_jktab_nodes<true><<<gp, 64, 0, st>>>(T, pg, a, b, c, d);
