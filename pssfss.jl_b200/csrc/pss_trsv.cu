@@ -7,8 +7,9 @@
 // taken in start order (atomicAdd), CTA b solves block b and only waits (bounded spin on
 // a per-block epoch flag) for blocks that started before it, so it never waits on a CTA
 // that is not resident.  Every CTA streams its share of the triangle (the bulk of the
-// bytes) concurrently; the serial chain per block is one 64x64 product with the
-// precomputed inverse of the diagonal block.  FP64 arithmetic for FP32 or FP64 factors.
+// bytes) concurrently; the serial chain per block is the product with its predecessor's tile
+// and the one with the precomputed inverse of the diagonal block.  FP32 arithmetic for FP32
+// factors, FP64 for FP64 factors.
 //
 // Refinement (LAPACK zcgesv's scheme): r = b - A x with the FP64 matrix, stop when
 // max|r_j| <= max|x_j| * ||A||_inf * eps * sqrt(n) for every rhs j (cabs1 norms).
@@ -18,7 +19,8 @@
 namespace {
 
 constexpr int BS = 64;        // block rows
-constexpr int kMaxRhs = 8;    // right-hand sides per pass
+constexpr int NJ = 4;         // right-hand sides of one chain
+constexpr int kChains = 16;   // chains (groups of NJ right-hand sides) of a matrix in one launch
 constexpr int kMaxRefRhs = 1024;          // right-hand sides of one refinement
 constexpr int kNX = kMaxRefRhs;           // norms layout: [max|r_j|] [max|x_j|] [||A||]
 constexpr int kNA = 2 * kMaxRefRhs;
@@ -39,7 +41,8 @@ struct Fac {  // row-major factor access: FP64 interleaved or FP32 planes
   }
 };
 
-// Per-matrix control words of a batch: [0] ticket, [1] error, [2] converged, [8..] flags.
+// Per-matrix control words of a batch: [1] error, [2] converged; from word 8 on, for each of up
+// to kChains chains, its ticket and its blocks' flags.
 struct Ctrl {
   int *base;
   int stride;
@@ -75,35 +78,57 @@ __device__ __forceinline__ void post_flag(int *flags, int b, int epoch) {
 }
 
 // Inverses of the 64x64 diagonal blocks: Dinv[(2*blk + 0)] = L_bb^{-1} (unit lower),
-// Dinv[(2*blk + 1)] = U_bb^{-1}; each 64x64 row-major FP64.
-__global__ void __launch_bounds__(64) k_diag_inv(Fac F0, int n, cd *Dinv0, long long dstride) {
+// Dinv[(2*blk + 1)] = U_bb^{-1}; each 64x64 row-major FP64.  Four lanes per column of the inverse,
+// each with 16 interleaved rows in registers; a finished entry goes to the other three by a
+// shuffle and the rows still open take it off at once (the one-thread-per-column form, a chain of
+// 64 dot products with both matrices in shared memory, took 1130 us for 12 factors of N = 3976).
+__global__ void __launch_bounds__(256) k_diag_inv(Fac F0, int n, cd *Dinv0, long long dstride) {
   const int blk = blockIdx.x, upper = blockIdx.y;
   const Fac F = F0.of(blockIdx.z);
-  cd *Dinv = Dinv0 + blockIdx.z * dstride;
   const int r0 = blk * BS, nb = min(BS, n - r0);
-  extern __shared__ cd sm[];
-  cd *T = sm;            // 64 x 64 block
-  cd *X = sm + BS * BS;  // 64 x 64 inverse, column k owned by thread k
-  const int k = threadIdx.x;
-  for (int i = 0; i < BS; ++i) T[i * BS + k] = (i < nb && k < nb) ? F.at(r0 + i, r0 + k) : mkcd(i == k, 0);
-  __syncthreads();
-  if (!upper) {
-    for (int i = 0; i < BS; ++i) {
-      cd v = mkcd(i == k, 0);
-      for (int t = k; t < i; ++t) v = v - T[i * BS + t] * X[t * BS + k];
-      X[i * BS + k] = (i < k) ? mkcd(0, 0) : v;
-    }
-  } else {
-    for (int i = BS - 1; i >= 0; --i) {
-      cd v = mkcd(i == k, 0);
-      for (int t = i + 1; t <= k; ++t) v = v - T[i * BS + t] * X[t * BS + k];
-      X[i * BS + k] = (i > k) ? mkcd(0, 0) : v / T[i * BS + i];
-    }
+  constexpr int LD = BS + 1;
+  extern __shared__ __align__(16) unsigned char dinv_smem[];
+  cd *T = (cd *)dinv_smem;  // 64 rows of LD
+  __shared__ cd rdiag[BS];
+  const int tid = threadIdx.x;
+  for (int e = tid; e < BS * BS; e += 256) {
+    const int i = e / BS, k = e % BS;
+    T[i * LD + k] = (i < nb && k < nb) ? F.at(r0 + i, r0 + k) : mkcd(i == k, 0);
   }
   __syncthreads();
-  cd *D = Dinv + (size_t)(2 * blk + upper) * BS * BS;
-  for (int i = 0; i < BS; ++i) D[i * BS + k] = X[i * BS + k];
+  if (upper && tid < BS) rdiag[tid] = mkcd(1.0, 0.0) / T[tid * LD + tid];
+  __syncthreads();
+  const int k = tid >> 2, p = tid & 3;  // column k, rows p + 4 i
+  cd x[BS / 4];
+#pragma unroll
+  for (int i = 0; i < BS / 4; ++i) x[i] = mkcd(p + 4 * i == k, 0);
+  if (!upper) {
+#pragma unroll
+    for (int j = 0; j < BS - 1; ++j) {
+      cd v;
+      v.x = __shfl_sync(0xffffffffu, x[j / 4].x, j % 4, 4);
+      v.y = __shfl_sync(0xffffffffu, x[j / 4].y, j % 4, 4);
+#pragma unroll
+      for (int i = j / 4; i < BS / 4; ++i)
+        if (p + 4 * i > j) x[i] = cmsub(x[i], T[(p + 4 * i) * LD + j], v);
+    }
+  } else {
+#pragma unroll
+    for (int j = BS - 1; j >= 0; --j) {
+      if (p == j % 4) x[j / 4] = x[j / 4] * rdiag[j];
+      cd v;
+      v.x = __shfl_sync(0xffffffffu, x[j / 4].x, j % 4, 4);
+      v.y = __shfl_sync(0xffffffffu, x[j / 4].y, j % 4, 4);
+#pragma unroll
+      for (int i = 0; i <= j / 4; ++i)
+        if (p + 4 * i < j) x[i] = cmsub(x[i], T[(p + 4 * i) * LD + j], v);
+    }
+  }
+  cd *D = Dinv0 + blockIdx.z * dstride + (size_t)(2 * blk + upper) * BS * BS;
+#pragma unroll
+  for (int i = 0; i < BS / 4; ++i) D[(p + 4 * i) * BS + k] = x[i];
 }
+constexpr int kDinvSmem = BS * (BS + 1) * (int)sizeof(cd);
 
 // perm[i] = original row that ends in position i after the LAPACK swap sequence ipiv.
 __global__ void __launch_bounds__(1024) k_ipiv_to_perm(int n, const int *ipiv0, int *perm0) {
@@ -143,274 +168,289 @@ __device__ __forceinline__ cf operator-(cf a, cf b) { return cf{a.x - b.x, a.y -
 template <class C>
 __device__ __forceinline__ C czero() { return C{0, 0}; }
 
-// One chained substitution pass over right-hand sides j0 .. j0+nj-1 (nj <= NJ):
+// One chained substitution pass, a chain of NJ right-hand sides per (matrix, chain) of the grid:
 //   lower: X[rows_b] = Linv_b (B[perm[rows_b]] - sum_{c<b} L[b,c] X[c])
 //   upper: X[rows_b] = Uinv_b (X[rows_b] - sum_{c>b} U[b,c] X[c])   (in place)
 // TRANS (the adjoint system Z^T y = b, Z = P^T L U, so U^T L^T (P y) = b): the lower pass
 // runs with U^T (block (b, c) read as the transpose of block (c, b) of the factor, the
 // diagonal inverse transposed) on B unpermuted, the upper pass with L^T in place; the
 // caller applies P^T to the result (pss_solve_lu_trans).
-// One CTA per 64-row block b (ticket order), 256 threads: row i = tid/4 of the block,
-// quarter p = tid%4 covers 16 columns of each 64-column tile.  Each tile of the factor is
-// loaded into registers BEFORE the wait for the CTA that produces x_c, so the wait hides
-// the load; Dinv_b (dynamic shared memory) and the block's right-hand side are staged at
-// the start.  Blocks of X written by other CTAs are read with L1-bypassing loads.
-template <bool LOWER, bool F32, int NJ, bool TRANS = false>
-__global__ void __launch_bounds__(256, F32 ? 2 : 1) k_trsv(Fac F0, int n, const int *__restrict__ perm0, const cd *__restrict__ B0,
-                                              cd *__restrict__ X0, long long vs, int nrhs, int j0,
-                                              const cd *__restrict__ Dinv0, long long dstride, Ctrl ctrl, int epoch,
-                                              int use_done) {
-  using T = SolveT<F32>;
-  using C = typename T::C;
-  // matrix of the batch: the grid runs matrix-fastest, so the CTAs start block row by block
-  // row across all matrices and every matrix's chain advances in the same waves
-  const int bm = blockIdx.x;
+//
+// One CTA per 64-row block b (ticket order).  The blocks of a chain finish one after another, so
+// what a step takes between its predecessor's flag and its own is the pass's time (63 steps at
+// N = 3976); everything else happens before that flag:
+//   * the tiles of all blocks but the predecessor's: a warp reads whole 128-byte row segments,
+//     looks up 32 flags at a time, and its partial sums are reduced across the CTA before the
+//     last wait;
+//   * the predecessor's tile waits in registers, the diagonal inverse in shared memory.
+// After the flag: x of the predecessor to shared memory, one 64 x 64 product from registers, one
+// with the inverse, the result and the flag.  The release of the flag after the block barrier
+// orders the block's stores; no further fence is needed.  660 -> 300 us per triangle of a batch of factors
+// (N = 3976, four right-hand sides, FP32).  Chains of more right-hand sides run side by side.
+template <bool F32>
+struct TrsvT {
+  static constexpr int T = F32 ? 256 : 512;    // threads
+  static constexpr int RW = 64 / (T / 32);     // tile rows of a warp
+  static constexpr int Q = T / 64;             // lanes of a row in the predecessor's product
+  static constexpr int LD = BS + 1;
+  using C = typename SolveT<F32>::C;
+  static constexpr int SMEM = BS * LD * (int)sizeof(C);                            // diagonal inverse
+  static constexpr int SMEM_T = SMEM + T / 32 * BS * NJ * (int)sizeof(C);          // + the warps' sums (TRANS)
+};
+template <bool LOWER, bool F32, bool TRANS>
+__global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
+    k_trsv(Fac F0, int n, const int *__restrict__ perm0, const cd *__restrict__ B0, cd *__restrict__ X0, long long vs,
+           int nrhs, int j00, int nchain, const cd *__restrict__ Dinv0, long long dstride, Ctrl ctrl, int epoch,
+           int use_done) {
+  using S = SolveT<F32>;
+  using P = TrsvT<F32>;
+  using C = typename S::C;
+  // the grid runs (matrix, chain) fastest, so the CTAs start block row by block row across all of
+  // them and every chain advances in the same waves
+  const int bm = blockIdx.x / nchain, ch = blockIdx.x % nchain;
   int *cw = ctrl.of(bm);
   if (use_done && cw[2]) return;
   const Fac F = F0.of(bm);
   const int *perm = perm0 + (long long)bm * n;
-  const cd *B = B0 + bm * vs;
-  cd *X = X0 + bm * vs;
-  const cd *Dinv = Dinv0 + bm * dstride;
-  int *ticket = cw, *err = cw + 1, *flags = cw + 8;
+  const int j0 = j00 + ch * NJ, nj = min(NJ, nrhs - j0);
+  const cd *B = B0 + bm * vs + (size_t)j0 * n;
+  cd *X = X0 + bm * vs + (size_t)j0 * n;
+  const int nblk = (n + BS - 1) / BS;
+  int *ticket = cw + 8 + ch * (nblk + 1), *flags = ticket + 1, *err = cw + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  C *Ds = (C *)smraw;  // BS x BS, row-major
+  C *Ds = (C *)smraw;
+  C *part = Ds + BS * P::LD;  // TRANS: [warp][64][NJ]
   __shared__ C y[BS][NJ];
   __shared__ C xs[BS][NJ];
+  __shared__ C xw[P::T / 32][P::RW][NJ];
   __shared__ int s_b;
-  const int tid = threadIdx.x;
-  const int i = tid >> 2, p = tid & 3;
-  const int nblk = (n + BS - 1) / BS;
-  const int nj = min(NJ, nrhs - j0);
-  if (tid == 0) s_b = atomicAdd(ticket, 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    const int t = atomicAdd(ticket, 1);
+    if (t == nblk - 1) *ticket = 0;  // every block has its ticket: ready for the next launch
+    s_b = t;
+  }
   __syncthreads();
-  const int tk = s_b;
-  const int b = LOWER ? tk : nblk - 1 - tk;
+  const int b = LOWER ? s_b : nblk - 1 - s_b;
   const int r0 = b * BS, nr = min(BS, n - r0);
   // diagonal block: L_bb^-1 (lower pass) or U_bb^-1 (upper pass); transposed, U_bb^-T for the
   // lower pass of the adjoint system and L_bb^-T for its upper pass
-  const cd *D = Dinv + (size_t)(2 * b + ((LOWER != TRANS) ? 0 : 1)) * BS * BS;
-  for (int e = tid; e < BS * BS; e += 256) Ds[e] = T::from(TRANS ? D[(e % BS) * BS + e / BS] : D[e]);
-  for (int e = tid; e < BS * NJ; e += 256) {
-    const int r = e / NJ, j = e % NJ;
+  const cd *D = Dinv0 + bm * dstride + (size_t)(2 * b + ((LOWER != TRANS) ? 0 : 1)) * BS * BS;
+  for (int e = tid; e < BS * BS; e += P::T) {
+    const int r = e / BS, c = e % BS;
+    if constexpr (TRANS) Ds[c * P::LD + r] = S::from(D[e]);
+    else Ds[r * P::LD + c] = S::from(D[e]);
+  }
+  if (tid < BS * NJ) {
+    const int r = tid / NJ, j = tid % NJ;
     cd v = mkcd(0, 0);
     if (r < nr && j < nj)
-      v = LOWER ? B[(size_t)(j0 + j) * n + (TRANS ? r0 + r : perm[r0 + r])] : ldcg(&X[(size_t)(j0 + j) * n + r0 + r]);
-    y[r][j] = T::from(v);
+      v = LOWER ? B[(size_t)j * n + (TRANS ? r0 + r : perm[r0 + r])] : ldcg(&X[(size_t)j * n + r0 + r]);
+    y[r][j] = S::from(v);
   }
-  const int c_lo = LOWER ? 0 : b + 1, c_hi = LOWER ? b : nblk;
-  if constexpr (F32 && !TRANS && NJ == 4) {
-    // Coalesced form for the FP32 factors of the sweep: warp w owns rows 8w .. 8w+7 of the
-    // block, lane l columns l and l + 32 of every 64-column tile, so each load instruction of
-    // a warp reads one contiguous 128-byte row segment; the lane's partial sums run over all
-    // tiles and are reduced across the warp once at the end.  Each warp waits for x_c on its
-    // own (lane 0 polls the flag), so no block barrier sits in the tile loop.
-    const int warp = tid >> 5, lane = tid & 31;
-    C a8[8][NJ];
+  // tiles in the order their blocks finish; the last one, the predecessor's, apart
+  const int nt = LOWER ? b : nblk - 1 - b;
+  auto block_of = [&](int t) { return LOWER ? t : nblk - 1 - t; };
+  // the predecessor's tile in registers: Q lanes per row, 64 / Q columns each
+  constexpr int CQ = 64 / P::Q;
+  const int pi = tid / P::Q, pq = tid % P::Q;
+  // ---- tiles 0 .. nt-2 ----
+  C acc[TRANS ? 2 : P::RW][NJ];
 #pragma unroll
-    for (int rr = 0; rr < 8; ++rr)
+  for (int r = 0; r < (TRANS ? 2 : P::RW); ++r)
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) a8[rr][j] = czero<C>();
-    for (int cc = c_lo; cc < c_hi; ++cc) {
-      const int c = LOWER ? cc : c_hi - 1 - (cc - c_lo);
-      const int t0 = c * BS, nt = min(BS, n - t0);
-      C lv[8][2];
+    for (int j = 0; j < NJ; ++j) acc[r][j] = czero<C>();
+  int ready = 0;  // tiles known to be finished
+#pragma unroll 1
+  for (int t = 0; t < nt - 1; ++t) {
+    const int t0 = block_of(t) * BS, ntc = min(BS, n - t0);
+    C lv[P::RW][2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int col = lane + 32 * h;
+    for (int h = 0; h < 2; ++h) {
+      const int col = lane + 32 * h;
 #pragma unroll
-        for (int rr = 0; rr < 8; ++rr) {
-          const int row = warp * 8 + rr;
-          lv[rr][h] = (row < nr && col < nt) ? T::fac(F, r0 + row, t0 + col) : czero<C>();
-        }
+      for (int rr = 0; rr < P::RW; ++rr) {
+        const int row = warp * P::RW + rr;
+        if constexpr (TRANS) lv[rr][h] = (col < nr && row < ntc) ? S::fac(F, t0 + row, r0 + col) : czero<C>();
+        else lv[rr][h] = (row < nr && col < ntc) ? S::fac(F, r0 + row, t0 + col) : czero<C>();
       }
-      if (lane == 0) {
-        wait_flag(flags, c, epoch, err);
-        __threadfence();
+    }
+    if (t >= ready) {  // look up the flags of the next 32 tiles; wait for this one's
+      const int u = t + lane;
+      bool up = false;
+      if (u < nt - 1) {
+        cuda::atomic_ref<int, cuda::thread_scope_device> f(flags[block_of(u)]);
+        up = f.load(cuda::memory_order_acquire) >= epoch;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, up);
+      ready = t + (m == 0xffffffffu ? 32 : __ffs(~m) - 1);
+      if (ready == t) {
+        if (lane == 0) wait_flag(flags, block_of(t), epoch, err);
+        ready = t + 1;
       }
       __syncwarp();
-      C xv[2][NJ];
+    }
+    if constexpr (TRANS) {
+      if (lane < P::RW * NJ) {
+        const int rr = lane / NJ, j = lane % NJ, row = warp * P::RW + rr;
+        xw[warp][rr][j] = (row < ntc && j < nj) ? S::from(ldcg(&X[(size_t)j * n + t0 + row])) : czero<C>();
+      }
+      __syncwarp();
+#pragma unroll
+      for (int rr = 0; rr < P::RW; ++rr)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const C xv = xw[warp][rr][j];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) acc[h][j] = cmac(acc[h][j], lv[rr][h], xv);
+        }
+      __syncwarp();
+    } else {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int col = lane + 32 * h;
+        C xv[NJ];
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
-          xv[h][j] = (col < nt && j < nj) ? T::from(ldcg(&X[(size_t)(j0 + j) * n + t0 + col])) : czero<C>();
+          xv[j] = (col < ntc && j < nj) ? S::from(ldcg(&X[(size_t)j * n + t0 + col])) : czero<C>();
+#pragma unroll
+        for (int rr = 0; rr < P::RW; ++rr)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) acc[rr][j] = cmac(acc[rr][j], lv[rr][h], xv[j]);
       }
+    }
+  }
+  if (nt > 1) {
+    if constexpr (TRANS) {
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int rr = 0; rr < 8; ++rr)
+        for (int j = 0; j < NJ; ++j) part[(warp * BS + lane + 32 * h) * NJ + j] = acc[h][j];
+      __syncthreads();
+      if (tid < BS * NJ) {
+        C v = czero<C>();
+        for (int w = 0; w < P::T / 32; ++w) {
+          const C q = part[w * BS * NJ + tid];
+          v = C{v.x + q.x, v.y + q.y};
+        }
+        y[tid / NJ][tid % NJ] = y[tid / NJ][tid % NJ] - v;
+      }
+    } else {
+      __syncthreads();  // y staged
 #pragma unroll
-          for (int j = 0; j < NJ; ++j) a8[rr][j] = cmac(a8[rr][j], lv[rr][h], xv[h][j]);
+      for (int rr = 0; rr < P::RW; ++rr)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          for (int o = 16; o > 0; o >>= 1) {
+            acc[rr][j].x += __shfl_xor_sync(0xffffffff, acc[rr][j].x, o);
+            acc[rr][j].y += __shfl_xor_sync(0xffffffff, acc[rr][j].y, o);
+          }
+          if (lane == 0) y[warp * P::RW + rr][j] = y[warp * P::RW + rr][j] - acc[rr][j];
+        }
     }
+  }
+  // ---- the predecessor's tile ----
+  if (nt > 0) {
+    const int c = block_of(nt - 1), t0 = c * BS, ntc = min(BS, n - t0);
+    C lv[CQ];
 #pragma unroll
-    for (int rr = 0; rr < 8; ++rr)
+    for (int q = 0; q < CQ; ++q) {
+      const int col = pq + P::Q * q;
+      lv[q] = (pi < nr && col < ntc) ? (TRANS ? S::fac(F, t0 + col, r0 + pi) : S::fac(F, r0 + pi, t0 + col)) : czero<C>();
+    }
+    if (lane == 0) wait_flag(flags, c, epoch, err);
+    __syncwarp();
+    if (tid < BS * NJ) {
+      const int r = tid % BS, j = tid / BS;
+      xs[r][j] = (r < ntc && j < nj) ? S::from(ldcg(&X[(size_t)j * n + t0 + r])) : czero<C>();
+    }
+    __syncthreads();
+    C s[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) s[j] = czero<C>();
+#pragma unroll
+    for (int q = 0; q < CQ; ++q)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) s[j] = cmac(s[j], lv[q], xs[pq + P::Q * q][j]);
+#pragma unroll
+    for (int o = 1; o < P::Q; o <<= 1)
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
-        for (int o = 16; o > 0; o >>= 1) {
-          a8[rr][j].x += __shfl_xor_sync(0xffffffff, a8[rr][j].x, o);
-          a8[rr][j].y += __shfl_xor_sync(0xffffffff, a8[rr][j].y, o);
-        }
-        if (lane == 0) xs[warp * 8 + rr][j] = a8[rr][j];
+        s[j].x += __shfl_xor_sync(0xffffffff, s[j].x, o);
+        s[j].y += __shfl_xor_sync(0xffffffff, s[j].y, o);
       }
-    __syncthreads();
-    for (int e = tid; e < BS * NJ; e += 256) {
-      const int r = e / NJ, j = e % NJ;
-      if (r < nr && j < nj) y[r][j] = y[r][j] - xs[r][j];
-    }
-    __syncthreads();
-  } else {
-  C acc[NJ];
+    if (pq == 0)
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) acc[j] = czero<C>();
-  for (int cc = c_lo; cc < c_hi; ++cc) {
-    const int c = LOWER ? cc : c_hi - 1 - (cc - c_lo);  // upper: the last block is ready first
-    const int t0 = c * BS, nt = min(BS, n - t0);
-    C lv[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int t = p * 16 + q;
-      lv[q] = (i < nr && t < nt) ? (TRANS ? T::fac(F, t0 + t, r0 + i) : T::fac(F, r0 + i, t0 + t)) : czero<C>();
-    }
-    if (tid == 0) {
-      wait_flag(flags, c, epoch, err);
-      __threadfence();
-    }
-    __syncthreads();
-    for (int e = tid; e < BS * NJ; e += 256) {
-      const int t = e / NJ, j = e % NJ;
-      xs[t][j] = (t < nt && j < nj) ? T::from(ldcg(&X[(size_t)(j0 + j) * n + t0 + t])) : czero<C>();
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[j] = cmac(acc[j], lv[q], xs[p * 16 + q][j]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NJ; ++j)
-    for (int o = 1; o < 4; o <<= 1) {
-      acc[j].x += __shfl_xor_sync(0xffffffff, acc[j].x, o);
-      acc[j].y += __shfl_xor_sync(0xffffffff, acc[j].y, o);
-    }
-  __syncthreads();
-  if (p == 0 && i < nr) {
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) y[i][j] = y[i][j] - acc[j];
+      for (int j = 0; j < NJ; ++j) y[pi][j] = y[pi][j] - s[j];
   }
   __syncthreads();
-  }
-  // X[rows] = Dinv_b * y: 4 threads per output, 16 terms each, combined by shuffles
-  for (int e0 = 0; e0 < nr * nj; e0 += 64) {
-    const int e = e0 + (tid >> 2), part = tid & 3;
-    const int r = e / nj, j = e % nj;
-    C s = czero<C>();
-    if (e < nr * nj) {
-#pragma unroll 4
-      for (int k = part * 16; k < part * 16 + 16; ++k)
-        if (k < nr) s = cmac(s, Ds[r * BS + k], y[k][j]);
+  // X[rows] = Dinv_b * y: one entry per T / 256 lanes
+  {
+    constexpr int H = P::T / (BS * NJ);
+    const int h = tid % H, e = tid / H, r = e / NJ, j = e % NJ;
+    C s0 = czero<C>(), s1 = czero<C>();
+#pragma unroll 8
+    for (int k = h; k < BS; k += 2 * H) {
+      s0 = cmac(s0, Ds[r * P::LD + k], y[k][j]);
+      s1 = cmac(s1, Ds[r * P::LD + k + H], y[k + H][j]);
     }
-    for (int o = 1; o < 4; o <<= 1) {
-      s.x += __shfl_xor_sync(0xffffffff, s.x, o);
-      s.y += __shfl_xor_sync(0xffffffff, s.y, o);
+    s0 = C{s0.x + s1.x, s0.y + s1.y};
+    if constexpr (H == 2) {
+      s0.x += __shfl_xor_sync(0xffffffff, s0.x, 1);
+      s0.y += __shfl_xor_sync(0xffffffff, s0.y, 1);
     }
-    if (part == 0 && e < nr * nj) stcg(&X[(size_t)(j0 + j) * n + r0 + r], T::to(s));
+    if (h == 0 && r < nr && j < nj) stcg(&X[(size_t)j * n + r0 + r], S::to(s0));
   }
   __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    post_flag(flags, b, epoch);
-  }
+  if (tid == 0) post_flag(flags, b, epoch);
 }
 
-// R = B - A X with max|r_j| (norms[j]), max|x_j| (norms[kNX + j]) and ||A||_inf (norms[kNA]).
-__global__ void __launch_bounds__(256) k_resid(int n, const cd *__restrict__ A0, long long ld, long long ms, int nrhs,
-                                               const cd *__restrict__ X0, const cd *__restrict__ B0,
-                                               cd *__restrict__ R0, long long vs, double *norms0, Ctrl ctrl) {
-  const int bm = blockIdx.y;
-  if (ctrl.of(bm)[2]) return;
-  const cd *A = A0 + bm * ms, *X = X0 + bm * vs, *B = B0 + bm * vs;
-  cd *R = R0 + bm * vs;
-  double *norms = norms0 + (long long)bm * kNormCount;
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row < n) {
-    const cd *a = A + (long long)row * ld;
-    for (int j0 = 0; j0 < nrhs; j0 += kMaxRhs) {
-      const int nj = min(kMaxRhs, nrhs - j0);
-      cd acc[kMaxRhs];
-      for (int j = 0; j < kMaxRhs; ++j) acc[j] = mkcd(0, 0);
-      double rs = 0;
-      for (int t = lane; t < n; t += 32) {
-        cd av = a[t];
-        if (j0 == 0) rs += cabs1(av);
-        for (int j = 0; j < nj; ++j) acc[j] = cmac(acc[j], av, X[(size_t)(j0 + j) * n + t]);
-      }
-      for (int j = 0; j < nj; ++j)
-        for (int o = 16; o > 0; o >>= 1) {
-          acc[j].x += __shfl_xor_sync(0xffffffff, acc[j].x, o);
-          acc[j].y += __shfl_xor_sync(0xffffffff, acc[j].y, o);
-        }
-      if (j0 == 0) {
-        for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffff, rs, o);
-        if (lane == 0) atomicMax((unsigned long long *)&norms[kNA], (unsigned long long)__double_as_longlong(rs));
-      }
-#pragma unroll
-      for (int j = 0; j < kMaxRhs; ++j) {
-        if (j < nj && lane == j) {
-          cd r = B[(size_t)(j0 + j) * n + row] - acc[j];
-          R[(size_t)(j0 + j) * n + row] = r;
-          atomicMax((unsigned long long *)&norms[j0 + j], (unsigned long long)__double_as_longlong(cabs1(r)));
-          double xv = cabs1(X[(size_t)(j0 + j) * n + row]);
-          atomicMax((unsigned long long *)&norms[kNX + j0 + j], (unsigned long long)__double_as_longlong(xv));
-        }
-      }
-    }
-  }
-}
-
-// Residual for up to 4 right-hand sides (the sweep's usual case): a CTA of 8 warps takes 16
-// rows, each warp 2 of them; the columns go in chunks whose X block (4 x 1024) is staged in
-// shared memory and reused by the rows of every warp, so the matrix rows are the only HBM
-// stream (each read once, streaming loads).  The column loop has no early exit (the ragged
-// last chunk is predicated), so the loads of several steps are in flight per lane; rows past
-// n are clamped to row n-1 for their loads and dropped at the end.
-constexpr int kResRows = 2, kResChunk = 1024;
-constexpr int kResSmem = 4 * kResChunk * (int)sizeof(cd);  // 64 KB
+// R = B - A X with max|r_j| (norms[j]), max|x_j| (norms[kNX + j]) and ||A||_inf (norms[kNA]), for
+// M right-hand sides from j0 = M * blockIdx.x on (4, the sweep's usual case; 8 at a time for
+// more, the groups of one row block side by side so that they share its rows in L2): a CTA of 8
+// warps takes 16 rows, each warp 2 of them; the columns go in chunks whose X block (M x 4096 / M
+// entries) is staged in shared memory and reused by the rows of every warp, so the matrix rows
+// are the only HBM stream (streaming loads).  The column loop has no early exit (the ragged last
+// chunk is predicated), so the loads of several steps are in flight per lane; rows past n are
+// clamped to row n-1 for their loads and dropped at the end.
+constexpr int kResRows = 2;
+constexpr int kResSmem = 4096 * (int)sizeof(cd);  // 64 KB
 __device__ __forceinline__ cd ldcs(const cd *p) {
   const double2 v = __ldcs(reinterpret_cast<const double2 *>(p));
   return cd{v.x, v.y};
 }
-__global__ void __launch_bounds__(256) k_resid4(int n, const cd *__restrict__ A0, long long ld, long long ms, int nrhs,
-                                                const cd *__restrict__ X0, const cd *__restrict__ B0,
-                                                cd *__restrict__ R0, long long vs, double *norms0, Ctrl ctrl) {
-  const int bm = blockIdx.y;
+template <int M>
+__global__ void __launch_bounds__(256, M == 4 ? 3 : 2) k_resid(int n, const cd *__restrict__ A0, long long ld, long long ms, int nrhs0,
+                                               const cd *__restrict__ X0, const cd *__restrict__ B0,
+                                               cd *__restrict__ R0, long long vs, double *norms0, Ctrl ctrl) {
+  constexpr int CH = 4096 / M;
+  const int bm = blockIdx.z;
   if (ctrl.of(bm)[2]) return;
-  const cd *A = A0 + bm * ms, *X = X0 + bm * vs, *B = B0 + bm * vs;
-  cd *R = R0 + bm * vs;
+  const int j0 = blockIdx.x * M, nrhs = min(M, nrhs0 - j0);
+  const cd *A = A0 + bm * ms, *X = X0 + bm * vs + (size_t)j0 * n, *B = B0 + bm * vs + (size_t)j0 * n;
+  cd *R = R0 + bm * vs + (size_t)j0 * n;
   double *norms = norms0 + (long long)bm * kNormCount;
   extern __shared__ __align__(16) unsigned char res_smem[];
-  cd(*xs)[kResChunk] = reinterpret_cast<cd(*)[kResChunk]>(res_smem);  // [4][kResChunk]
+  double2(*xs)[CH] = reinterpret_cast<double2(*)[CH]>(res_smem);  // [M][CH]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * (8 * kResRows) + warp * kResRows;
+  const int r0 = blockIdx.y * (8 * kResRows) + warp * kResRows;
   const cd *arow[kResRows];
-  cd acc[kResRows][4];
+  cd acc[kResRows][M];
   double rs[kResRows];
 #pragma unroll
   for (int i = 0; i < kResRows; ++i) {
     arow[i] = A + (long long)min(r0 + i, n - 1) * ld;
     rs[i] = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = mkcd(0, 0);
+    for (int j = 0; j < M; ++j) acc[i][j] = mkcd(0, 0);
   }
-  for (int t0 = 0; t0 < n; t0 += kResChunk) {
-    const int len = min(kResChunk, n - t0);
+  for (int t0 = 0; t0 < n; t0 += CH) {
+    const int len = min(CH, n - t0);
     __syncthreads();
-    for (int e = threadIdx.x; e < 4 * kResChunk; e += blockDim.x) {
-      const int j = e / kResChunk, t = e % kResChunk;
-      xs[j][t] = (j < nrhs && t < len) ? X[(size_t)j * n + t0 + t] : mkcd(0, 0);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < M * CH; e += 256) {
+      const int j = e / CH, t = e % CH;
+      xs[j][t] = (j < nrhs && t < len) ? *reinterpret_cast<const double2 *>(&X[(size_t)j * n + t0 + t]) : make_double2(0, 0);
     }
     __syncthreads();
     const int qn = (len + 31) >> 5;
@@ -420,15 +460,15 @@ __global__ void __launch_bounds__(256) k_resid4(int n, const cd *__restrict__ A0
       const bool ok = t < len;
       cd av[kResRows];
 #pragma unroll
-      for (int i = 0; i < kResRows; ++i) av[i] = ok ? ldcs(arow[i] + t0 + t) : mkcd(0, 0);
-      cd xv[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) xv[j] = xs[j][t];
-#pragma unroll
       for (int i = 0; i < kResRows; ++i) {
+        av[i] = ok ? ldcs(arow[i] + t0 + t) : mkcd(0, 0);
         rs[i] += cabs1(av[i]);
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = cmac(acc[i][j], av[i], xv[j]);
+      for (int j = 0; j < M; ++j) {
+        const double2 v = xs[j][t];
+#pragma unroll
+        for (int i = 0; i < kResRows; ++i) acc[i][j] = cmac(acc[i][j], av[i], mkcd(v.x, v.y));
       }
     }
   }
@@ -438,22 +478,23 @@ __global__ void __launch_bounds__(256) k_resid4(int n, const cd *__restrict__ A0
     for (int o = 16; o > 0; o >>= 1) {
       rs[i] += __shfl_xor_sync(0xffffffff, rs[i], o);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < M; ++j) {
         acc[i][j].x += __shfl_xor_sync(0xffffffff, acc[i][j].x, o);
         acc[i][j].y += __shfl_xor_sync(0xffffffff, acc[i][j].y, o);
       }
     }
     const int row = r0 + i;
     if (row >= n) continue;
-    if (lane == 0) atomicMax((unsigned long long *)&norms[kNA], (unsigned long long)__double_as_longlong(rs[i]));
+    if (lane == 0 && j0 == 0)
+      atomicMax((unsigned long long *)&norms[kNA], (unsigned long long)__double_as_longlong(rs[i]));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < M; ++j) {
       if (j < nrhs && lane == j) {
         const cd r = B[(size_t)j * n + row] - acc[i][j];
         R[(size_t)j * n + row] = r;
-        atomicMax((unsigned long long *)&norms[j], (unsigned long long)__double_as_longlong(cabs1(r)));
+        atomicMax((unsigned long long *)&norms[j0 + j], (unsigned long long)__double_as_longlong(cabs1(r)));
         const double xv = cabs1(X[(size_t)j * n + row]);
-        atomicMax((unsigned long long *)&norms[kNX + j], (unsigned long long)__double_as_longlong(xv));
+        atomicMax((unsigned long long *)&norms[kNX + j0 + j], (unsigned long long)__double_as_longlong(xv));
       }
     }
   }
@@ -526,23 +567,34 @@ __global__ void __launch_bounds__(kTrCols) k_resid_t1(int n, const cd *__restric
   const int nch = (int)gridDim.y;
   cd *part = part0 + (long long)bm * pstride;
   double *cabs = cabs0 + (long long)bm * nch * n;
-  if (j >= n) return;
-  for (int j0 = 0; j0 < nrhs; j0 += kMaxRhs) {
-    const int nj = min(kMaxRhs, nrhs - j0);
-    cd acc[kMaxRhs];
+  __shared__ double2 ys[kTrRows][NJ];
+  for (int j0 = 0; j0 < nrhs; j0 += NJ) {
+    const int nj = min(NJ, nrhs - j0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < kTrRows * NJ; e += kTrCols) {
+      const int t = e / kTrRows, i = e % kTrRows;
+      const cd v = (t < nj && i0 + i < i1) ? Y[(size_t)(j0 + t) * n + i0 + i] : mkcd(0, 0);
+      ys[i][t] = make_double2(v.x, v.y);
+    }
+    __syncthreads();
+    if (j >= n) continue;
+    cd acc[NJ];
 #pragma unroll
-    for (int t = 0; t < kMaxRhs; ++t) acc[t] = mkcd(0, 0);
+    for (int t = 0; t < NJ; ++t) acc[t] = mkcd(0, 0);
     double cs = 0.0;
+#pragma unroll 8
     for (int i = i0; i < i1; ++i) {
-      const cd a = A[(long long)i * ld + j];
-      if (j0 == 0) cs += cabs1(a);
+      const cd a = ldcs(A + (long long)i * ld + j);
+      cs += cabs1(a);
 #pragma unroll
-      for (int t = 0; t < kMaxRhs; ++t)
-        if (t < nj) acc[t] = acc[t] + a * Y[(size_t)(j0 + t) * n + i];
+      for (int t = 0; t < NJ; ++t) {
+        const double2 v = ys[i - i0][t];
+        acc[t] = cmac(acc[t], a, mkcd(v.x, v.y));
+      }
     }
     if (j0 == 0) cabs[(long long)q * n + j] = cs;
 #pragma unroll
-    for (int t = 0; t < kMaxRhs; ++t)
+    for (int t = 0; t < NJ; ++t)
       if (t < nj) part[((long long)q * nrhs + j0 + t) * n + j] = acc[t];
   }
 }
@@ -575,17 +627,36 @@ __global__ void k_resid_t2(int n, int nch, int nrhs, const cd *__restrict__ part
   }
 }
 
-template <bool LOWER>
+template <bool LOWER, bool F32, bool TRANS>
 cudaError_t set_trsv_smem() {
-  const int s64 = BS * BS * (int)sizeof(cd);
-  cudaError_t e = cudaFuncSetAttribute(k_trsv<LOWER, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, s64);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_trsv<LOWER, false, kMaxRhs>, cudaFuncAttributeMaxDynamicSharedMemorySize, s64);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_trsv<LOWER, false, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s64);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_trsv<LOWER, false, kMaxRhs, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s64);
-  return e;  // the FP32 forms stage 32 KB, under the default limit
+  return cudaFuncSetAttribute(k_trsv<LOWER, F32, TRANS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              TRANS ? TrsvT<F32>::SMEM_T : TrsvT<F32>::SMEM);
+}
+
+// Both passes of a solve for every group of kChains chains.
+template <bool F32, bool TRANS>
+int trsv_passes(SolveWS &ws, int nb, const Fac &F, int nrhs, const cd *B, cd *X, long long vs, int use_done,
+                cudaStream_t st) {
+  static DeviceOnce once;
+  if (int rc = device_once(once, [] {
+        PSS_CUDA_TRY((set_trsv_smem<true, F32, TRANS>()));
+        PSS_CUDA_TRY((set_trsv_smem<false, F32, TRANS>()));
+        return 0;
+      }))
+    return rc;
+  const Ctrl ctrl{ws.ctrl, ws.cstride};
+  const int smem = TRANS ? TrsvT<F32>::SMEM_T : TrsvT<F32>::SMEM;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int j0 = 0; j0 < nrhs; j0 += NJ * kChains) {
+      const int nchain = min(kChains, (nrhs - j0 + NJ - 1) / NJ);
+      ++ws.epoch;
+      pss_count_launch();
+      auto kern = pass == 0 ? k_trsv<true, F32, TRANS> : k_trsv<false, F32, TRANS>;
+      kern<<<dim3(nb * nchain, ws.nblk), TrsvT<F32>::T, smem, st>>>(F, ws.n, ws.perm, B, X, vs, nrhs, j0, nchain,
+                                                                    ws.Dinv, ws.dstride, ctrl, ws.epoch, use_done);
+    }
+  PSS_CUDA_TRY(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace
@@ -595,7 +666,7 @@ cudaError_t set_trsv_smem() {
 size_t pss_solve_ws_bytes(int n, int nb) {
   int nblk = (n + BS - 1) / BS;
   return (size_t)nb * ((size_t)nblk * 2 * BS * BS * sizeof(cd) + (size_t)n * sizeof(int) +
-                       (size_t)(nblk + 64) * sizeof(int) + kNormCount * sizeof(double)) + 512;
+                       (size_t)(8 + kChains * (nblk + 1)) * sizeof(int) + kNormCount * sizeof(double)) + 512;
 }
 
 void SolveWS::bind(void *base, int n_, int nb_) {
@@ -603,13 +674,13 @@ void SolveWS::bind(void *base, int n_, int nb_) {
   nb = nb_;
   nblk = (n + BS - 1) / BS;
   dstride = (long long)nblk * 2 * BS * BS;
-  cstride = nblk + 64;
+  cstride = 8 + kChains * (nblk + 1);
   char *p = (char *)base;
   Dinv = (cd *)p;
   p += (size_t)nb * dstride * sizeof(cd);
   perm = (int *)p;
   p += (size_t)nb * n * sizeof(int);
-  ctrl = (int *)p;  // per matrix: [0] ticket, [1] error, [2] converged, [8..8+nblk) flags
+  ctrl = (int *)p;
   p += (size_t)nb * cstride * sizeof(int);
   p = (char *)(((uintptr_t)p + 15) & ~(uintptr_t)15);
   norms = (double *)p;
@@ -626,12 +697,12 @@ int pss_solve_prepare(SolveWS &ws, int nb, const cd *LU64, const float *Lr, cons
   static DeviceOnce once;
   if (int rc = device_once(once, [] {
         PSS_CUDA_TRY(
-            cudaFuncSetAttribute(k_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * BS * BS * (int)sizeof(cd)));
+            cudaFuncSetAttribute(k_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kDinvSmem));
         return 0;
       }))
     return rc;
   pss_count_launch();
-  k_diag_inv<<<dim3(ws.nblk, 2, nb), BS, 2 * BS * BS * sizeof(cd), st>>>(F, ws.n, ws.Dinv, ws.dstride);
+  k_diag_inv<<<dim3(ws.nblk, 2, nb), 256, kDinvSmem, st>>>(F, ws.n, ws.Dinv, ws.dstride);
   PSS_CUDA_TRY(cudaMemsetAsync(ws.ctrl, 0, (size_t)nb * ws.cstride * sizeof(int), st));
   PSS_CUDA_TRY(cudaMemsetAsync(ws.norms, 0, (size_t)nb * kNormCount * sizeof(double), st));
   ws.epoch = 0;
@@ -642,39 +713,9 @@ int pss_solve_prepare(SolveWS &ws, int nb, const cd *LU64, const float *Lr, cons
 // elements apart).  use_done: skip matrices whose refinement has converged.
 int pss_solve_lu(SolveWS &ws, int nb, const cd *LU64, const float *Lr, const float *Li, long long ld, long long ms,
                  int nrhs, const cd *B, cd *X, long long vs, int use_done, cudaStream_t st) {
-  Fac F{LU64, Lr, Li, ld, ms};
-  const Ctrl ctrl{ws.ctrl, ws.cstride};
-  static DeviceOnce once;
-  if (int rc = device_once(once, [] {
-        PSS_CUDA_TRY(set_trsv_smem<true>());
-        PSS_CUDA_TRY(set_trsv_smem<false>());
-        return 0;
-      }))
-    return rc;
-  const bool f32 = LU64 == nullptr;
-  for (int pass = 0; pass < 2; ++pass)
-    for (int j0 = 0; j0 < nrhs; j0 += kMaxRhs) {
-      ++ws.epoch;
-      // tickets of every matrix back to zero (the flags keep their epochs)
-      PSS_CUDA_TRY(cudaMemset2DAsync(ws.ctrl, ws.cstride * sizeof(int), 0, sizeof(int), nb, st));
-      pss_count_launch();
-      const bool small = nrhs - j0 <= 4;
-      const dim3 grid(nb, ws.nblk);
-      auto go = [&](auto kern, size_t smem) {
-        kern<<<grid, 256, smem, st>>>(F, ws.n, ws.perm, B, X, vs, nrhs, j0, ws.Dinv, ws.dstride, ctrl, ws.epoch,
-                                      use_done);
-      };
-      const size_t s64 = BS * BS * sizeof(cd), s32 = BS * BS * sizeof(cf);
-      if (pass == 0) {
-        if (f32) small ? go(k_trsv<true, true, 4>, s32) : go(k_trsv<true, true, kMaxRhs>, s32);
-        else small ? go(k_trsv<true, false, 4>, s64) : go(k_trsv<true, false, kMaxRhs>, s64);
-      } else {
-        if (f32) small ? go(k_trsv<false, true, 4>, s32) : go(k_trsv<false, true, kMaxRhs>, s32);
-        else small ? go(k_trsv<false, false, 4>, s64) : go(k_trsv<false, false, kMaxRhs>, s64);
-      }
-    }
-  PSS_CUDA_TRY(cudaGetLastError());
-  return 0;
+  const Fac F{LU64, Lr, Li, ld, ms};
+  return LU64 ? trsv_passes<false, false>(ws, nb, F, nrhs, B, X, vs, use_done, st)
+              : trsv_passes<true, false>(ws, nb, F, nrhs, B, X, vs, use_done, st);
 }
 
 // A timed-out wait in a solve (never expected) marks the point (status[b]).
@@ -691,7 +732,8 @@ int pss_refine(SolveWS &ws, int nb, const cd *A, long long ld, long long ms, con
   const Ctrl ctrl{ws.ctrl, ws.cstride};
   static DeviceOnce once;
   if (int rc = device_once(once, [] {
-        PSS_CUDA_TRY(cudaFuncSetAttribute(k_resid4, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem));
+        PSS_CUDA_TRY(cudaFuncSetAttribute(k_resid<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem));
+        PSS_CUDA_TRY(cudaFuncSetAttribute(k_resid<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem));
         return 0;
       }))
     return rc;
@@ -700,11 +742,12 @@ int pss_refine(SolveWS &ws, int nb, const cd *A, long long ld, long long ms, con
   const long long total = (long long)ws.n * nrhs;
   for (int it = 0; it <= maxit; ++it) {
     pss_count_launch();
+    const unsigned rows = cdiv_u(ws.n, 8 * kResRows);
     if (nrhs <= 4)
-      k_resid4<<<dim3(cdiv_u(ws.n, 8 * kResRows), nb), 256, kResSmem, st>>>(ws.n, A, ld, ms, nrhs, X, B, R, vs,
-                                                                            ws.norms, ctrl);
+      k_resid<4><<<dim3(1, rows, nb), 256, kResSmem, st>>>(ws.n, A, ld, ms, nrhs, X, B, R, vs, ws.norms, ctrl);
     else
-      k_resid<<<dim3(cdiv_u(ws.n, 8), nb), 256, 0, st>>>(ws.n, A, ld, ms, nrhs, X, B, R, vs, ws.norms, ctrl);
+      k_resid<8><<<dim3(cdiv_u(nrhs, 8), rows, nb), 256, kResSmem, st>>>(ws.n, A, ld, ms, nrhs, X, B, R, vs, ws.norms,
+                                                                         ctrl);
     pss_count_launch();
     k_ir_check<<<nb, 1, 0, st>>>(ws.n, nrhs, ws.norms, ctrl, status, it == maxit);
     if (it == maxit) break;
@@ -723,36 +766,11 @@ int pss_refine(SolveWS &ws, int nb, const cd *A, long long ld, long long ms, con
 int pss_solve_lu_trans(SolveWS &ws, int nb, const cd *LU64, const float *Lr, const float *Li, long long ld,
                        long long ms, int nrhs, const cd *B, cd *Y, cd *W, long long vs, int use_done,
                        cudaStream_t st) {
-  Fac F{LU64, Lr, Li, ld, ms};
+  const Fac F{LU64, Lr, Li, ld, ms};
   const Ctrl ctrl{ws.ctrl, ws.cstride};
-  static DeviceOnce once;
-  if (int rc = device_once(once, [] {
-        PSS_CUDA_TRY(set_trsv_smem<true>());
-        PSS_CUDA_TRY(set_trsv_smem<false>());
-        return 0;
-      }))
+  if (int rc = LU64 ? trsv_passes<false, true>(ws, nb, F, nrhs, B, W, vs, use_done, st)
+                    : trsv_passes<true, true>(ws, nb, F, nrhs, B, W, vs, use_done, st))
     return rc;
-  const bool f32 = LU64 == nullptr;
-  for (int pass = 0; pass < 2; ++pass)
-    for (int j0 = 0; j0 < nrhs; j0 += kMaxRhs) {
-      ++ws.epoch;
-      PSS_CUDA_TRY(cudaMemset2DAsync(ws.ctrl, ws.cstride * sizeof(int), 0, sizeof(int), nb, st));
-      pss_count_launch();
-      const bool small = nrhs - j0 <= 4;
-      const dim3 grid(nb, ws.nblk);
-      auto go = [&](auto kern, size_t smem) {
-        kern<<<grid, 256, smem, st>>>(F, ws.n, ws.perm, B, W, vs, nrhs, j0, ws.Dinv, ws.dstride, ctrl, ws.epoch,
-                                      use_done);
-      };
-      const size_t s64 = BS * BS * sizeof(cd), s32 = BS * BS * sizeof(cf);
-      if (pass == 0) {
-        if (f32) small ? go(k_trsv<true, true, 4, true>, s32) : go(k_trsv<true, true, kMaxRhs, true>, s32);
-        else small ? go(k_trsv<true, false, 4, true>, s64) : go(k_trsv<true, false, kMaxRhs, true>, s64);
-      } else {
-        if (f32) small ? go(k_trsv<false, true, 4, true>, s32) : go(k_trsv<false, true, kMaxRhs, true>, s32);
-        else small ? go(k_trsv<false, false, 4, true>, s64) : go(k_trsv<false, false, kMaxRhs, true>, s64);
-      }
-    }
   pss_count_launch();
   k_unpermute<<<dim3(cdiv_u((long long)ws.n * nrhs, 256), nb), 256, 0, st>>>(ws.n, nrhs, ws.perm, W, Y, vs, ctrl,
                                                                           use_done);
