@@ -68,7 +68,6 @@ void pss_set_error(const char *fmt, ...) {
 namespace {
 
 constexpr int kRing0 = 160;  // ring budget of the first table pass (mmax <= 320)
-constexpr int kTableChunk = 16;
 constexpr int kMaxRefine = 10;  // refinement steps before the FP64 fallback (zcgesv allows 30)
 
 struct DevBuf {
@@ -358,7 +357,7 @@ int build_tables(pss_ctx *c, const StackParams &S, const PointParams *dP, int np
   if (c->dense.ensure((size_t)chunk * pstride * sizeof(cd))) return -3;
   if (c->conv.ensure((size_t)chunk * (R0 + 1) + 64)) return -3;
   if (c->mm.ensure(2 * sizeof(int) * (size_t)chunk + 64)) return -3;
-  if (c->stage.ensure(2 * (size_t)(2 * R0) * (2 * R0) * sizeof(cd))) return -3;
+  if (c->stage.ensure((size_t)chunk * 2 * (2 * R0) * (2 * R0) * sizeof(cd))) return -3;
   // points base .. base+npts-1 of the call; a multi-problem call sizes the table store for
   // all its points before the first problem, so this never reallocates under earlier tables
   if (c->tables.ensure((size_t)(base + npts) * 2 * cap0 * sizeof(cd))) return -3;
@@ -396,17 +395,28 @@ int build_tables(pss_ctx *c, const StackParams &S, const PointParams *dP, int np
         if (c->stage.ensure(2 * (size_t)mmax * mmax * sizeof(cd))) return -3;
         tabs[i].t = c->bigtables[i].as<cd>();
         tabs[i].mmax = mmax;
-        int rc = pss_tables_finish(c->bigdense.as<cd>(), R1, mmax, dP + il, c->stage.as<cd>(), tabs[i].t,
-                                   st);
+        const TableGroup one{1, {0}};
+        int rc = pss_tables_finish(c->bigdense.as<cd>(), 0, R1, mmax, dP + il, one, c->stage.as<cd>(), tabs[i].t, 0, st);
         if (rc) return rc;
         continue;
       }
       if (flag == 1) hstatus[i] |= PSS_ST_TABLE_NOCONV;
       tabs[i].t = c->tables.as<cd>() + (size_t)i * 2 * cap0;
       tabs[i].mmax = mmax;
-      int rc = pss_tables_finish(c->dense.as<cd>() + (size_t)q * pstride, R0, mmax, dP + il, c->stage.as<cd>(),
-                                 tabs[i].t, st);
-      if (rc) return rc;
+      hm[q] = mmax;
+      hm[chunk + q] = -1;  // to be finished with the chunk's other points of this mmax
+    }
+    for (int q = 0; q < nc; ++q) {
+      if (hm[chunk + q] != -1) continue;
+      TableGroup g{};
+      for (int t = q; t < nc; ++t)
+        if (hm[chunk + t] == -1 && hm[t] == hm[q]) {
+          g.q[g.n++] = t;
+          hm[chunk + t] = 0;
+        }
+      if (int rc = pss_tables_finish(c->dense.as<cd>(), pstride, R0, hm[q], dP + c0, g, c->stage.as<cd>(),
+                                     c->tables.as<cd>() + (size_t)(base + c0) * 2 * cap0, 2 * cap0, st))
+        return rc;
     }
   }
   PSS_CUDA_TRY(cudaStreamSynchronize(st));

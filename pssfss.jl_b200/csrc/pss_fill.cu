@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(256, 3) k_assemble(SheetDev G, const PointPara
 // of G[a + b*nm] = sum_m Lam[m, a] y[m, b] to part[x + y*gridDim.x] (rows in a fixed order, no
 // atomics: the shares are added in a fixed order by k_adj_reduce, so the result is deterministic).
 // Vectors are nbf x nm column-major.
-constexpr int kAdjNB = 8;
-__global__ void __launch_bounds__(256) k_adj_contract(SheetDev G, const PointParams *__restrict__ Pp,
+template <int kAdjNB>
+__global__ void __launch_bounds__(256, 2) k_adj_contract(SheetDev G, const PointParams *__restrict__ Pp,
                                                       const cd *__restrict__ zb, const cd *__restrict__ X,
                                                       const cd *__restrict__ R, const cd *__restrict__ Lam, int nm,
                                                       int b0, cd *__restrict__ part) {
@@ -324,9 +324,12 @@ size_t pss_adj_part_bytes(int nbf, int nm) { return (size_t)cdiv_u(nbf, 32) * kA
 void pss_adj_contract(const SheetDev &G, const PointParams *dP1, const cd *zb, const cd *X, const cd *R,
                       const cd *Lam, int nm, cd *part, cd *Gout, cudaStream_t st) {
   const int nblk = cdiv_u(G.nbf, 32);
-  for (int b0 = 0; b0 < nm; b0 += kAdjNB) {
+  for (int b0 = 0; b0 < nm;) {  // four right-hand sides at a time where that is all there is
+    const int nb = nm - b0 <= 4 ? 4 : 8;
+    auto kern = nb == 4 ? k_adj_contract<4> : k_adj_contract<8>;
     pss_count_launch();
-    k_adj_contract<<<dim3(nblk, kAdjChunks), dim3(32, 8), 0, st>>>(G, dP1, zb, X, R, Lam, nm, b0, part);
+    kern<<<dim3(nblk, kAdjChunks), dim3(32, 8), 0, st>>>(G, dP1, zb, X, R, Lam, nm, b0, part);
+    b0 += nb;
   }
   pss_count_launch();
   k_adj_reduce<<<nm * nm, 256, 0, st>>>(nblk * kAdjChunks, nm * nm, part, Gout);

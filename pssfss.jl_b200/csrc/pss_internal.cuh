@@ -181,7 +181,14 @@ void pss_tables_ring_fill(const StackParams &S, const PointParams *dP, int npts,
 void pss_tables_ring_sums(const PointParams *dP, int npts, int R, const cd *dense, size_t point_stride,
                           double convtest, unsigned char *conv, cudaStream_t st);
 void pss_tables_find_mmax(int npts, int R, const unsigned char *conv, int *mmax, int *flag, cudaStream_t st);
-int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t, cudaStream_t st);
+// Up to kTableChunk points of one mmax (their slots in the chunk) finished together.
+constexpr int kTableChunk = 32;
+struct TableGroup {
+  int n;
+  int q[kTableChunk];
+};
+int pss_tables_finish(const cd *dense, size_t pstride, int R, int mmax, const PointParams *dP, const TableGroup &g,
+                      cd *stage, cd *t, size_t tstride, cudaStream_t st);
 size_t pss_table_cap(int mmax);  // (mmax+2)^2 entries per padded table
 
 // Face-pair integrals and matrix fill (pss_fill.cu)

@@ -162,8 +162,11 @@ __global__ void k_find_mmax(int npts, int R, const unsigned char *__restrict__ c
 }
 
 // FFT input: a[p + q*mmax] = table[p - mo2, q - mo2] (PGF.jl:311-312).
-__global__ void k_fft_gather(const cd *__restrict__ dense, int R, int mmax, cd *__restrict__ a1,
-                             cd *__restrict__ a2) {
+// The points of a group (blockIdx.y), all of one mmax: slot g.q[y] of the chunk.
+__global__ void k_fft_gather(const cd *__restrict__ dense0, size_t pstride, TableGroup g, int R, int mmax,
+                             cd *__restrict__ stage) {
+  const cd *dense = dense0 + g.q[blockIdx.y] * pstride;
+  cd *a1 = stage + 2 * (size_t)blockIdx.y * mmax * mmax, *a2 = a1 + (size_t)mmax * mmax;
   const int W = 2 * R + 1;
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)mmax * mmax) return;
@@ -220,11 +223,12 @@ struct Radices {
   int r[16];
 };
 
-// Forward DFT of one line per CTA (line l at base + l*line_stride, element stride es).
+// Forward DFT of one line per CTA (line l at base + l*line_stride, element stride es) of
+// transform blockIdx.y (n*n elements each).
 __global__ void k_fft_lines(cd *__restrict__ data, int n, long long line_stride, long long es, Radices rad) {
   extern __shared__ cd sm[];
   cd *A = sm, *B = sm + n;
-  cd *line = data + (long long)blockIdx.x * line_stride;
+  cd *line = data + (size_t)blockIdx.y * n * n + (long long)blockIdx.x * line_stride;
   for (int i = threadIdx.x; i < n; i += blockDim.x) A[i] = line[(long long)i * es];
   __syncthreads();
   int Ns = 1;
@@ -283,8 +287,11 @@ __device__ __forceinline__ cd pad_value(const cd *__restrict__ A, int mmax, cons
   return ic2 * (ic1 * ext(mmax - 1, mmax - 1));
 }
 
-__global__ void k_phase_pad(const cd *__restrict__ a1, const cd *__restrict__ a2, int mmax,
-                            const PointParams *__restrict__ Pp, cd *__restrict__ tab) {
+__global__ void k_phase_pad(const cd *__restrict__ stage, int mmax, const PointParams *__restrict__ P0, TableGroup g,
+                            cd *__restrict__ tab0, size_t tstride) {
+  const cd *a1 = stage + 2 * (size_t)blockIdx.y * mmax * mmax, *a2 = a1 + (size_t)mmax * mmax;
+  const PointParams *Pp = P0 + g.q[blockIdx.y];
+  cd *tab = tab0 + g.q[blockIdx.y] * tstride;
   const int L = mmax + 2;
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)L * L) return;
@@ -307,7 +314,8 @@ int factor235(int n, Radices &rad) {
   return n == 1 ? k : -1;
 }
 
-int fft2d(cd *a, int n, cudaStream_t st) {
+// cnt n x n transforms in place.
+int fft2d(cd *a, int n, int cnt, cudaStream_t st) {
   if (n <= 1) return 0;
   Radices rad;
   if (n > PSS_MMAX_CAP || factor235(n, rad) < 0) { pss_set_error("fft size %d not supported", n); return -2; }
@@ -315,9 +323,9 @@ int fft2d(cd *a, int n, cudaStream_t st) {
   int thr = 256;
   // columns: contiguous lines; rows: stride n
   pss_count_launch();
-  k_fft_lines<<<n, thr, smem, st>>>(a, n, n, 1, rad);
+  k_fft_lines<<<dim3(n, cnt), thr, smem, st>>>(a, n, n, 1, rad);
   pss_count_launch();
-  k_fft_lines<<<n, thr, smem, st>>>(a, n, 1, n, rad);
+  k_fft_lines<<<dim3(n, cnt), thr, smem, st>>>(a, n, 1, n, rad);
   return 0;
 }
 
@@ -343,9 +351,12 @@ void pss_tables_find_mmax(int npts, int R, const unsigned char *conv, int *mmax,
   k_find_mmax<<<cdiv_u(npts, 64), 64, 0, st>>>(npts, R, conv, mmax, flag);
 }
 
-// dense: this point's (2R+1)^2 x 2 tables; stage: >= 2*mmax^2 entries; t: 2*(mmax+2)^2.
-int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, cd *stage, cd *t,
-                      cudaStream_t st) {
+// The points of a group, one launch per step for all of them (a point's own launches, 2 x 2
+// passes of a few microseconds each on one stream, were 65 us a point before any worker started):
+// dense + q*pstride: the point's (2R+1)^2 x 2 tables; stage: >= 2*mmax^2 entries per point;
+// t + q*tstride: its 2*(mmax+2)^2 table entries; dP + q: its parameters.
+int pss_tables_finish(const cd *dense, size_t pstride, int R, int mmax, const PointParams *dP, const TableGroup &g,
+                      cd *stage, cd *t, size_t tstride, cudaStream_t st) {
   static DeviceOnce once;
   if (int rc = device_once(once, [] {
         PSS_CUDA_TRY(cudaFuncSetAttribute(k_fft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -353,19 +364,15 @@ int pss_tables_finish(const cd *dense, int R, int mmax, const PointParams *dP1, 
         return 0;
       }))
     return rc;
-  long long nn = (long long)mmax * mmax;
-  cd *a1 = stage, *a2 = stage + nn;
+  const long long nn = (long long)mmax * mmax;
   if (nn > 0) {
     pss_count_launch();
-    k_fft_gather<<<cdiv_u(nn, 256), 256, 0, st>>>(dense, R, mmax, a1, a2);
-    int rc = fft2d(a1, mmax, st);
-    if (rc) return rc;
-    rc = fft2d(a2, mmax, st);
-    if (rc) return rc;
+    k_fft_gather<<<dim3(cdiv_u(nn, 256), g.n), 256, 0, st>>>(dense, pstride, g, R, mmax, stage);
+    if (int rc = fft2d(stage, mmax, 2 * g.n, st)) return rc;
   }
-  long long L2 = (long long)(mmax + 2) * (mmax + 2);
+  const long long L2 = (long long)(mmax + 2) * (mmax + 2);
   pss_count_launch();
-  k_phase_pad<<<cdiv_u(L2, 256), 256, 0, st>>>(a1, a2, mmax, dP1, t);
+  k_phase_pad<<<dim3(cdiv_u(L2, 256), g.n), 256, 0, st>>>(stage, mmax, dP, g, t, tstride);
   PSS_CUDA_TRY(cudaGetLastError());
   return 0;
 }
