@@ -75,21 +75,14 @@ struct DevBuf {
   size_t n = 0;
   int ensure(size_t bytes) {
     if (bytes <= n) return 0;
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
+    release();
     if (bytes == 0) return 0;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-      pss_set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
-      p = nullptr;
-      return -3;
-    }
+    if (int rc = pss_dev_alloc(&p, bytes)) return rc;
     n = bytes;
     return 0;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p) pss_dev_free(p);
     p = nullptr;
     n = 0;
   }
@@ -183,6 +176,49 @@ struct Worker {
     return 0;
   }
 };
+
+// Sheet upload: the caller's 1-based 64-bit class map and representatives as 0-based 32-bit ones,
+// and each representative's (match, source) faces.
+__global__ void k_class_map(long long n, long long nufp, const long long *__restrict__ in, int *__restrict__ out,
+                            int *bad) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long v = in[i];
+  if (v < 1 || v > nufp) *bad = 1;
+  out[i] = (int)(v - 1);
+}
+__global__ void k_class_reps(long long nufp, int nface, const long long *__restrict__ in, int *__restrict__ rep,
+                             int2 *__restrict__ faces, int *bad) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= nufp) return;
+  const long long v = in[i];
+  if (v < 1 || v > (long long)nface * nface) { *bad = 1; return; }
+  const int p = (int)(v - 1);
+  rep[i] = p;
+  faces[i] = make_int2(p % nface, p / nface);
+}
+
+// Column-major n x n system (pss_lu_solve) to the row-major FP64 matrix and, in the FP32 form, the
+// float planes with their padding zeroed; 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) k_system_rows(int n, const cd *__restrict__ Z, cd *__restrict__ A,
+                                                     float *__restrict__ Ar, float *__restrict__ Ai, long long ldf) {
+  __shared__ cd tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  for (int y = ty; y < 32; y += 8)
+    tile[y][tx] = (c0 + y < n && r0 + tx < n) ? Z[(size_t)(c0 + y) * n + r0 + tx] : mkcd(0, 0);
+  __syncthreads();
+  for (int y = ty; y < 32; y += 8) {
+    const int r = r0 + y, c = c0 + tx;
+    if (r >= n) continue;
+    const cd v = tile[tx][y];
+    if (c < n) A[(size_t)r * n + c] = v;
+    if (Ar && c < ldf) {
+      Ar[(size_t)r * ldf + c] = (float)v.x;
+      Ai[(size_t)r * ldf + c] = (float)v.y;
+    }
+  }
+}
 
 // Batch-local status words OR-ed into the points' status words.
 constexpr int kMaxBatch = 32;
@@ -532,6 +568,7 @@ int pss_ctx_destroy(pss_ctx *c) {
                     &c->dS, &c->status})
     b->release();
   for (auto &b : c->bigtables) b.release();
+  pss_dev_trim();
   delete c;
   return 0;
 }
@@ -566,20 +603,36 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     hfv[i] = (int)(fv[i] - 1);
     if (fe[i] < 1 || fe[i] > nedge) { pss_set_error("fe[%lld] out of range", (long long)i); delete sh; return -1; }
   }
-  // device copy in the reference's order (match face fastest): the assembly gathers a column
-  // of a Z tile - consecutive match faces against one source face - whose classes are then
-  // consecutive entries of this map
-  std::vector<int> hufpm((size_t)nface * nface);
-  for (size_t i = 0; i < hufpm.size(); ++i) {
-    if (ufpm[i] < 1 || ufpm[i] > nufp) { pss_set_error("ufpm entry out of range"); delete sh; return -1; }
-    hufpm[i] = (int)(ufpm[i] - 1);
-  }
-  std::vector<int> hrep(nufp), hpf(2 * nufp);
-  for (int64_t i = 0; i < nufp; ++i) {
-    if (ufp_rep[i] < 1 || ufp_rep[i] > nface * nface) { pss_set_error("ufp_rep out of range"); delete sh; return -1; }
-    hrep[i] = (int)(ufp_rep[i] - 1);
-    hpf[2 * i] = (int)((ufp_rep[i] - 1) % nface);
-    hpf[2 * i + 1] = (int)((ufp_rep[i] - 1) / nface);
+  // The class map and the representatives are converted to 0-based int32 on the device, which
+  // also checks their range (the map keeps the reference's order, match face fastest: the assembly
+  // gathers a column of a Z tile - consecutive match faces against one source face - whose classes
+  // are then consecutive entries).
+  {
+    const size_t np2 = (size_t)nface * nface;
+    LocalBuf raw, bad;
+    int hbad[2] = {0, 0};
+    if (raw.ensure(std::max(np2, (size_t)nufp) * sizeof(int64_t)) || upload(bad, hbad, 2) ||
+        sh->ufpm.ensure(np2 * sizeof(int)) || sh->rep.ensure(nufp * sizeof(int)) ||
+        sh->pfaces.ensure(nufp * sizeof(int2))) {
+      delete sh;
+      return -3;
+    }
+    auto convert = [&]() -> int {
+      PSS_CUDA_TRY(cudaMemcpy(raw.p, ufpm, np2 * sizeof(int64_t), cudaMemcpyHostToDevice));
+      pss_count_launch();
+      k_class_map<<<cdiv_u((long long)np2, 256), 256>>>((long long)np2, nufp, raw.as<long long>(), sh->ufpm.as<int>(),
+                                                        bad.as<int>());
+      PSS_CUDA_TRY(cudaMemcpy(raw.p, ufp_rep, nufp * sizeof(int64_t), cudaMemcpyHostToDevice));
+      pss_count_launch();
+      k_class_reps<<<cdiv_u(nufp, 256), 256>>>(nufp, (int)nface, raw.as<long long>(), sh->rep.as<int>(),
+                                               sh->pfaces.as<int2>(), bad.as<int>() + 1);
+      PSS_CUDA_TRY(cudaMemcpy(hbad, bad.p, sizeof(hbad), cudaMemcpyDeviceToHost));
+      return 0;
+    };
+    int rc = convert();
+    if (!rc && hbad[0]) { pss_set_error("ufpm entry out of range"); rc = -1; }
+    if (!rc && hbad[1]) { pss_set_error("ufp_rep out of range"); rc = -1; }
+    if (rc) { sh->rep.release(); sh->ufpm.release(); sh->pfaces.release(); delete sh; return rc; }
   }
   // basis-function incidences: (face, local edge, sign, edge code), fixed order
   std::vector<int> icnt(nbf, 0), iface(4 * nbf, 0), iloc(4 * nbf, 0), isgn(4 * nbf, 0), ieci(4 * nbf, 0);
@@ -642,8 +695,6 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   int rc = 0;
   rc |= upload(sh->rho, rho, 2 * (size_t)nnode);
   rc |= upload(sh->fv, hfv.data(), hfv.size());
-  rc |= upload(sh->ufpm, hufpm.data(), hufpm.size());
-  rc |= upload(sh->rep, hrep.data(), hrep.size());
   rc |= upload(sh->fr, hfr.data(), hfr.size());
   rc |= upload(sh->ls, hls.data(), hls.size());
   rc |= upload(sh->a48, ha48.data(), ha48.size());
@@ -653,7 +704,6 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   rc |= upload(sh->inc_sgn, isgn.data(), isgn.size());
   rc |= upload(sh->inc_eci, ieci.data(), ieci.size());
   rc |= upload(sh->face_m, hfm.data(), hfm.size());
-  rc |= upload(sh->pfaces, hpf.data(), hpf.size());
   rc |= upload(sh->inc, hinc.data(), hinc.size());
   if (rc) { delete sh; return -3; }
   SheetDev &G = sh->G;
@@ -1339,38 +1389,29 @@ int pss_lu_solve(pss_ctx *c, int n, const double *Z, int nrhs, const double *B, 
   Worker &w = c->w[0];
   cudaStream_t st = w.st;
   const size_t nn = (size_t)n * n;
-  std::vector<cd> h(nn);
-  for (size_t m = 0; m < (size_t)n; ++m)
-    for (size_t q = 0; q < (size_t)n; ++q) h[m * n + q] = mkcd(Z[2 * (m + q * n)], Z[2 * (m + q * n) + 1]);
-  if (w.z64.ensure(nn * sizeof(cd)) || w.ensure_solver(n, nrhs, 1)) return -3;
-  DevBuf st_buf;
+  const bool f32 = precision == PSS_FP32_REFINE;
+  const size_t ldf = (size_t)Worker::ld32(n), nf = (size_t)n * ldf;
+  LocalBuf raw, st_buf;  // the caller's column-major matrix, transposed on the device
+  if (raw.ensure(nn * sizeof(cd)) || w.z64.ensure(nn * sizeof(cd)) || w.ensure_solver(n, nrhs, 1)) return -3;
+  if (f32 && (w.zr.ensure(nf * sizeof(float)) || w.zi.ensure(nf * sizeof(float)))) return -3;
   if (st_buf.ensure(sizeof(int))) return -3;
-  PSS_CUDA_TRY(cudaMemset(st_buf.p, 0, sizeof(int)));
-  PSS_CUDA_TRY(cudaMemset(w.info.p, 0, sizeof(int)));
-  PSS_CUDA_TRY(cudaMemcpy(w.z64.p, h.data(), nn * sizeof(cd), cudaMemcpyHostToDevice));
-  PSS_CUDA_TRY(cudaMemcpy(w.rhs.p, B, (size_t)n * nrhs * sizeof(cd), cudaMemcpyHostToDevice));
+  PSS_CUDA_TRY(cudaMemsetAsync(st_buf.p, 0, sizeof(int), st));
+  PSS_CUDA_TRY(cudaMemsetAsync(w.info.p, 0, sizeof(int), st));
+  PSS_CUDA_TRY(cudaMemcpyAsync(raw.p, Z, nn * sizeof(cd), cudaMemcpyHostToDevice, st));
+  PSS_CUDA_TRY(cudaMemcpyAsync(w.rhs.p, B, (size_t)n * nrhs * sizeof(cd), cudaMemcpyHostToDevice, st));
+  pss_count_launch();
+  k_system_rows<<<dim3(cdiv_u((long long)ldf, 32), cdiv_u(n, 32)), 256, 0, st>>>(
+      n, raw.as<cd>(), w.z64.as<cd>(), f32 ? w.zr.as<float>() : nullptr, f32 ? w.zi.as<float>() : nullptr, (long long)ldf);
   int rc;
-  if (precision == PSS_FP32_REFINE) {
-    const size_t ldf = (size_t)Worker::ld32(n), nf = (size_t)n * ldf;
-    if (w.zr.ensure(nf * sizeof(float)) || w.zi.ensure(nf * sizeof(float))) return -3;
-    std::vector<float> hr(nf, 0.f), hi(nf, 0.f);
-    for (size_t m = 0; m < (size_t)n; ++m)
-      for (size_t q = 0; q < (size_t)n; ++q) {
-        hr[m * ldf + q] = (float)h[m * n + q].x;
-        hi[m * ldf + q] = (float)h[m * n + q].y;
-      }
-    PSS_CUDA_TRY(cudaMemcpy(w.zr.p, hr.data(), nf * sizeof(float), cudaMemcpyHostToDevice));
-    PSS_CUDA_TRY(cudaMemcpy(w.zi.p, hi.data(), nf * sizeof(float), cudaMemcpyHostToDevice));
-  }
   if ((rc = w.factor_solve(n, 1, precision, nrhs, kMaxRefine, st_buf.as<int>()))) return rc;
   PSS_CUDA_TRY(cudaStreamSynchronize(st));
   PSS_CUDA_TRY(cudaGetLastError());
   int hs = 0;
   PSS_CUDA_TRY(cudaMemcpy(&hs, st_buf.p, sizeof(int), cudaMemcpyDeviceToHost));
   if (precision == PSS_FP32_REFINE && (hs & (PSS_ST_REFINE_NOCONV | PSS_ST_NONFINITE))) {
-    // stalled refinement: FP64 factorisation of the original matrix
-    PSS_CUDA_TRY(cudaMemset(st_buf.p, 0, sizeof(int)));
-    PSS_CUDA_TRY(cudaMemcpy(w.z64.p, h.data(), nn * sizeof(cd), cudaMemcpyHostToDevice));
+    // stalled refinement: FP64 factorisation of the original matrix (z64, which the FP32 form
+    // only reads)
+    PSS_CUDA_TRY(cudaMemsetAsync(st_buf.p, 0, sizeof(int), st));
     if ((rc = w.factor_solve(n, 1, PSS_FP64, nrhs, 0, st_buf.as<int>()))) return rc;
     PSS_CUDA_TRY(cudaStreamSynchronize(st));
     PSS_CUDA_TRY(cudaMemcpy(&hs, st_buf.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1378,7 +1419,6 @@ int pss_lu_solve(pss_ctx *c, int n, const double *Z, int nrhs, const double *B, 
   }
   PSS_CUDA_TRY(cudaMemcpy(X, w.X.p, (size_t)n * nrhs * sizeof(cd), cudaMemcpyDeviceToHost));
   if (status) *status = hs;
-  st_buf.release();
   return 0;
 }
 

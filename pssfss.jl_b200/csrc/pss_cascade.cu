@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kCascadeThreads) k_cascade(CascadeArgs a) {
 struct ScopedDev {
   void *p = nullptr;
   ~ScopedDev() {
-    if (p) cudaFree(p);
+    if (p) pss_dev_free(p);
   }
 };
 
@@ -206,13 +206,13 @@ extern "C" int pss_cascade(pss_ctx *ctx, int npts, int nblk, const int *dims, co
   const size_t b_gsm = (size_t)npts * goff[nblk] * sizeof(cd), b_prop = (size_t)npts * ptot * sizeof(cd);
   const size_t b_out = (size_t)npts * out_per * sizeof(cd), b_scr = (size_t)npts * spp * sizeof(cd);
   ScopedDev dg, dp, dout, dscr, dgo, ddims, dsing;
-  PSS_CUDA_TRY(cudaMalloc(&dg.p, b_gsm));
-  PSS_CUDA_TRY(cudaMalloc(&dp.p, b_prop));
-  PSS_CUDA_TRY(cudaMalloc(&dout.p, b_out));
-  PSS_CUDA_TRY(cudaMalloc(&dscr.p, b_scr));
-  PSS_CUDA_TRY(cudaMalloc(&dgo.p, (nblk + 1) * sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&ddims.p, (nblk + 1) * sizeof(int)));
-  PSS_CUDA_TRY(cudaMalloc(&dsing.p, npts * sizeof(int)));
+  if (pss_dev_alloc(&dg.p, b_gsm)) return -3;
+  if (pss_dev_alloc(&dp.p, b_prop)) return -3;
+  if (pss_dev_alloc(&dout.p, b_out)) return -3;
+  if (pss_dev_alloc(&dscr.p, b_scr)) return -3;
+  if (pss_dev_alloc(&dgo.p, (nblk + 1) * sizeof(long long))) return -3;
+  if (pss_dev_alloc(&ddims.p, (nblk + 1) * sizeof(int))) return -3;
+  if (pss_dev_alloc(&dsing.p, npts * sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemcpy(dg.p, gsm, b_gsm, cudaMemcpyHostToDevice));
   PSS_CUDA_TRY(cudaMemcpy(dp.p, prop, b_prop, cudaMemcpyHostToDevice));
   PSS_CUDA_TRY(cudaMemcpy(dgo.p, goff.data(), (nblk + 1) * sizeof(long long), cudaMemcpyHostToDevice));

@@ -174,7 +174,7 @@ __global__ void k_ufp_assign(long long npairs, const int *__restrict__ slot_of, 
 struct Buf {
   void *p = nullptr;
   ~Buf() {
-    if (p) cudaFree(p);
+    if (p) pss_dev_free(p);
   }
 };
 
@@ -199,31 +199,31 @@ extern "C" int pss_face_pair_classes(pss_ctx *ctx, int64_t nface, const double *
   const long long npairs = (long long)nface * nface;
   const long long nblk = (npairs + kScanBlock - 1) / kScanBlock;
   Buf dcen, dr1, dshape, dslot, dflag, drank, dbsum, dtot, dufpm, drep, derr;
-  PSS_CUDA_TRY(cudaMalloc(&dcen.p, 2 * nface * sizeof(double)));
-  PSS_CUDA_TRY(cudaMalloc(&dr1.p, 2 * nface * sizeof(double)));
-  PSS_CUDA_TRY(cudaMalloc(&dshape.p, nface * sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&dslot.p, npairs * sizeof(int)));
-  PSS_CUDA_TRY(cudaMalloc(&dflag.p, npairs * sizeof(int)));
-  PSS_CUDA_TRY(cudaMalloc(&drank.p, npairs * sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&dbsum.p, nblk * sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&dtot.p, sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&dufpm.p, npairs * sizeof(int)));
-  PSS_CUDA_TRY(cudaMalloc(&drep.p, rep_cap * sizeof(long long)));
-  PSS_CUDA_TRY(cudaMalloc(&derr.p, sizeof(int)));
+  if (pss_dev_alloc(&dcen.p, 2 * nface * sizeof(double))) return -3;
+  if (pss_dev_alloc(&dr1.p, 2 * nface * sizeof(double))) return -3;
+  if (pss_dev_alloc(&dshape.p, nface * sizeof(long long))) return -3;
+  if (pss_dev_alloc(&dslot.p, npairs * sizeof(int))) return -3;
+  if (pss_dev_alloc(&dflag.p, npairs * sizeof(int))) return -3;
+  if (pss_dev_alloc(&drank.p, npairs * sizeof(long long))) return -3;
+  if (pss_dev_alloc(&dbsum.p, nblk * sizeof(long long))) return -3;
+  if (pss_dev_alloc(&dtot.p, sizeof(long long))) return -3;
+  if (pss_dev_alloc(&dufpm.p, npairs * sizeof(int))) return -3;
+  if (pss_dev_alloc(&drep.p, rep_cap * sizeof(long long))) return -3;
+  if (pss_dev_alloc(&derr.p, sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemcpy(dcen.p, cen, 2 * nface * sizeof(double), cudaMemcpyHostToDevice));
   PSS_CUDA_TRY(cudaMemcpy(dr1.p, r1, 2 * nface * sizeof(double), cudaMemcpyHostToDevice));
   PSS_CUDA_TRY(cudaMemcpy(dshape.p, shape, nface * sizeof(long long), cudaMemcpyHostToDevice));
   // the table: the power of two at or above twice the pairs (every key fits at a load of at
   // most one half, whatever the sheet's symmetry: a structured meander has a class for
   // every 2.5 pairs, a perturbed one nearly one per pair), at most 2^28 slots (7.5 GB)
-  unsigned long long cap = 1ull << 20;
+  unsigned long long cap = 1ull << 12;
   while (cap < 2ull * (unsigned long long)npairs && cap < (1ull << 28)) cap <<= 1;
   {
     Buf w0, w1, state, first;
-    PSS_CUDA_TRY(cudaMalloc(&w0.p, cap * sizeof(unsigned long long)));
-    PSS_CUDA_TRY(cudaMalloc(&w1.p, cap * sizeof(unsigned long long)));
-    PSS_CUDA_TRY(cudaMalloc(&state.p, cap * sizeof(int)));
-    PSS_CUDA_TRY(cudaMalloc(&first.p, cap * sizeof(long long)));
+    if (pss_dev_alloc(&w0.p, cap * sizeof(unsigned long long))) return -3;
+    if (pss_dev_alloc(&w1.p, cap * sizeof(unsigned long long))) return -3;
+    if (pss_dev_alloc(&state.p, cap * sizeof(int))) return -3;
+    if (pss_dev_alloc(&first.p, cap * sizeof(long long))) return -3;
     PSS_CUDA_TRY(cudaMemset(state.p, 0, cap * sizeof(int)));
     PSS_CUDA_TRY(cudaMemset(first.p, 0x7f, cap * sizeof(long long)));  // 0x7f7f...: above any pair index
     PSS_CUDA_TRY(cudaMemset(derr.p, 0, sizeof(int)));
