@@ -713,6 +713,7 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   G.inc_cnt = sh->inc_cnt.as<int>(); G.inc_face = sh->inc_face.as<int>(); G.inc_loc = sh->inc_loc.as<int>();
   G.inc_sgn = sh->inc_sgn.as<int>(); G.inc_eci = sh->inc_eci.as<int>();
   G.face_m = sh->face_m.as<double>(); G.pair_faces = sh->pfaces.as<int2>(); G.inc = sh->inc.as<int4>();
+  G.two_inc = std::all_of(icnt.begin(), icnt.end(), [](int c) { return c <= 2; }) ? 1 : 0;
   G.has_res = std::any_of(hfr.begin(), hfr.end(), [](double r) { return r != 0.0; }) ? 1 : 0;
   G.ext1 = hi[0] - lo[0]; G.ext2 = hi[1] - lo[1];
   *out = sh;

@@ -73,6 +73,7 @@ struct SheetDev {
   const int2 *pair_faces;// nufp: (match face, source face) of the class representative
   const int4 *inc;       // nbf: packed incidences, face << 8 | slot << 4 | minus << 3 | edge code
   int has_res;           // some face has a surface resistance
+  int two_inc;           // no basis function has more than two incidences
   double ext1, ext2;     // extents of the vertices in lattice coordinates (along s1 and s2)
 };
 
