@@ -658,7 +658,7 @@ int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const
     else if (np == 2) k_filljk_tab<2, false><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
     else k_filljk_tab<kJKGroup, false><<<gt, kTabThreads, 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk);
   }
-  k_filljk_list<<<dim3(148, np), jk_threads<1>(), 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk, nonconv);
+  k_filljk_list<<<dim3(148 * 6, np), jk_threads<1>(), 0, st>>>(G, ulocal, pg, a, b, c, d, T, jk, nonconv);
   PSS_CUDA_TRY(cudaGetLastError());
   return 0;
 }

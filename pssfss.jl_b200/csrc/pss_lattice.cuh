@@ -51,6 +51,7 @@ __device__ __forceinline__ unsigned jksums_group(double urx, double ury, int np,
                                                  const cd (*__restrict__ ph2)[kPhase], const double *__restrict__ etab,
                                                  cd *jout, cd *kout) {
   const int rmin = 5;
+  constexpr int UNR = NP == 1 ? 2 : 1;  // two summands in flight where the registers allow
   const double small = 1e-5, convtest = 1e-8;
   double arg = sqrt(urx * urx + ury * ury);
   double rterm = exp_neg(arg, etab);
@@ -92,12 +93,16 @@ __device__ __forceinline__ unsigned jksums_group(double urx, double ury, int np,
     {
       const double dr = (double)r;
       double dn = -dr;
+#pragma unroll UNR
       for (int i = -r; i <= r; ++i, dn += 1.0) summand(r, i, dr, dn);
       dn = -dr;
+#pragma unroll UNR
       for (int i = -r; i <= r; ++i, dn += 1.0) summand(-r, i, -dr, dn);
       double dm = 1.0 - dr;
+#pragma unroll UNR
       for (int i = 1 - r; i < r; ++i, dm += 1.0) summand(i, -r, dm, -dr);
       dm = 1.0 - dr;
+#pragma unroll UNR
       for (int i = 1 - r; i < r; ++i, dm += 1.0) summand(i, r, dm, dr);
     }
 #pragma unroll
