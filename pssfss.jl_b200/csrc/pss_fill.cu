@@ -187,6 +187,40 @@ __device__ __forceinline__ cd assemble_entry(const SheetDev &G, const cd *ff, bo
   return acc;
 }
 
+// Four entries of a row of a sheet without resistance whose basis functions all have at most two
+// incidences: no branches, all class numbers and then all pair terms in flight together.
+__device__ __forceinline__ void assemble_four(const SheetDev &G, const cd *ff, const cd *__restrict__ zb,
+                                              const RowInc &M, const int (&n)[4], cd (&z)[4]) {
+  int2 e[4];  // the columns' packed incidences
+  bool two[4];
+  int iu[4][4];
+  cd v[4][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    e[k] = __ldg(reinterpret_cast<const int2 *>(G.inc + n[k]));
+    two[k] = __ldg(G.inc_cnt + n[k]) > 1;
+    if (!two[k]) e[k].y = e[k].x;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      iu[k][t] = __ldg(G.ufpm + (size_t)M.face[t >> 1] + (size_t)((t & 1 ? e[k].y : e[k].x) >> 8) * G.nface);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      v[k][t] = ld_cd(zb + (size_t)(3 * (((t & 1 ? e[k].y : e[k].x) >> 4) & 3) + M.loc[t >> 1]) * G.nufp + iu[k][t]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    cd sf[2] = {ff[e[k].x & 7], ff[e[k].y & 7]};
+    if (e[k].x & 8) sf[0] = -sf[0];
+    if (e[k].y & 8) sf[1] = -sf[1];
+    if (!two[k]) sf[1] = mkcd(0, 0);
+    z[k] = mkcd(0, 0);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) z[k] = cmac(z[k], M.flag[t >> 1] * sf[t & 1], v[k][t]);
+  }
+}
+
 // Z[m, n], row-major (z64 with leading dimension ld, the FP32 planes with ldf), one 32 x 64
 // tile per CTA of 32 x 8 threads.  The gathers run with a warp along the 32 rows of a tile
 // column (consecutive match basis functions against one source basis function: consecutive
@@ -214,36 +248,14 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) k_assemble(SheetDev G, const
   if constexpr (TWO) {
 #pragma unroll
     for (int k0 = 0; k0 < 8; k0 += 4) {
-      int2 e[4];   // the column's packed incidences
-      bool two[4];
-      int iu[4][4];
-      cd v[4][4];
+      int n[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int n = min(n0 + ty + 8 * (k0 + k), G.nbf - 1);
-        e[k] = __ldg(reinterpret_cast<const int2 *>(G.inc + n));
-        two[k] = __ldg(G.inc_cnt + n) > 1;
-        if (!two[k]) e[k].y = e[k].x;
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-          iu[k][t] = __ldg(G.ufpm + (size_t)M.face[t >> 1] + (size_t)((t & 1 ? e[k].y : e[k].x) >> 8) * G.nface);
-      }
+      for (int k = 0; k < 4; ++k) n[k] = min(n0 + ty + 8 * (k0 + k), G.nbf - 1);
+      cd z[4];
+      assemble_four(G, ff, zb, M, n, z);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-          v[k][t] = ld_cd(zb + (size_t)(3 * (((t & 1 ? e[k].y : e[k].x) >> 4) & 3) + M.loc[t >> 1]) * G.nufp + iu[k][t]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cd sf[2] = {ff[e[k].x & 7], ff[e[k].y & 7]};
-        if (e[k].x & 8) sf[0] = -sf[0];
-        if (e[k].y & 8) sf[1] = -sf[1];
-        if (!two[k]) sf[1] = mkcd(0, 0);
-        cd acc = mkcd(0, 0);
-#pragma unroll
-        for (int t = 0; t < 4; ++t) acc = cmac(acc, M.flag[t >> 1] * sf[t & 1], v[k][t]);
-        *reinterpret_cast<double2 *>(&tile[tx][ty + 8 * (k0 + k)]) = make_double2(acc.x, acc.y);
-      }
+        *reinterpret_cast<double2 *>(&tile[tx][ty + 8 * (k0 + k)]) = make_double2(z[k].x, z[k].y);
     }
   } else {
 #pragma unroll
@@ -284,7 +296,7 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 3) k_assemble(SheetDev G, const
 // of G[a + b*nm] = sum_m Lam[m, a] y[m, b] to part[x + y*gridDim.x] (rows in a fixed order, no
 // atomics: the shares are added in a fixed order by k_adj_reduce, so the result is deterministic).
 // Vectors are nbf x nm column-major.
-template <int kAdjNB>
+template <int kAdjNB, bool TWO>
 __global__ void __launch_bounds__(256, 2) k_adj_contract(SheetDev G, const PointParams *__restrict__ Pp,
                                                       const cd *__restrict__ zb, const cd *__restrict__ X,
                                                       const cd *__restrict__ R, const cd *__restrict__ Lam, int nm,
@@ -307,12 +319,29 @@ __global__ void __launch_bounds__(256, 2) k_adj_contract(SheetDev G, const Point
     const int mc = min(m, nbf - 1);  // rows past the end repeat the last and are dropped below
     RowInc M;
     unpack_inc(__ldg(G.inc + mc), ff, __ldg(G.inc_cnt + mc), true, M);
-#pragma unroll 2
-    for (int n = c0 + ty; n < c1; n += 8) {
-      const cd z = assemble_entry(G, ff, res, zb, M, n);
+    if constexpr (TWO) {
+      for (int nn = c0 + ty; nn < c1; nn += 32) {
+        int n[4];
+        cd z[4];
 #pragma unroll
-      for (int b = 0; b < kAdjNB; ++b)
-        if (b < nb) acc[b] = cmac(acc[b], z, X[(size_t)(b0 + b) * nbf + n]);
+        for (int k = 0; k < 4; ++k) n[k] = min(nn + 8 * k, c1 - 1);
+        assemble_four(G, ff, zb, M, n, z);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (nn + 8 * k >= c1) break;
+#pragma unroll
+          for (int b = 0; b < kAdjNB; ++b)
+            if (b < nb) acc[b] = cmac(acc[b], z[k], X[(size_t)(b0 + b) * nbf + n[k]]);
+        }
+      }
+    } else {
+#pragma unroll 2
+      for (int n = c0 + ty; n < c1; n += 8) {
+        const cd z = assemble_entry(G, ff, res, zb, M, n);
+#pragma unroll
+        for (int b = 0; b < kAdjNB; ++b)
+          if (b < nb) acc[b] = cmac(acc[b], z, X[(size_t)(b0 + b) * nbf + n]);
+      }
     }
   }
 #pragma unroll
@@ -365,7 +394,9 @@ void pss_adj_contract(const SheetDev &G, const PointParams *dP1, const cd *zb, c
   const int nblk = cdiv_u(G.nbf, 32);
   for (int b0 = 0; b0 < nm;) {  // four right-hand sides at a time where that is all there is
     const int nb = nm - b0 <= 4 ? 4 : 8;
-    auto kern = nb == 4 ? k_adj_contract<4> : k_adj_contract<8>;
+    const bool two = G.two_inc && !G.has_res;
+    auto kern = nb == 4 ? (two ? k_adj_contract<4, true> : k_adj_contract<4, false>)
+                        : (two ? k_adj_contract<8, true> : k_adj_contract<8, false>);
     pss_count_launch();
     kern<<<dim3(nblk, kAdjChunks), dim3(32, 8), 0, st>>>(G, dP1, zb, X, R, Lam, nm, b0, part);
     b0 += nb;
