@@ -603,6 +603,13 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     hfv[i] = (int)(fv[i] - 1);
     if (fe[i] < 1 || fe[i] > nedge) { pss_set_error("fe[%lld] out of range", (long long)i); delete sh; return -1; }
   }
+  auto refuse = [&](int rc) {  // what is on the device by now goes with the sheet
+    for (DevBuf *d : {&sh->rho, &sh->fv, &sh->ufpm, &sh->rep, &sh->fr, &sh->ls, &sh->a48, &sh->inc_cnt, &sh->inc_face,
+                      &sh->inc_loc, &sh->inc_sgn, &sh->inc_eci, &sh->face_m, &sh->pfaces, &sh->inc})
+      d->release();
+    delete sh;
+    return rc;
+  };
   // The class map and the representatives are converted to 0-based int32 on the device, which
   // also checks their range (the map keeps the reference's order, match face fastest: the assembly
   // gathers a column of a Z tile - consecutive match faces against one source face - whose classes
@@ -613,10 +620,8 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     int hbad[2] = {0, 0};
     if (raw.ensure(std::max(np2, (size_t)nufp) * sizeof(int64_t)) || upload(bad, hbad, 2) ||
         sh->ufpm.ensure(np2 * sizeof(int)) || sh->rep.ensure(nufp * sizeof(int)) ||
-        sh->pfaces.ensure(nufp * sizeof(int2))) {
-      delete sh;
-      return -3;
-    }
+        sh->pfaces.ensure(nufp * sizeof(int2)))
+      return refuse(-3);
     auto convert = [&]() -> int {
       PSS_CUDA_TRY(cudaMemcpy(raw.p, ufpm, np2 * sizeof(int64_t), cudaMemcpyHostToDevice));
       pss_count_launch();
@@ -632,7 +637,7 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     int rc = convert();
     if (!rc && hbad[0]) { pss_set_error("ufpm entry out of range"); rc = -1; }
     if (!rc && hbad[1]) { pss_set_error("ufp_rep out of range"); rc = -1; }
-    if (rc) { sh->rep.release(); sh->ufpm.release(); sh->pfaces.release(); delete sh; return rc; }
+    if (rc) return refuse(rc);
   }
   // basis-function incidences: (face, local edge, sign, edge code), fixed order
   std::vector<int> icnt(nbf, 0), iface(4 * nbf, 0), iloc(4 * nbf, 0), isgn(4 * nbf, 0), ieci(4 * nbf, 0);
@@ -641,15 +646,15 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
       int64_t e = fe[3 * f + k];
       int64_t b = ebf[e - 1];
       if (b == 0) continue;
-      if (b < 1 || b > nbf) { pss_set_error("ebf entry out of range"); delete sh; return -1; }
+      if (b < 1 || b > nbf) { pss_set_error("ebf entry out of range"); return refuse(-1); }
       int sgn;
       if (bff[2 * (b - 1)] - 1 == f) sgn = 1;
       else if (bff[2 * (b - 1) + 1] - 1 == f) sgn = -1;
-      else { pss_set_error("Impossible situation in edge loop (face %lld, bf %lld)", (long long)f + 1, (long long)b); delete sh; return -1; }
+      else { pss_set_error("Impossible situation in edge loop (face %lld, bf %lld)", (long long)f + 1, (long long)b); return refuse(-1); }
       int &cnt = icnt[b - 1];
-      if (cnt >= 4) { pss_set_error("basis function %lld has more than 4 face incidences", (long long)b); delete sh; return -1; }
+      if (cnt >= 4) { pss_set_error("basis function %lld has more than 4 face incidences", (long long)b); return refuse(-1); }
       int64_t code = eci[e - 1];
-      if (code < 0 || code > 4) { pss_set_error("eci entry out of range"); delete sh; return -1; }
+      if (code < 0 || code > 4) { pss_set_error("eci entry out of range"); return refuse(-1); }
       iface[4 * (b - 1) + cnt] = (int)f;
       iloc[4 * (b - 1) + cnt] = k;
       isgn[4 * (b - 1) + cnt] = sgn;
@@ -705,7 +710,7 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
   rc |= upload(sh->inc_eci, ieci.data(), ieci.size());
   rc |= upload(sh->face_m, hfm.data(), hfm.size());
   rc |= upload(sh->inc, hinc.data(), hinc.size());
-  if (rc) { delete sh; return -3; }
+  if (rc) return refuse(-3);
   SheetDev &G = sh->G;
   G.nface = sh->nface; G.nbf = sh->nbf; G.nufp = sh->nufp; G.nnode = sh->nnode; G.upm = units_per_meter;
   G.rho = sh->rho.as<double>(); G.fv = sh->fv.as<int>(); G.ufpm = sh->ufpm.as<int>(); G.ufp_rep = sh->rep.as<int>();

@@ -4,7 +4,10 @@
 // few bytes to hundreds of megabytes; cudaMalloc and cudaFree of those, each with its
 // synchronisation and page mapping, took longer than the device work of a small sheet (15 ms of a
 // two-sheet stack, 9 ms of a sheet of 1648 faces).  The pool keeps up to kKeep bytes of freed
-// memory mapped and is emptied when a context is destroyed or an allocation fails.
+// memory mapped and is emptied when a context is destroyed or an allocation fails.  A pool's
+// release threshold counts the memory in use as well, so it follows that: with a fixed one the
+// buffers of a large sweep alone exceeded it, every synchronisation unmapped all that was free,
+// and setting a sheet of 3960 faces up took 500 ms instead of 93.
 #include "pss_internal.cuh"
 
 namespace {
@@ -41,6 +44,14 @@ int current_pool(Pool **out) {
   return 0;
 }
 
+// At most kKeep bytes beyond what is in use stay mapped.
+void follow_use(Pool *q) {
+  unsigned long long used = 0;
+  if (cudaMemPoolGetAttribute(q->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
+  unsigned long long keep = used + kKeep;
+  cudaMemPoolSetAttribute(q->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 }  // namespace
 
 // Memory of the current device, usable on every stream when the call returns.
@@ -55,7 +66,10 @@ int pss_dev_alloc(void **p, size_t bytes) {
     cudaMemPoolTrimTo(q->pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, q->pool, q->st);
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(q->st);
+  if (e == cudaSuccess) {
+    follow_use(q);
+    e = cudaStreamSynchronize(q->st);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -71,6 +85,7 @@ void pss_dev_free(void *p) {
   if (!p || current_pool(&q)) return;
   cudaDeviceSynchronize();
   cudaFreeAsync(p, q->st);
+  follow_use(q);
 }
 
 void pss_dev_trim() {
