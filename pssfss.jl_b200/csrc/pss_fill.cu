@@ -352,8 +352,10 @@ __global__ void __launch_bounds__(256, 2) k_adj_contract(SheetDev G, const Point
     for (int b = 0; b < kAdjNB; ++b) {
       cd sdot = mkcd(0, 0);
       for (int w = 0; w < 8; ++w) sdot = sdot + red[w][tx][b];
-      const cd rb = blockIdx.y == 0 ? R[(size_t)(b0 + b) * nbf + m] : mkcd(0, 0);
-      yrow[tx][b] = (m < nbf && b < nb) ? rb - sdot : mkcd(0, 0);
+      // rows past the last and right-hand sides past nm lie outside R: they are not read
+      const bool ok = m < nbf && b < nb;
+      const cd rb = ok && blockIdx.y == 0 ? R[(size_t)(b0 + b) * nbf + m] : mkcd(0, 0);
+      yrow[tx][b] = ok ? rb - sdot : mkcd(0, 0);
     }
   }
   __syncthreads();
