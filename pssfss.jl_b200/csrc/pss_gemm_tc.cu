@@ -460,8 +460,7 @@ int make_map(CUtensorMap *m, const float *planes, int rows, int KP, int nplanes)
   return 0;
 }
 
-constexpr int kMaxDevices = 64;
-int g_num_sms[kMaxDevices] = {};  // per device, written once under g_setup
+int g_num_sms[kMaxDevices] = {};  // per device, written under g_setup
 DeviceOnce g_setup;
 std::atomic<long long> g_wait_cap{kWaitCap};  // pss_set_wait_limit
 

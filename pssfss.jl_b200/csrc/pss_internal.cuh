@@ -6,25 +6,28 @@
 #include "pss_common.cuh"
 #include "pssfss_b200.h"
 
-// Per-device one-time set-up (kernel attributes and the like), safe to reach from several
-// host threads: f() runs once for each device it is first called on (that device current).
+// The current device and the identifier of its current CUDA context (pss_mem.cu).  A context's
+// handle comes back after a reset of the device, its identifier does not.
+constexpr int kMaxDevices = 64;
+int pss_context_id(int *dev, unsigned long long *id);
+
+// One-time set-up per device and context (kernel attributes and the like), safe to reach from
+// several host threads: f() runs once for each context it is first called in (that context
+// current), so what it sets is set again after a device reset.
 struct DeviceOnce {
-  std::atomic<unsigned long long> done{0};
+  std::atomic<unsigned long long> done[kMaxDevices] = {};  // the context's identifier (from 1 on)
   std::mutex mu;
 };
 template <class F>
 int device_once(DeviceOnce &o, F &&f) {
   int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-    pss_set_error("no usable current device (%d) for kernel set-up", dev);
-    return -3;
-  }
-  const unsigned long long bit = 1ull << dev;
-  if (o.done.load(std::memory_order_acquire) & bit) return 0;
+  unsigned long long id = 0;
+  if (int rc = pss_context_id(&dev, &id)) return rc;
+  if (o.done[dev].load(std::memory_order_acquire) == id) return 0;
   std::lock_guard<std::mutex> lk(o.mu);
-  if (o.done.load(std::memory_order_relaxed) & bit) return 0;
+  if (o.done[dev].load(std::memory_order_relaxed) == id) return 0;
   const int rc = f();
-  if (!rc) o.done.fetch_or(bit, std::memory_order_release);
+  if (!rc) o.done[dev].store(id, std::memory_order_release);
   return rc;
 }
 

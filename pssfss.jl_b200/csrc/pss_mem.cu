@@ -8,12 +8,16 @@
 // release threshold counts the memory in use as well, so it follows that: with a fixed one the
 // buffers of a large sweep alone exceeded it, every synchronisation unmapped all that was free,
 // and setting a sheet of 3960 faces up took 500 ms instead of 93.
+//
+// A pool and its stream end with their context (a device reset), so both are made anew when the
+// device's context is another one than theirs.
+#include <cuda.h>
+
 #include "pss_internal.cuh"
 
 namespace {
 
 constexpr unsigned long long kKeep = 2ull << 30;
-constexpr int kMaxDevices = 64;
 
 struct Pool {
   cudaMemPool_t pool = nullptr;
@@ -24,8 +28,8 @@ DeviceOnce g_once;
 
 int current_pool(Pool **out) {
   int dev = 0;
-  PSS_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxDevices) { pss_set_error("device %d out of range", dev); return -3; }
+  unsigned long long id = 0;
+  if (int rc = pss_context_id(&dev, &id)) return rc;
   if (int rc = device_once(g_once, [dev] {
         Pool p;
         cudaMemPoolProps props = {};
@@ -52,7 +56,46 @@ void follow_use(Pool *q) {
   cudaMemPoolSetAttribute(q->pool, cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
+using CtxGetCurrentFn = CUresult (*)(CUcontext *);
+using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long *);
+struct DriverFns {
+  CtxGetCurrentFn current = nullptr;
+  CtxGetIdFn id = nullptr;
+};
+
+template <class Fn>
+bool driver_fn(const char *name, Fn &out) {
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+    return false;
+  out = (Fn)fn;
+  return fn != nullptr;
+}
+
 }  // namespace
+
+int pss_context_id(int *dev, unsigned long long *id) {
+  static const DriverFns drv = [] {
+    DriverFns d;
+    if (!driver_fn("cuCtxGetCurrent", d.current) || !driver_fn("cuCtxGetId", d.id)) d = DriverFns{};
+    return d;
+  }();
+  if (!drv.id) { pss_set_error("cuCtxGetCurrent or cuCtxGetId unavailable"); return -3; }
+  *dev = -1;
+  PSS_CUDA_TRY(cudaGetDevice(dev));
+  if (*dev < 0 || *dev >= kMaxDevices) { pss_set_error("device %d out of range", *dev); return -3; }
+  auto read = [&] {
+    CUcontext ctx = nullptr;
+    return drv.current(&ctx) == CUDA_SUCCESS && ctx && drv.id(ctx, id) == CUDA_SUCCESS;
+  };
+  if (read()) return 0;
+  cudaFree(nullptr);  // the device's context is not there yet, or was reset: the runtime makes it
+  if (read()) return 0;
+  cudaGetLastError();
+  pss_set_error("no current CUDA context on device %d", *dev);
+  return -3;
+}
 
 // Memory of the current device, usable on every stream when the call returns.
 int pss_dev_alloc(void **p, size_t bytes) {

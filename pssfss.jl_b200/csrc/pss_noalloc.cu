@@ -24,11 +24,9 @@
 //   * the first call on each device resolves the scratch array's address with
 //     cudaGetSymbolAddress (a one-time set-up, done with that device current); make that
 //     first call before any stream capture on the device.  The address belongs to the
-//     device's current CUDA context: it is cached together with that context's handle and
+//     device's current CUDA context: it is cached together with that context's identifier and
 //     resolved again when a call finds another context current (after cudaDeviceReset, or
 //     a context the caller created itself), so a stale address is never used.
-#include <cuda.h>
-
 #include <mutex>
 
 #include "pss_internal.cuh"
@@ -42,38 +40,16 @@ constexpr size_t kScratchBytes = 1024;
 
 static __device__ __align__(256) unsigned char g_lu_scratch[kScratchBytes];
 
-constexpr int kMaxDevices = 64;
 void *g_scratch_ptr[kMaxDevices] = {};
-CUcontext g_scratch_ctx[kMaxDevices] = {};  // the context each cached address belongs to
+unsigned long long g_scratch_ctx[kMaxDevices] = {};  // the context each cached address belongs to
 std::mutex g_setup_mu;
-
-using CtxGetCurrentFn = CUresult (*)(CUcontext *);
-CtxGetCurrentFn g_ctx_get_current = nullptr;  // cuCtxGetCurrent, resolved once under g_setup_mu
 
 // Set-up per device (the caller's current device) and context: the array's device address.
 int scratch_for_current_device(void **out) {
   int dev = -1;
-  PSS_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxDevices) {
-    pss_set_error("device %d out of range for the no-allocation scratch table", dev);
-    return -3;
-  }
+  unsigned long long ctx = 0;
+  if (int rc = pss_context_id(&dev, &ctx)) return rc;
   std::lock_guard<std::mutex> lk(g_setup_mu);
-  if (!g_ctx_get_current) {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn) {
-      pss_set_error("cuCtxGetCurrent unavailable");
-      return -3;
-    }
-    g_ctx_get_current = (CtxGetCurrentFn)fn;
-  }
-  CUcontext ctx = nullptr;
-  if (g_ctx_get_current(&ctx) != CUDA_SUCCESS || !ctx) {
-    pss_set_error("no current CUDA context on device %d", dev);
-    return -3;
-  }
   if (!g_scratch_ptr[dev] || g_scratch_ctx[dev] != ctx) {
     void *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_lu_scratch);
