@@ -68,6 +68,7 @@ void pss_set_error(const char *fmt, ...) {
 namespace {
 
 constexpr int kRing0 = 160;  // ring budget of the first table pass (mmax <= 320)
+constexpr size_t kSystemPiece = 64ull << 20;  // bytes of a caller's matrix on the device beside its transpose
 constexpr int kMaxRefine = 10;  // refinement steps before the FP64 fallback (zcgesv allows 30)
 
 struct DevBuf {
@@ -198,15 +199,16 @@ __global__ void k_class_reps(long long nufp, int nface, const long long *__restr
   faces[i] = make_int2(p % nface, p / nface);
 }
 
-// Column-major n x n system (pss_lu_solve) to the row-major FP64 matrix and, in the FP32 form, the
-// float planes with their padding zeroed; 32 x 32 tiles through shared memory.
-__global__ void __launch_bounds__(256) k_system_rows(int n, const cd *__restrict__ Z, cd *__restrict__ A,
+// Columns cb, cb + 1, ... of a column-major n x n system (pss_lu_solve; Z holds them from column
+// cb on) to the row-major FP64 matrix and, in the FP32 form, the float planes with their padding
+// zeroed; 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) k_system_rows(int n, int cb, const cd *__restrict__ Z, cd *__restrict__ A,
                                                      float *__restrict__ Ar, float *__restrict__ Ai, long long ldf) {
   __shared__ cd tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  const int c0 = cb + blockIdx.x * 32, r0 = blockIdx.y * 32;
   for (int y = ty; y < 32; y += 8)
-    tile[y][tx] = (c0 + y < n && r0 + tx < n) ? Z[(size_t)(c0 + y) * n + r0 + tx] : mkcd(0, 0);
+    tile[y][tx] = (c0 + y < n && r0 + tx < n) ? Z[(size_t)(c0 - cb + y) * n + r0 + tx] : mkcd(0, 0);
   __syncthreads();
   for (int y = ty; y < 32; y += 8) {
     const int r = r0 + y, c = c0 + tx;
@@ -1397,17 +1399,25 @@ int pss_lu_solve(pss_ctx *c, int n, const double *Z, int nrhs, const double *B, 
   const size_t nn = (size_t)n * n;
   const bool f32 = precision == PSS_FP32_REFINE;
   const size_t ldf = (size_t)Worker::ld32(n), nf = (size_t)n * ldf;
-  LocalBuf raw, st_buf;  // the caller's column-major matrix, transposed on the device
-  if (raw.ensure(nn * sizeof(cd)) || w.z64.ensure(nn * sizeof(cd)) || w.ensure_solver(n, nrhs, 1)) return -3;
+  // the caller's column-major matrix is transposed on the device a piece of its columns at a time:
+  // one more copy of the whole matrix would halve the orders that fit beside a host's own pool
+  const int piece = std::max(32, std::min((n + 31) & ~31, (int)(kSystemPiece / ((size_t)n * sizeof(cd))) & ~31));
+  LocalBuf raw, st_buf;
+  if (raw.ensure((size_t)std::min(piece, n) * n * sizeof(cd)) || w.z64.ensure(nn * sizeof(cd)) ||
+      w.ensure_solver(n, nrhs, 1))
+    return -3;
   if (f32 && (w.zr.ensure(nf * sizeof(float)) || w.zi.ensure(nf * sizeof(float)))) return -3;
   if (st_buf.ensure(sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemsetAsync(st_buf.p, 0, sizeof(int), st));
   PSS_CUDA_TRY(cudaMemsetAsync(w.info.p, 0, sizeof(int), st));
-  PSS_CUDA_TRY(cudaMemcpyAsync(raw.p, Z, nn * sizeof(cd), cudaMemcpyHostToDevice, st));
+  for (int cb = 0; cb < n; cb += piece) {
+    const int cols = std::min(piece, n - cb);
+    PSS_CUDA_TRY(cudaMemcpyAsync(raw.p, Z + 2 * (size_t)cb * n, (size_t)cols * n * sizeof(cd), cudaMemcpyHostToDevice, st));
+    pss_count_launch();
+    k_system_rows<<<dim3(cdiv_u(cols, 32), cdiv_u(n, 32)), 256, 0, st>>>(
+        n, cb, raw.as<cd>(), w.z64.as<cd>(), f32 ? w.zr.as<float>() : nullptr, f32 ? w.zi.as<float>() : nullptr, (long long)ldf);
+  }
   PSS_CUDA_TRY(cudaMemcpyAsync(w.rhs.p, B, (size_t)n * nrhs * sizeof(cd), cudaMemcpyHostToDevice, st));
-  pss_count_launch();
-  k_system_rows<<<dim3(cdiv_u((long long)ldf, 32), cdiv_u(n, 32)), 256, 0, st>>>(
-      n, raw.as<cd>(), w.z64.as<cd>(), f32 ? w.zr.as<float>() : nullptr, f32 ? w.zi.as<float>() : nullptr, (long long)ldf);
   int rc;
   if ((rc = w.factor_solve(n, 1, precision, nrhs, kMaxRefine, st_buf.as<int>()))) return rc;
   PSS_CUDA_TRY(cudaStreamSynchronize(st));
