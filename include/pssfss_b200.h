@@ -58,6 +58,14 @@ int64_t pss_kernel_launches(void);
 /* One context per device; nworkers CUDA streams process frequency points concurrently. */
 int pss_ctx_create(int device, int nworkers, pss_ctx **out);
 int pss_ctx_destroy(pss_ctx *ctx);
+/* Device memory that the library frees (a sheet's arrays, a call's scratch) stays with it for its
+ * next calls, up to 2 GiB per device beyond what is in use; no other allocator of the process sees
+ * it meanwhile.  This call gives it back to the driver, after waiting for the device; the buffers
+ * that contexts and sheets hold stay.  Destroying a context gives it back too, and an allocation
+ * of the library's own that fails does so before it tries again.  A host whose own pool
+ * (CUDA.jl, PyTorch) needs the memory calls it between two phases of work, or when that pool
+ * runs out. */
+int pss_release_memory(pss_ctx *ctx);
 /* The device a context runs on. */
 int pss_ctx_device(const pss_ctx *ctx, int *device);
 

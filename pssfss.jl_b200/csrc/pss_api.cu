@@ -575,6 +575,12 @@ int pss_ctx_destroy(pss_ctx *c) {
   return 0;
 }
 
+int pss_release_memory(pss_ctx *c) {
+  if (!c) { pss_set_error("null argument"); return -1; }
+  if (set_device(c)) return -3;
+  return pss_dev_trim();
+}
+
 int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const double *s1, const double *s2,
                      const double *beta1, const double *beta2, int64_t nnode, const double *rho,
                      int64_t nface, const int64_t *fv, const int64_t *fe, const double *fr, int64_t nedge,

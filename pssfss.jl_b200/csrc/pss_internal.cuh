@@ -174,7 +174,7 @@ extern "C" int pss_ctx_device(const pss_ctx *c, int *dev);
 // Device memory (pss_mem.cu): a bounded pool per device with cudaMalloc / cudaFree semantics.
 int pss_dev_alloc(void **p, size_t bytes);
 void pss_dev_free(void *p);
-void pss_dev_trim();  // gives the current device's kept memory back
+int pss_dev_trim();  // gives the current device's kept memory back
 
 // Counts every kernel the library launches (reported by pss_kernel_launches()).
 void pss_count_launch();

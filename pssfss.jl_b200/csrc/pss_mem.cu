@@ -4,7 +4,8 @@
 // few bytes to hundreds of megabytes; cudaMalloc and cudaFree of those, each with its
 // synchronisation and page mapping, took longer than the device work of a small sheet (15 ms of a
 // two-sheet stack, 9 ms of a sheet of 1648 faces).  The pool keeps up to kKeep bytes of freed
-// memory mapped and is emptied when a context is destroyed or an allocation fails.  A pool's
+// memory mapped and is emptied when a context is destroyed, an allocation fails or the caller asks
+// (pss_release_memory: no other allocator of the process can use what the pool keeps).  A pool's
 // release threshold counts the memory in use as well, so it follows that: with a fixed one the
 // buffers of a large sweep alone exceeded it, every synchronisation unmapped all that was free,
 // and setting a sheet of 3960 faces up took 500 ms instead of 93.
@@ -131,9 +132,10 @@ void pss_dev_free(void *p) {
   follow_use(q);
 }
 
-void pss_dev_trim() {
+int pss_dev_trim() {
   Pool *q = nullptr;
-  if (current_pool(&q)) return;
-  cudaDeviceSynchronize();
-  cudaMemPoolTrimTo(q->pool, 0);
+  if (int rc = current_pool(&q)) return rc;
+  PSS_CUDA_TRY(cudaDeviceSynchronize());
+  PSS_CUDA_TRY(cudaMemPoolTrimTo(q->pool, 0));
+  return 0;
 }

@@ -42,6 +42,7 @@ SIGNATURES = {
     "pss_kernel_launches": (_L, []),
     "pss_ctx_create": (_I, [_I, _I, _P]),
     "pss_ctx_destroy": (_I, [_P]),
+    "pss_release_memory": (_I, [_P]),
     "pss_ctx_device": (_I, [_P, _P]),
     "pss_cascade": (_I, [_P, _I, _I, _P, _P, _P, _P, _P]),
     "pss_face_pair_classes": (_I, [_P, _L, _P, _P, _P, _D, _P, _P, _L, _P]),
@@ -156,6 +157,12 @@ def context(device=0, nworkers=None):
             _check(L.pss_ctx_create(device, nworkers, ctypes.byref(h)), "pss_ctx_create")
             c = _ctx[key] = h
     return c
+
+
+def release_memory(device=0, nworkers=None):
+    """Give the freed device memory that the library keeps for its next calls (up to 2 GiB beyond
+    what is in use) back to the driver, for PyTorch or another allocator (``pss_release_memory``)."""
+    _check(lib().pss_release_memory(context(device, nworkers)), "pss_release_memory")
 
 
 def region_arrays(layers):
