@@ -422,7 +422,7 @@ int pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi
   }
   const double a = ulocal * s1[0], b = ulocal * s1[1], c = ulocal * s2[0], d = ulocal * s2[1];
   JKTabPlan plan;
-  if (pss_jktab_plan(G, ulocal, s1, s2, pg.n, plan) && ws && ws_bytes >= plan.bytes)
+  if (pss_jktab_plan(G, ulocal, s1, s2, pg.n, plan) && ws_bytes >= plan.bytes)
     return pss_jktab_launch(G, ulocal, pg, s1, s2, jg, nonconv, plan, ws, st);
   const long long lanes = (long long)G.nufp * 8;
   pss_count_launch();

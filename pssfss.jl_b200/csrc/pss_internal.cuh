@@ -201,7 +201,7 @@ int pss_tables_finish(const cd *dense, size_t pstride, int R, int mmax, const Po
 size_t pss_table_cap(int mmax);  // (mmax+2)^2 entries per padded table
 
 // Face-pair integrals and matrix fill (pss_fill.cu)
-// ws: scratch of pss_jktab_bytes (may be null: every pair's lattice sums then run ring by ring).
+// ws: scratch of at least pss_jktab_bytes; in a smaller one every pair's lattice sums run ring by ring.
 int pss_filljk(const SheetDev &G, double ulocal, double psi1, double psi2, const double s1[2], const double s2[2],
                JKDev jk, int *nonconv, void *ws, size_t ws_bytes, cudaStream_t st);
 // np <= kJKGroup phasings at once into jk[0..np), non-convergence counts into nonconv[0..np)

@@ -50,7 +50,6 @@ struct TabDev {
   double *val[kJKGroup];          // [panel][R0 / R0+1][node a][J, K][node b] (real: one double each)
   double *ring[kJKGroup];         // ring R0 alone at the nodes, laid out like one slot of val
   unsigned char *flag[kJKGroup];  // per panel: 0 whole, 1 map, 2 direct
-  unsigned char *r0[kJKGroup];
   unsigned char *map[kJKGroup];   // [panel][kSub][kSub]
   int *list, *count;              // pairs left to the direct form, per phasing
 };
@@ -172,10 +171,7 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
   if (near_zero(js, corner[0]) || near_zero(ks, corner[1])) atomicMax(&hi, 1000);
   __syncthreads();
   const bool direct = lo == 1000;
-  if (tid == 0) {
-    T.flag[p][panel] = direct ? 2 : hi == lo ? 0 : 1;
-    T.r0[p][panel] = (unsigned char)(direct ? kRMin : lo);
-  }
+  if (tid == 0) T.flag[p][panel] = direct ? 2 : hi == lo ? 0 : 1;
   const int r0 = direct ? 1 : lo - (kRMin - 1);
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -605,7 +601,7 @@ bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const 
   P.b0 = -W2;
   P.ra = P.na / (2 * W1);
   P.rb = P.nb / (2 * W2);
-  const size_t per = align256(panels * 3 * 64 * 4 * sizeof(double)) + 2 * align256(panels) + align256(panels * kSub * kSub);
+  const size_t per = align256(panels * 3 * 64 * 4 * sizeof(double)) + align256(panels) + align256(panels * kSub * kSub);
   P.bytes = (size_t)np * (per + (size_t)G.nufp * sizeof(int)) + 512;
   return true;
 }
@@ -630,7 +626,6 @@ int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const
     T.ring[p] = T.val[p] + panels * 2 * 64 * 4;
     w += align256(panels * 3 * 64 * 4 * sizeof(double));
     T.flag[p] = (unsigned char *)w; w += align256(panels);
-    T.r0[p] = (unsigned char *)w; w += align256(panels);
     T.map[p] = (unsigned char *)w; w += align256(panels * kSub * kSub);
   }
   T.count = (int *)w; w += 64;

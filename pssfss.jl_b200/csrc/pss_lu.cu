@@ -43,8 +43,6 @@ template <class E>
 __device__ __forceinline__ E cmulE(E a, E b) { return E{a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
 template <class E>
 __device__ __forceinline__ E csubE(E a, E b) { return E{a.x - b.x, a.y - b.y}; }
-template <class E>
-__device__ __forceinline__ E caddE(E a, E b) { return E{a.x + b.x, a.y + b.y}; }
 
 // Matrix accessor: FP64 interleaved (A), FP32 planes (Ar, Ai).
 template <bool F32>
