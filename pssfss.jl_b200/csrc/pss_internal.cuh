@@ -213,6 +213,7 @@ int pss_filljk_group(const SheetDev &G, double ulocal, int np, const double *psi
 struct JKTabPlan {
   int na = 0, nb = 0;  // panels along the two lattice vectors
   double a0 = 0, b0 = 0, ra = 0, rb = 0;  // first panel's corner; panels per unit lattice coordinate
+  double dmin = 0;     // distance of the offsets to the nearest image of ring 2 (u-scaled)
   size_t bytes = 0;
 };
 bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const double s2[2], int np, JKTabPlan &P);

@@ -8,22 +8,30 @@
 //     Chebyshev nodes.  A panel's half-width is at most 1/48 of the distance D to the nearest
 //     tabulated image: the Bernstein ellipse through that image has radius 96 in both
 //     directions, so the interpolation error is about 96^-8 = 1.4e-16 of the far sum, which is
-//     itself at most a few tenths of the whole;
+//     itself at most a few tenths of the whole.  Nor is a half-width above 0.15, where e^-d's own
+//     change over a panel adds h^8 / (2^7 8!) = 5e-14 of the far sum; panels that wide belong to
+//     compact sheets, whose far sum is below 1 % of the whole;
 //   * the reference stops a sum at its own ring R (relative change below 1e-8), so R is part of
 //     the result.  R depends on the offset alone: a panel stores the far sum through ring R0
-//     and through R0 + 1.  Panels whose nodes all stop at R0, clear of the threshold, are taken
-//     as a whole; the others carry a map of 32 x 32 sub-cells that says R0, R0 + 1 or unknown.
-//     Near a zero of a sum its relative change, and so R, is large: where the values at the
-//     nodes (corners) are not larger than their differences, the panel needs a map (the
-//     sub-cell is unknown);
-//   * pairs with a point in an unknown sub-cell (about 0.3-0.5 % of the points) go to a list
-//     and through the direct form (filljk_pair), bit for bit as before.
+//     and through R0 + 1, R0 the first ring that not every point of the panel surely passes over.
+//     Panels whose points all surely stop at R0 are taken as a whole; the others carry a map of
+//     32 x 32 sub-cells that says R0, R0 + 1 or unknown;
+//   * "surely" is a bound, not a sample.  A node speaks for the points within the distance de of
+//     it (which together cover the panel) by the sums' Lipschitz constants; in a sub-cell a sum
+//     lies within (wa^2 + wb^2)/8 times its second derivative of the convex hull of its four
+//     corner values, so its modulus is bounded on both sides.  The constants come from the same
+//     summands without their phases.  So zeros of a ring's sum (the reference may stop there
+//     early) and of the whole sum are seen however small their surroundings are;
+//   * pairs with a point in an unknown sub-cell (at the sweeps' smoothing parameter 0.4-0.9 % of
+//     the points, up to 5 % at phasings of pi, whose real ring sums vanish along curves) go to a
+//     list and through the direct form (filljk_pair), bit for bit as before.
 // What bounds it: the direct form issues about 4200 FP64 operations per quadrature point and is
 // bound by the FP64 pipe; this one issues about 400 and reads 64 nodes from L1/L2.  A pair's
 // eight lanes own one column of the panel each, so a node row is one 128-byte line, and a lane
 // keeps its column in registers while consecutive quadrature points stay in the panel.
-// Measured (direct -> tabulated, tables included): 17.6 -> 3.2 ms for the 3.19M classes of the
-// N = 3976 meander at normal incidence, 18.1 -> 4.7 ms for four phasings of a ring of 1168 faces.
+// Measured (direct -> tabulated, tables included): 17.6 -> 2.9 ms for the 3.19M classes of the
+// N = 3976 meander at normal incidence (nodes 0.22, map 0.11, sums 2.20, list 0.41), 18.1 -> 4.75 ms
+// for four phasings of a ring of 1168 faces (0.38, 0.17, 3.47, 0.73).
 #include <algorithm>
 #include <cmath>
 
@@ -36,19 +44,26 @@ constexpr int kSub = 32;                // sub-cells per panel and direction
 constexpr int kRMin = 6;                // first ring the reference tests
 constexpr int kRec = 9;                 // far sums recorded at a node: through rings kRMin - 1 .. 13
 constexpr double kConv = 1e-8;          // its threshold
-// How far a node (sub-cell corner) must be from the threshold |ring| = kConv |sum| to speak for
-// its surroundings: a share of |sum| for the slope, and an absolute part for the curvature of the
-// sums, of order 1 in u-scaled lengths (a panel is at most 0.16 wide, a sub-cell 0.005).
-constexpr double kMargin = 0.1, kCurve = 3e-3;
-constexpr double kSubMargin = 1e-4, kSubCurve = 4e-6;
+constexpr double kTol = 1e-6;           // share of the threshold left to rounding on either side
+constexpr double kNodeGap = 0.1951;     // a point's distance from a node, in half-widths per direction
+// Growth of a derivative bound from where it is formed to the points it speaks for, e^t (1 - t/d)^-3
+// for a distance t from there and d to the image: rings 2 and beyond, d at least 48 half-widths and
+// t at most 0.39 of them (0.059); ring 1 at a node, d at least 4 t; ring 1 at a corner, d at least 4
+// sub-cell sides (0.019).
+constexpr double kFar = 1.1, kNear = 2.6;
+constexpr int kBounds = 6;
 constexpr int kMaxPanels = 8192;
 
 struct TabDev {
   double iv[4];           // u-scaled offset -> lattice coordinates
   double a0, b0, ra, rb;
+  double wa, wb;          // sides of a panel, u-scaled
+  double q;               // reciprocal of the distance to the nearest image of ring 2
   int na, nb;
   double *val[kJKGroup];          // [panel][R0 / R0+1][node a][J, K][node b] (real: one double each)
   double *ring[kJKGroup];         // ring R0 alone at the nodes, laid out like one slot of val
+  // per panel, bounds on second derivatives: ring R0 of J and K, ring R0 + 1, rings 2 .. R0 + 1
+  float *bound[kJKGroup];
   unsigned char *flag[kJKGroup];  // per panel: 0 whole, 1 map, 2 direct
   unsigned char *map[kJKGroup];   // [panel][kSub][kSub]
   int *list, *count;              // pairs left to the direct form, per phasing
@@ -60,39 +75,44 @@ __constant__ double c_node[kND] = {0.9807852804032304, 0.8314696123025452, 0.555
 __constant__ double c_nodew[kND] = {3.121445152258054, -8.889123728313642, 13.30351379684073, -15.692564486451692,
                                     15.692564486451692, -13.303513796840717, 8.889123728313624, -3.121445152258053};
 
-// Sums at one offset, ring by ring as in jksums; the far part (rings >= 2) through each ring r
-// in 5 .. 13 is handed to rec.  Returns the ring the reference stops at (0: beyond the record),
-// whether the test is clear of its threshold there (at) and one ring before (before), and the
-// sums.
-__device__ __forceinline__ bool clear_of(double ring, double sum, double margin, double curve, bool below) {
-  const double t = kConv * sum - ring, m = kConv * (margin * sum + curve);
-  return below ? t > m : t < -m;
-}
+// Sums at a node, ring by ring as in jksums; the far part (rings >= 2) through each ring r in
+// 5 .. 13 and the ring's sums without phases (r = 5: of rings 2 .. 5) are handed to rec.
+// Returns the first ring that some point within de of the node may stop at (0: beyond the record);
+// sure: all of them do.
+// Derivatives: |d1 (e^-d / d)| <= e^-d (1/d + 1/d^2), |d2 (e^-d / d)| <= e^-d (1/d + 2/d^2 + 2/d^3),
+// |d1 e^-d| <= e^-d, |d2 e^-d| <= e^-d (1 + 1/d).
+__device__ __forceinline__ double slope_of(double q) { return 1 + q; }  // per e^-d / d, 1/d <= q
+__device__ __forceinline__ double curve_of(double q) { return fma(2 * q, 1 + q, 1.0); }
 template <bool REAL, class Rec>
 __device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, double us1y, double us2x, double us2y,
                                           const cd *__restrict__ ph1, const cd *__restrict__ ph2,
-                                          const double *__restrict__ etab, bool &at, bool &before, cd &jsum, cd &ksum,
-                                          Rec &&rec) {
+                                          const double *__restrict__ etab, double de, double q, bool &sure, Rec &&rec) {
   const double arg = sqrt(urx * urx + ury * ury);
   const double rterm = exp_neg(arg, etab);
-  ksum = mkcd(rterm, 0.0);
-  jsum = arg <= 1e-5 ? mkcd((-arg / 6 + 0.5) * arg - 1, 0.0) : mkcd((rterm - 1) / arg, 0.0);
+  cd ksum = mkcd(rterm, 0.0);
+  cd jsum = arg <= 1e-5 ? mkcd((-arg / 6 + 0.5) * arg - 1, 0.0) : mkcd((rterm - 1) / arg, 0.0);
   cd jfar = mkcd(0, 0), kfar = jfar;
+  double lipj = 0.5, lipk = 1.0, farj = 0, fark = 0;  // Lipschitz constants: of the (0, 0) term
+  const double slope = kFar * slope_of(q);
   int R = 0;
-  at = before = true;
+  sure = false;
   for (int r = 1; r < kRMin - 1 + kRec; ++r) {
     cd jr = mkcd(0, 0), kr = jr;
+    double sj = 0, sk = 0, ramax = 0;
     auto summand = [&](int m, int n, double dm, double dn) {
       const double dx = urx - (dm * us1x + dn * us2x), dy = ury - (dm * us1y + dn * us2y);
-      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
+      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab), ej = er * ra;
       if constexpr (REAL) {
-        jr.x += er * ra;
+        jr.x += ej;
         kr.x += er;
       } else {
         const cd f = ph1[m + PSS_JKRINGMAX] * ph2[n + PSS_JKRINGMAX];
         jr = jr + mkcd(er * f.x * ra, er * f.y * ra);
         kr = kr + mkcd(er * f.x, er * f.y);
+        sj += ej;
+        sk += er;
       }
+      if (r == 1) ramax = fmax(ramax, ra);
     };
     const double dr = (double)r;
     double d = -dr;
@@ -105,36 +125,50 @@ __device__ __forceinline__ int scan_rings(double urx, double ury, double us1x, d
       summand(i, -r, d, -dr);
       summand(i, r, d, dr);
     }
-    if (r >= 2) { jfar = jfar + jr; kfar = kfar + kr; }
-    if (r >= kRMin - 1) rec(r - (kRMin - 1), jfar, kfar);
+    if constexpr (REAL) { sj = jr.x; sk = kr.x; }
+    lipk += kFar * sk;
+    if (r == 1) {
+      lipj += 4 * de * ramax < 1 ? kNear * slope_of(ramax) * sj : 1e300;  // no bound beside an image
+    } else {
+      jfar = jfar + jr;
+      kfar = kfar + kr;
+      farj += sj;
+      fark += sk;
+      lipj += slope * sj;
+    }
+    if (r == kRMin - 1) rec(0, jfar, kfar, farj, fark);
+    if (r >= kRMin) rec(r - (kRMin - 1), jfar, kfar, sj, sk);
     if (R) return R;  // one ring past R has been recorded
     jsum = jsum + jr;
     ksum = ksum + kr;
     if (r >= kRMin) {
       const double aj = cabsd(jsum), ak = cabsd(ksum), rj = cabsd(jr), rk = cabsd(kr);
-      const bool stop = fmax(cabsd(jr / jsum), cabsd(kr / ksum)) < kConv;
-      const bool cj = clear_of(rj, aj, kMargin, kCurve, stop), ck = clear_of(rk, ak, kMargin, kCurve, stop);
-      if (stop) {
+      const double ej = slope * de * sj, ek = kFar * de * sk, dj = de * lipj, dk = de * lipk;
+      constexpr double up = kConv * (1 + kTol), dn = kConv * (1 - kTol);
+      if (!(rj - ej > up * (aj + dj) || rk - ek > up * (ak + dk))) {
         R = r;
-        at = cj && ck;
-      } else {
-        before = cj || ck;
+        sure = rj + ej < dn * (aj - dj) && rk + ek < dn * (ak - dk);
       }
     }
   }
-  return 0;  // not below the threshold by the last recorded ring, or R + 1 not recorded
+  return 0;  // passed over to the last recorded ring, or R + 1 not recorded
 }
 
-// Whether a sum may vanish near v: v is no larger than its distance from one of the corner values.
-__device__ __forceinline__ bool near_zero(cd v, const cd *corner) {
-  bool z = false;
-  const double a = v.x * v.x + v.y * v.y;
+// Bounds on the modulus over a sub-cell's convex hull of four corner values.
+__device__ __forceinline__ double hull_max(const cd (&v)[4]) {
+  double m = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const double dx = v.x - corner[k].x, dy = v.y - corner[k].y;
-    z = z || a <= dx * dx + dy * dy;
-  }
-  return z;
+  for (int k = 0; k < 4; ++k) m = fmax(m, v[k].x * v[k].x + v[k].y * v[k].y);
+  return sqrt(m);
+}
+__device__ __forceinline__ double hull_min(const cd (&v)[4]) {  // along the mean's direction
+  const double mx = (v[0].x + v[1].x) + (v[2].x + v[3].x), my = (v[0].y + v[1].y) + (v[2].y + v[3].y);
+  const double m2 = mx * mx + my * my;
+  if (!(m2 > 0)) return 0.0;
+  double m = 1e300;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) m = fmin(m, v[k].x * mx + v[k].y * my);
+  return m * rsqrt(m2);
 }
 
 // One CTA of 64 threads per panel (x) and phasing (y): node (i, j) = (tid / 8, tid % 8).
@@ -143,8 +177,10 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
                                                     double us2y) {
   __shared__ cd ph1[1][kPhase], ph2[1][kPhase];
   __shared__ double etab[256];
-  __shared__ cd rj[kRec][64], rk[kRec][64], corner[2][4];
+  __shared__ cd rj[kRec][64], rk[kRec][64];
+  __shared__ float sj[kRec][64], sk[kRec][64];  // sums without phases
   __shared__ int lo, hi;
+  __shared__ unsigned bound[kBounds];  // positive floats, which order as their bits do
   const int p = blockIdx.y, panel = blockIdx.x, tid = threadIdx.x;
   PsiGroup one{};
   one.n = 1;
@@ -152,27 +188,46 @@ __global__ void __launch_bounds__(64) k_jktab_nodes(TabDev T, PsiGroup pg, doubl
   one.psi2[0] = pg.psi2[p];
   fill_phases<1>(one, 1, ph1, ph2, etab);
   if (tid == 0) { lo = 1000; hi = 0; }
-  for (int r = 0; r < kRec; ++r) rj[r][tid] = rk[r][tid] = mkcd(0, 0);
+  if (tid < kBounds) bound[tid] = 0;
+  for (int r = 0; r < kRec; ++r) {
+    rj[r][tid] = rk[r][tid] = mkcd(0, 0);
+    sj[r][tid] = sk[r][tid] = 0.f;
+  }
   __syncthreads();
   const int i = tid >> 3, j = tid & 7, ia = panel % T.na, ib = panel / T.na;
   const double a = T.a0 + (ia + 0.5 * (1.0 + c_node[i])) / T.ra, b = T.b0 + (ib + 0.5 * (1.0 + c_node[j])) / T.rb;
-  bool at, before;
-  cd js, ks;
-  const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0],
-                                 etab, at, before, js, ks, [&](int r, cd jf, cd kf) { rj[r][tid] = jf; rk[r][tid] = kf; });
-  if (tid == 0 || tid == 7 || tid == 56 || tid == 63) {
-    corner[0][(tid & 1) + (tid >> 5) * 2] = js;
-    corner[1][(tid & 1) + (tid >> 5) * 2] = ks;
-  }
-  // the stopping rings that points near this node may have
-  if (R) atomicMin(&lo, R > kRMin && !before ? R - 1 : R);
-  atomicMax(&hi, R == 0 ? 1000 : !at ? R + 1 : R);
-  __syncthreads();
-  if (near_zero(js, corner[0]) || near_zero(ks, corner[1])) atomicMax(&hi, 1000);
+  bool sure;
+  const int R = scan_rings<REAL>(a * us1x + b * us2x, a * us1y + b * us2y, us1x, us1y, us2x, us2y, ph1[0], ph2[0], etab,
+                                 kNodeGap * 0.5 * (T.wa + T.wb), T.q, sure, [&](int r, cd jf, cd kf, double vj, double vk) {
+                                   rj[r][tid] = jf;
+                                   rk[r][tid] = kf;
+                                   sj[r][tid] = __double2float_ru(vj);
+                                   sk[r][tid] = __double2float_ru(vk);
+                                 });
+  if (R) atomicMin(&lo, R);
+  atomicMax(&hi, sure ? R : 1000);
   __syncthreads();
   const bool direct = lo == 1000;
   if (tid == 0) T.flag[p][panel] = direct ? 2 : hi == lo ? 0 : 1;
   const int r0 = direct ? 1 : lo - (kRMin - 1);
+  {
+    float far_j = 0, far_k = 0;
+    for (int r = 0; r <= r0 + 1; ++r) {
+      far_j = __fadd_ru(far_j, sj[r][tid]);
+      far_k = __fadd_ru(far_k, sk[r][tid]);
+    }
+    const float cj = __double2float_ru(curve_of(T.q));
+    const float v[kBounds] = {__fmul_ru(cj, sj[r0][tid]),     __fadd_ru(sj[r0][tid], sk[r0][tid]),
+                              __fmul_ru(cj, sj[r0 + 1][tid]), __fadd_ru(sj[r0 + 1][tid], sk[r0 + 1][tid]),
+                              __fmul_ru(cj, far_j),           __fadd_ru(far_j, far_k)};
+#pragma unroll
+    for (int k = 0; k < kBounds; ++k) {
+      const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(v[k]));
+      if ((tid & 31) == 0) atomicMax(&bound[k], m);
+    }
+    __syncthreads();
+    if (tid < kBounds) T.bound[p][panel * kBounds + tid] = __uint_as_float(bound[tid]);
+  }
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const cd J = rj[r0 + s][tid], K = rk[r0 + s][tid];
@@ -212,22 +267,23 @@ __device__ __forceinline__ void basis8(double t, double s, double *out) {
   }
 }
 
-// Sub-cell maps of the panels that need one: the stopping ring at the 33 x 33 corners, from the
-// nearest images and the panel's own interpolants of the far sums (through R0 and R0 + 1) and of
-// ring R0: about 400 operations per corner, where summing the rings anew would take 5000.
-constexpr int kC = kSub + 1, kCorners = kC * kC;
+// Sub-cell maps of the panels that need one: the sums and their rings R0 and R0 + 1 at the 33 x 33
+// corners, from the nearest images and the panel's own interpolants of the far sums (through R0
+// and R0 + 1) and of ring R0: about 400 operations per corner, where summing the rings anew would
+// take 5000.  Strips of kStrip sub-cell rows, so that three CTAs fit an SM.
+constexpr int kC = kSub + 1, kStrip = 11, kCorners = (kStrip + 1) * kC;
 template <bool REAL>
-__global__ void __launch_bounds__(256) k_jktab_map(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
+__global__ void __launch_bounds__(256, 2) k_jktab_map(TabDev T, PsiGroup pg, double us1x, double us1y, double us2x,
                                                    double us2y) {
   constexpr int W = REAL ? 6 : 12;  // reals per node: far R0 (J, K), far R0 + 1, ring R0
   __shared__ double etab[256];
   __shared__ cd fnear[9];
   __shared__ double lag[kC][kND];
   __shared__ double node[64][W];
-  __shared__ unsigned char cls[kCorners];
   extern __shared__ __align__(16) unsigned char map_smem[];
-  cd *cj = (cd *)map_smem, *ck = cj + kCorners;
-  double *half = (double *)(ck + kCorners);  // [corner i][node j][W]
+  cd *cs = (cd *)map_smem;  // [J, K through R0; ring R0; ring R0 + 1][corner]
+  float *cn = (float *)(cs + 6 * kCorners);  // [J, K][corner]: second-derivative bound of the near terms
+  double *half = (double *)(cn + 2 * kCorners);  // [corner i][node j][W]
   const int p = blockIdx.y, panel = blockIdx.x, tid = threadIdx.x;
   if (T.flag[p][panel] != 1) return;
   etab[tid] = exp2((double)tid / 256.0);
@@ -252,59 +308,88 @@ __global__ void __launch_bounds__(256) k_jktab_map(TabDev T, PsiGroup pg, double
     for (int k = 0; k < kND; ++k) s = fma(lag[i][k], node[k * 8 + j][w], s);
     half[e] = s;
   }
-  __syncthreads();
   const int ia = panel % T.na, ib = panel / T.na;
-  for (int e = tid; e < kCorners; e += 256) {
-    const int i = e / kC, j = e % kC;
-    double v[12];
+  const double wa = T.wa / kSub, wb = T.wb / kSub, diag = wa + wb, q8 = (wa * wa + wb * wb) / 8;
+  const float *bnd = T.bound[p] + panel * kBounds;
+  const double fj = kFar * q8 * bnd[0], fk = kFar * q8 * bnd[1], gj = kFar * q8 * bnd[2], gk = kFar * q8 * bnd[3];
+  const double sj = kFar * q8 * bnd[4], sk = kFar * q8 * bnd[5];
+  for (int i0 = 0; i0 < kSub; i0 += kStrip) {
+    const int rows = min(kStrip, kSub - i0);
+    __syncthreads();  // half written, the previous strip read
+    for (int e = tid; e < (rows + 1) * kC; e += 256) {
+      const int i = i0 + e / kC, j = e % kC;
+      double v[12];
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      double s = 0;
+      for (int w = 0; w < W; ++w) {
+        double s = 0;
 #pragma unroll
-      for (int k = 0; k < kND; ++k) s = fma(lag[j][k], half[(i * kND + k) * W + w], s);
-      v[w] = s;
+        for (int k = 0; k < kND; ++k) s = fma(lag[j][k], half[(i * kND + k) * W + w], s);
+        v[w] = s;
+      }
+      const double a = T.a0 + (ia + (double)i / kSub) / T.ra, b = T.b0 + (ib + (double)j / kSub) / T.rb;
+      const double ux = a * us1x + b * us2x, uy = a * us1y + b * us2y;
+      const double arg = sqrt(ux * ux + uy * uy), rterm = exp_neg(arg, etab);
+      cd js = mkcd(arg <= 1e-5 ? (-arg / 6 + 0.5) * arg - 1 : (rterm - 1) / arg, 0.0), ks = mkcd(rterm, 0.0);
+      // the (0, 0) term's kink at the origin: beside it, the Lipschitz constants' equivalent
+      const bool off = arg > 2 * diag;
+      double nj = off ? 1.0 / 3 + 0.5 / (arg - diag) : 0.5 * diag / q8, nk = off ? 1.0 + 1.0 / (arg - diag) : diag / q8;
+      double s1 = 0, s0 = 0, ramax = 0;  // of e^-d / d, of e^-d, the nearest image's 1/d
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        if (q == 4) continue;
+        const double m = q / 3 - 1, n = q % 3 - 1;
+        const double dx = ux - (m * us1x + n * us2x), dy = uy - (m * us1y + n * us2y);
+        const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
+        const cd f = fnear[q];
+        js = js + mkcd(er * f.x * ra, er * f.y * ra);
+        ks = ks + mkcd(er * f.x, er * f.y);
+        s1 = fma(er, ra, s1);
+        s0 += er;
+        ramax = fmax(ramax, ra);
+      }
+      nj += 4 * diag * ramax < 1 ? kNear * curve_of(ramax) * s1 : 1e300;  // beside an image: unknown
+      nk += 4 * diag * ramax < 1 ? kNear * (s0 + s1) : 1e300;
+      auto val = [&](int k) { return REAL ? mkcd(v[k], 0.0) : mkcd(v[2 * k], v[2 * k + 1]); };  // (slot, J / K)
+      cs[e] = js + val(0);
+      cs[kCorners + e] = ks + val(1);
+      cs[2 * kCorners + e] = val(4);
+      cs[3 * kCorners + e] = val(5);
+      cs[4 * kCorners + e] = val(2) - val(0);
+      cs[5 * kCorners + e] = val(3) - val(1);
+      cn[e] = __double2float_ru(nj);
+      cn[kCorners + e] = __double2float_ru(nk);
     }
-    const double a = T.a0 + (ia + (double)i / kSub) / T.ra, b = T.b0 + (ib + (double)j / kSub) / T.rb;
-    const double ux = a * us1x + b * us2x, uy = a * us1y + b * us2y;
-    const double arg = sqrt(ux * ux + uy * uy), rterm = exp_neg(arg, etab);
-    cd js = mkcd(arg <= 1e-5 ? (-arg / 6 + 0.5) * arg - 1 : (rterm - 1) / arg, 0.0), ks = mkcd(rterm, 0.0);
+    __syncthreads();
+    for (int e = tid; e < rows * kSub; e += 256) {
+      const int e0 = e / kSub * kC + e % kSub;
+      const int c[4] = {e0, e0 + 1, e0 + kC, e0 + kC + 1};
+      cd v[6][4];
+      float nj = 0, nk = 0;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      if (q == 4) continue;
-      const double m = q / 3 - 1, n = q % 3 - 1;
-      const double dx = ux - (m * us1x + n * us2x), dy = uy - (m * us1y + n * us2y);
-      const double d2 = dx * dx + dy * dy, ra = rsqrt(d2), er = exp_neg(d2 * ra, etab);
-      const cd f = fnear[q];
-      js = js + mkcd(er * f.x * ra, er * f.y * ra);
-      ks = ks + mkcd(er * f.x, er * f.y);
-    }
-    auto val = [&](int k) { return REAL ? mkcd(v[k], 0.0) : mkcd(v[2 * k], v[2 * k + 1]); };  // (slot, J / K)
-    const cd j0 = js + val(0), k0 = ks + val(1), j1 = js + val(2), k1 = ks + val(3);
-    const double a0 = cabsd(j0), b0 = cabsd(k0), r0 = cabsd(val(4)), s0 = cabsd(val(5));
-    int c = 2;
-    if (clear_of(r0, a0, kSubMargin, kSubCurve, true) && clear_of(s0, b0, kSubMargin, kSubCurve, true)) {
-      c = 0;
-    } else if (clear_of(r0, a0, kSubMargin, kSubCurve, false) || clear_of(s0, b0, kSubMargin, kSubCurve, false)) {
-      const double r1 = cabsd(val(2) - val(0)), s1 = cabsd(val(3) - val(1));
-      if (clear_of(r1, cabsd(j1), kSubMargin, kSubCurve, true) && clear_of(s1, cabsd(k1), kSubMargin, kSubCurve, true)) c = 1;
-    }
-    cls[e] = (unsigned char)c;
-    cj[e] = c == 0 ? j0 : j1;
-    ck[e] = c == 0 ? k0 : k1;
-  }
-  __syncthreads();
-  for (int e = tid; e < kSub * kSub; e += 256) {
-    const int e0 = e / kSub * kC + e % kSub;
-    const int c[4] = {e0, e0 + 1, e0 + kC, e0 + kC + 1};
-    int v = cls[c[0]];
-    const cd j4[4] = {cj[c[0]], cj[c[1]], cj[c[2]], cj[c[3]]}, k4[4] = {ck[c[0]], ck[c[1]], ck[c[2]], ck[c[3]]};
+      for (int q = 0; q < 4; ++q) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (cls[c[q]] != v || near_zero(j4[q], j4) || near_zero(k4[q], k4)) v = 2;
-    T.map[p][(size_t)panel * kSub * kSub + e] = (unsigned char)v;
+        for (int k = 0; k < 6; ++k) v[k][q] = cs[k * kCorners + c[q]];
+        nj = fmaxf(nj, cn[c[q]]);
+        nk = fmaxf(nk, cn[kCorners + c[q]]);
+      }
+      constexpr double up = kConv * (1 + kTol), dn = kConv * (1 - kTol);
+      const double ej = fma(q8, (double)nj, sj), ek = fma(q8, (double)nk, sk);  // of the whole sums
+      int state = 2;
+      if (hull_max(v[2]) + fj < dn * (hull_min(v[0]) - ej) && hull_max(v[3]) + fk < dn * (hull_min(v[1]) - ek)) {
+        state = 0;
+      } else if (hull_min(v[2]) - fj > up * (hull_max(v[0]) + ej) || hull_min(v[3]) - fk > up * (hull_max(v[1]) + ek)) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // through ring R0 + 1
+          v[0][q] = v[0][q] + v[4][q];
+          v[1][q] = v[1][q] + v[5][q];
+        }
+        if (hull_max(v[4]) + gj < dn * (hull_min(v[0]) - ej) && hull_max(v[5]) + gk < dn * (hull_min(v[1]) - ek)) state = 1;
+      }
+      T.map[p][(size_t)panel * kSub * kSub + i0 * kSub + e] = (unsigned char)state;
+    }
   }
 }
-constexpr int kMapSmem = 2 * kCorners * (int)sizeof(cd) + kC * kND * 12 * (int)sizeof(double);
+constexpr int kMapSmem = kCorners * (6 * (int)sizeof(cd) + 2 * (int)sizeof(float)) + kC * kND * 12 * (int)sizeof(double);
 
 constexpr int kTabThreads = 128;
 // The seven points in a walk around the triangle (vertex, midpoint, ..., centroid): neighbours
@@ -597,11 +682,13 @@ bool pss_jktab_plan(const SheetDev &G, double ulocal, const double s1[2], const 
   P.nb = std::max(1, (int)cb);
   const size_t panels = (size_t)P.na * P.nb;
   if ((size_t)G.nufp < 55 * panels) return false;
+  P.dmin = dmin;
   P.a0 = -W1;
   P.b0 = -W2;
   P.ra = P.na / (2 * W1);
   P.rb = P.nb / (2 * W2);
-  const size_t per = align256(panels * 3 * 64 * 4 * sizeof(double)) + align256(panels) + align256(panels * kSub * kSub);
+  const size_t per = align256(panels * 3 * 64 * 4 * sizeof(double)) + align256(panels * kBounds * sizeof(float)) +
+                     align256(panels) + align256(panels * kSub * kSub);
   P.bytes = (size_t)np * (per + (size_t)G.nufp * sizeof(int)) + 512;
   return true;
 }
@@ -620,11 +707,15 @@ int pss_jktab_launch(const SheetDev &G, double ulocal, const PsiGroup &pg, const
   TabDev T{};
   T.iv[0] = d / det; T.iv[1] = -c / det; T.iv[2] = -b / det; T.iv[3] = a / det;
   T.a0 = P.a0; T.b0 = P.b0; T.ra = P.ra; T.rb = P.rb; T.na = P.na; T.nb = P.nb;
+  T.wa = std::hypot(a, b) / P.ra;
+  T.wb = std::hypot(c, d) / P.rb;
+  T.q = 1 / P.dmin;
   char *w = (char *)(((uintptr_t)ws + 255) & ~(uintptr_t)255);
   for (int p = 0; p < np; ++p) {
     T.val[p] = (double *)w;
     T.ring[p] = T.val[p] + panels * 2 * 64 * 4;
     w += align256(panels * 3 * 64 * 4 * sizeof(double));
+    T.bound[p] = (float *)w; w += align256(panels * kBounds * sizeof(float));
     T.flag[p] = (unsigned char *)w; w += align256(panels);
     T.map[p] = (unsigned char *)w; w += align256(panels * kSub * kSub);
   }
