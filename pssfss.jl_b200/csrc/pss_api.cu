@@ -292,11 +292,23 @@ int set_device(pss_ctx *c) {
   return 0;
 }
 
-template <class T>
-int upload(DevBuf &b, const T *h, size_t n) {
-  if (b.ensure(std::max<size_t>(n, 1) * sizeof(T))) return -3;
-  if (n) PSS_CUDA_TRY(cudaMemcpy(b.p, h, n * sizeof(T), cudaMemcpyHostToDevice));
+// Waits for copies and memsets issued on the legacy stream.  cudaMemcpy from pageable memory returns
+// once the data are staged, possibly before they have reached the device, and the workers' streams
+// do not wait for the legacy stream: what they read goes through here first (a factorisation
+// that began before the end of its matrix had arrived gave wrong factors in one call of 24 at
+// order 736).
+int settle() {
+  PSS_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
   return 0;
+}
+
+// wait = false: the caller settles after the last of several.
+template <class T>
+int upload(DevBuf &b, const T *h, size_t n, bool wait = true) {
+  if (b.ensure(std::max<size_t>(n, 1) * sizeof(T))) return -3;
+  if (n == 0) return 0;
+  PSS_CUDA_TRY(cudaMemcpy(b.p, h, n * sizeof(T), cudaMemcpyHostToDevice));
+  return wait ? settle() : 0;
 }
 
 int make_stack(int nl, const double *eps, const double *mu, const double *width, int s, StackParams &S) {
@@ -626,7 +638,7 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     const size_t np2 = (size_t)nface * nface;
     LocalBuf raw, bad;
     int hbad[2] = {0, 0};
-    if (raw.ensure(std::max(np2, (size_t)nufp) * sizeof(int64_t)) || upload(bad, hbad, 2) ||
+    if (raw.ensure(std::max(np2, (size_t)nufp) * sizeof(int64_t)) || upload(bad, hbad, 2, false) ||
         sh->ufpm.ensure(np2 * sizeof(int)) || sh->rep.ensure(nufp * sizeof(int)) ||
         sh->pfaces.ensure(nufp * sizeof(int2)))
       return refuse(-3);
@@ -706,19 +718,19 @@ int pss_sheet_create(pss_ctx *ctx, char cls, double units_per_meter, const doubl
     }
   std::vector<double> hfr(fr, fr + nface);
   int rc = 0;
-  rc |= upload(sh->rho, rho, 2 * (size_t)nnode);
-  rc |= upload(sh->fv, hfv.data(), hfv.size());
-  rc |= upload(sh->fr, hfr.data(), hfr.size());
-  rc |= upload(sh->ls, hls.data(), hls.size());
-  rc |= upload(sh->a48, ha48.data(), ha48.size());
-  rc |= upload(sh->inc_cnt, icnt.data(), icnt.size());
-  rc |= upload(sh->inc_face, iface.data(), iface.size());
-  rc |= upload(sh->inc_loc, iloc.data(), iloc.size());
-  rc |= upload(sh->inc_sgn, isgn.data(), isgn.size());
-  rc |= upload(sh->inc_eci, ieci.data(), ieci.size());
-  rc |= upload(sh->face_m, hfm.data(), hfm.size());
-  rc |= upload(sh->inc, hinc.data(), hinc.size());
-  if (rc) return refuse(-3);
+  rc |= upload(sh->rho, rho, 2 * (size_t)nnode, false);
+  rc |= upload(sh->fv, hfv.data(), hfv.size(), false);
+  rc |= upload(sh->fr, hfr.data(), hfr.size(), false);
+  rc |= upload(sh->ls, hls.data(), hls.size(), false);
+  rc |= upload(sh->a48, ha48.data(), ha48.size(), false);
+  rc |= upload(sh->inc_cnt, icnt.data(), icnt.size(), false);
+  rc |= upload(sh->inc_face, iface.data(), iface.size(), false);
+  rc |= upload(sh->inc_loc, iloc.data(), iloc.size(), false);
+  rc |= upload(sh->inc_sgn, isgn.data(), isgn.size(), false);
+  rc |= upload(sh->inc_eci, ieci.data(), ieci.size(), false);
+  rc |= upload(sh->face_m, hfm.data(), hfm.size(), false);
+  rc |= upload(sh->inc, hinc.data(), hinc.size(), false);
+  if (rc || settle()) return refuse(-3);
   SheetDev &G = sh->G;
   G.nface = sh->nface; G.nbf = sh->nbf; G.nufp = sh->nufp; G.nnode = sh->nnode; G.upm = units_per_meter;
   G.rho = sh->rho.as<double>(); G.fv = sh->fv.as<int>(); G.ufpm = sh->ufpm.as<int>(); G.ufp_rep = sh->rep.as<int>();
@@ -884,6 +896,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
   }
   if (c->dS.ensure(std::max<size_t>(nd, 1) * sizeof(cd)) || c->status.ensure((size_t)total * sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemset(c->status.p, 0, (size_t)total * sizeof(int)));
+  if (settle()) return -3;  // the workers' streams read these
   int *dstatus = c->status.as<int>();
 
   // Face-pair integrals: a problem whose points share (ψ1, ψ2) uses its sheet's cache,
@@ -1180,6 +1193,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
       std::vector<int> cleared(total);
       for (int g = 0; g < total; ++g) cleared[g] = hst[g] & ~(PSS_ST_REFINE_NOCONV | PSS_ST_NONFINITE);
       PSS_CUDA_TRY(cudaMemcpy(c->status.p, cleared.data(), (size_t)total * sizeof(int), cudaMemcpyHostToDevice));
+      if (settle()) return -3;
       size_t k = 0;
       for (size_t p = 0; p < PR.size(); ++p) {
         Item it{};
@@ -1457,8 +1471,8 @@ int pss_lu32_factor(pss_ctx *c, int n, const double *Z, float *LU, int *ipiv, in
       hr[m * ldf + q] = (float)Z[2 * (m + q * n)];
       hi[m * ldf + q] = (float)Z[2 * (m + q * n) + 1];
     }
-  PSS_CUDA_TRY(cudaMemcpy(w.zr.p, hr.data(), nf * sizeof(float), cudaMemcpyHostToDevice));
-  PSS_CUDA_TRY(cudaMemcpy(w.zi.p, hi.data(), nf * sizeof(float), cudaMemcpyHostToDevice));
+  PSS_CUDA_TRY(cudaMemcpyAsync(w.zr.p, hr.data(), nf * sizeof(float), cudaMemcpyHostToDevice, st));
+  PSS_CUDA_TRY(cudaMemcpyAsync(w.zi.p, hi.data(), nf * sizeof(float), cudaMemcpyHostToDevice, st));
   PSS_CUDA_TRY(cudaMemsetAsync(w.info.p, 0, sizeof(int), st));
   if (int rc = pss_lu32_batched(n, 1, w.zr.as<float>(), w.zi.as<float>(), (long long)ldf, (long long)nf,
                                 w.ipiv.as<int>(), w.info.as<int>(), w.luws.p, w.luws.n, st))
@@ -1470,7 +1484,7 @@ int pss_lu32_factor(pss_ctx *c, int n, const double *Z, float *LU, int *ipiv, in
   std::vector<int> hp(n);
   PSS_CUDA_TRY(cudaMemcpy(hp.data(), w.ipiv.p, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost));
   PSS_CUDA_TRY(cudaMemcpy(info, w.info.p, sizeof(int), cudaMemcpyDeviceToHost));
-  PSS_CUDA_TRY(cudaMemset(w.info.p, 0, sizeof(int)));
+  PSS_CUDA_TRY(cudaMemsetAsync(w.info.p, 0, sizeof(int), st));
   for (size_t m = 0; m < (size_t)n; ++m)
     for (size_t q = 0; q < (size_t)n; ++q) {
       LU[2 * (m + q * n)] = hr[m * ldf + q];
@@ -1667,7 +1681,7 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
       const double *pp = ppsi + 2 * ((size_t)k * npts + i);
       make_params(magnetic, Sk[k], b1m, b2m, pu[k], k0[i], pp[0], pp[1], hP[1 + k]);
     }
-    PSS_CUDA_TRY(cudaMemcpy(pbuf.p, hP.data(), hP.size() * sizeof(PointParams), cudaMemcpyHostToDevice));
+    PSS_CUDA_TRY(cudaMemcpyAsync(pbuf.p, hP.data(), hP.size() * sizeof(PointParams), cudaMemcpyHostToDevice, st));
     const PointParams *dP = pbuf.as<PointParams>();
     for (int q = 0; q <= K; ++q) {
       const size_t off = q == 0 ? (size_t)i * nm : ((size_t)(q - 1) * npts + i) * nm;
@@ -1675,10 +1689,10 @@ extern "C" int pss_partial_gsms_lin(pss_sheet *sh, int nl, const double *eps, co
       const double *sv = q == 0 ? src : psrc;
       const double *tv = q == 0 ? tobs : ptobs;
       const double *wv = q == 0 ? wobs : pwobs;
-      PSS_CUDA_TRY(cudaMemcpy(kv_of(q), kv + 2 * off, nm * 2 * sizeof(double), cudaMemcpyHostToDevice));
-      PSS_CUDA_TRY(cudaMemcpy(src_of(q), sv + 4 * off, nm * 2 * sizeof(cd), cudaMemcpyHostToDevice));
-      PSS_CUDA_TRY(cudaMemcpy(tob_of(q), tv + 2 * off, nm * 2 * sizeof(double), cudaMemcpyHostToDevice));
-      PSS_CUDA_TRY(cudaMemcpy(wob_of(q), wv + 2 * off, nm * sizeof(cd), cudaMemcpyHostToDevice));
+      PSS_CUDA_TRY(cudaMemcpyAsync(kv_of(q), kv + 2 * off, nm * 2 * sizeof(double), cudaMemcpyHostToDevice, st));
+      PSS_CUDA_TRY(cudaMemcpyAsync(src_of(q), sv + 4 * off, nm * 2 * sizeof(cd), cudaMemcpyHostToDevice, st));
+      PSS_CUDA_TRY(cudaMemcpyAsync(tob_of(q), tv + 2 * off, nm * 2 * sizeof(double), cudaMemcpyHostToDevice, st));
+      PSS_CUDA_TRY(cudaMemcpyAsync(wob_of(q), wv + 2 * off, nm * sizeof(cd), cudaMemcpyHostToDevice, st));
     }
     // tables and face-pair integrals of every set
     TableDev t0;
