@@ -393,28 +393,30 @@ __global__ void __launch_bounds__(256) k_rowsolve(Mat<F32> M0, long long ms, int
     }
     __syncthreads();
     {
+      // an entry's products are summed apart and subtracted from it once
       const int c = tid / T::LANES, p = tid % T::LANES;
-      E x[T::NI];
+      E x[T::NI], a[T::NI];
 #pragma unroll
       for (int i = 0; i < T::NI; ++i) {
         const int r = p + T::LANES * i;
         x[i] = r < nc ? X[(b0 + r) * T::COLS + c] : E{0, 0};
+        a[i] = E{0, 0};
       }
 #pragma unroll
       for (int j = 0; j < T::S - 1; ++j) {
-        E xj;
-        xj.x = __shfl_sync(0xffffffffu, x[j / T::LANES].x, j % T::LANES, T::LANES);
-        xj.y = __shfl_sync(0xffffffffu, x[j / T::LANES].y, j % T::LANES, T::LANES);
+        E xj = csubE(x[j / T::LANES], a[j / T::LANES]);
+        xj.x = __shfl_sync(0xffffffffu, xj.x, j % T::LANES, T::LANES);
+        xj.y = __shfl_sync(0xffffffffu, xj.y, j % T::LANES, T::LANES);
 #pragma unroll
         for (int i = j / T::LANES; i < T::NI; ++i) {
           const int r = p + T::LANES * i;
-          if (r > j && r < nc) x[i] = cmsub(x[i], L[r * T::LP + j], xj);
+          if (r > j && r < nc) a[i] = cmac_nested(a[i], L[r * T::LP + j], xj);
         }
       }
 #pragma unroll
       for (int i = 0; i < T::NI; ++i) {
         const int r = p + T::LANES * i;
-        if (r < nc) X[(b0 + r) * T::COLS + c] = x[i];
+        if (r < nc) X[(b0 + r) * T::COLS + c] = csubE(x[i], a[i]);
       }
     }
     if (b0 + T::S >= jb) break;
@@ -437,7 +439,7 @@ __global__ void __launch_bounds__(256) k_rowsolve(Mat<F32> M0, long long ms, int
         if (i >= ni) break;
         const E l = L[min(T::S + ty + 16 * i, T::S + rem - 1) * T::LP + k];
 #pragma unroll
-        for (int q = 0; q < T::CQ; ++q) acc[i][q] = cmac(acc[i][q], l, xv[q]);
+        for (int q = 0; q < T::CQ; ++q) acc[i][q] = cmac_nested(acc[i][q], l, xv[q]);
       }
     }
 #pragma unroll

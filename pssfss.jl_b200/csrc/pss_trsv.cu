@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
   C *Ds = (C *)smraw;
   C *part = Ds + BS * P::LD;  // TRANS: [warp][64][NJ]
   __shared__ C y[BS][NJ];
+  __shared__ C ya[BS][NJ];  // products of all tiles but the predecessor's
   __shared__ C xs[BS][NJ];
   __shared__ C xw[P::T / 32][P::RW][NJ];
   __shared__ int s_b;
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
     if (r < nr && j < nj)
       v = LOWER ? B[(size_t)j * n + (TRANS ? r0 + r : perm[r0 + r])] : ldcg(&X[(size_t)j * n + r0 + r]);
     y[r][j] = S::from(v);
+    ya[r][j] = czero<C>();
   }
   // tiles in the order their blocks finish; the last one, the predecessor's, apart
   const int nt = LOWER ? b : nblk - 1 - b;
@@ -333,10 +335,10 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
           const C q = part[w * BS * NJ + tid];
           v = C{v.x + q.x, v.y + q.y};
         }
-        y[tid / NJ][tid % NJ] = y[tid / NJ][tid % NJ] - v;
+        ya[tid / NJ][tid % NJ] = v;
       }
     } else {
-      __syncthreads();  // y staged
+      __syncthreads();  // ya cleared
 #pragma unroll
       for (int rr = 0; rr < P::RW; ++rr)
 #pragma unroll
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
             acc[rr][j].x += __shfl_xor_sync(0xffffffff, acc[rr][j].x, o);
             acc[rr][j].y += __shfl_xor_sync(0xffffffff, acc[rr][j].y, o);
           }
-          if (lane == 0) y[warp * P::RW + rr][j] = y[warp * P::RW + rr][j] - acc[rr][j];
+          if (lane == 0) ya[warp * P::RW + rr][j] = acc[rr][j];
         }
     }
   }
@@ -381,7 +383,10 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
       }
     if (pq == 0)
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) y[pi][j] = y[pi][j] - s[j];
+      for (int j = 0; j < NJ; ++j) {  // all products first, then one rounding at y's size
+        const C q = ya[pi][j];
+        y[pi][j] = y[pi][j] - C{q.x + s[j].x, q.y + s[j].y};
+      }
   }
   __syncthreads();
   // X[rows] = Dinv_b * y: one entry per T / 256 lanes
@@ -411,9 +416,13 @@ __global__ void __launch_bounds__(TrsvT<F32>::T, F32 ? 2 : 1)
 // warps takes 16 rows, each warp 2 of them; the columns go in chunks whose X block (M x 4096 / M
 // entries) is staged in shared memory and reused by the rows of every warp, so the matrix rows
 // are the only HBM stream (streaming loads).  The column loop has no early exit (the ragged last
-// chunk is predicated), so the loads of several steps are in flight per lane; rows past n are
-// clamped to row n-1 for their loads and dropped at the end.
-constexpr int kResRows = 2;
+// chunk is predicated); rows past n are clamped to row n-1 for their loads and dropped at the end.
+// A lane takes kResG columns at a time and sums their products on their own before it adds them to
+// the running sum: 5 operations a component for two products and one rounding at the running
+// sum's size, where adding each takes 6 and two, and nested multiply-adds take 4 and four.  The
+// residual's own rounding is what limits a refined solution: order 1501, error against 64 bits
+// 4.0e-16 with nested multiply-adds.  593 us for 12 matrices of N = 3976 (nested 594, each 770).
+constexpr int kResRows = 2, kResG = 2;
 constexpr int kResSmem = 4096 * (int)sizeof(cd);  // 64 KB
 __device__ __forceinline__ cd ldcs(const cd *p) {
   const double2 v = __ldcs(reinterpret_cast<const double2 *>(p));
@@ -454,21 +463,31 @@ __global__ void __launch_bounds__(256, M == 4 ? 3 : 2) k_resid(int n, const cd *
     }
     __syncthreads();
     const int qn = (len + 31) >> 5;
-#pragma unroll 4
-    for (int q = 0; q < qn; ++q) {
-      const int t = q * 32 + lane;
-      const bool ok = t < len;
-      cd av[kResRows];
+#pragma unroll 2
+    for (int q0 = 0; q0 < qn; q0 += kResG) {  // the staged block's rows past len are zero
+      cd av[kResG][kResRows];
 #pragma unroll
-      for (int i = 0; i < kResRows; ++i) {
-        av[i] = ok ? ldcs(arow[i] + t0 + t) : mkcd(0, 0);
-        rs[i] += cabs1(av[i]);
+      for (int g = 0; g < kResG; ++g) {
+        const int t = (q0 + g) * 32 + lane;
+        const bool ok = t < len;
+#pragma unroll
+        for (int i = 0; i < kResRows; ++i) {
+          av[g][i] = ok ? ldcs(arow[i] + t0 + t) : mkcd(0, 0);
+          rs[i] += cabs1(av[g][i]);
+        }
       }
 #pragma unroll
       for (int j = 0; j < M; ++j) {
-        const double2 v = xs[j][t];
+        cd p[kResRows];
 #pragma unroll
-        for (int i = 0; i < kResRows; ++i) acc[i][j] = cmac(acc[i][j], av[i], mkcd(v.x, v.y));
+        for (int g = 0; g < kResG; ++g) {
+          const double2 v = xs[j][(q0 + g) * 32 + lane];
+#pragma unroll
+          for (int i = 0; i < kResRows; ++i)
+            p[i] = g == 0 ? av[g][i] * mkcd(v.x, v.y) : cmac_nested(p[i], av[g][i], mkcd(v.x, v.y));
+        }
+#pragma unroll
+        for (int i = 0; i < kResRows; ++i) acc[i][j] = acc[i][j] + p[i];
       }
     }
   }
