@@ -483,7 +483,7 @@ int refresh_jk_cache(pss_sheet *sh, double psi1, double psi2, double ulocal, Wor
   if (!jk_key_stale(sh, psi1, psi2, ulocal)) return 0;
   cudaStream_t st = w.st;
   if (sh->cache.ensure(sh->nufp)) return -3;
-  if (w.jkws.ensure(pss_jktab_bytes(sh->G, ulocal, sh->s1, sh->s2, 1))) return -3;
+  (void)w.jkws.ensure(pss_jktab_bytes(sh->G, ulocal, sh->s1, sh->s2, 1));  // refused: the direct form runs
   DevBuf nc;
   if (nc.ensure(sizeof(int))) return -3;
   PSS_CUDA_TRY(cudaMemsetAsync(nc.p, 0, sizeof(int), st));
@@ -994,7 +994,7 @@ int sweep_impl(pss_ctx *c, std::vector<Problem> &PR, int precision, const AdjSpe
     }
     for (int k = 0; k < nwk; ++k) {
       if (int rc = ensure_worker_dims(c->w[k], mufp, mn, mnm, precision, ojk, mB)) return rc;
-      if (c->w[k].jkws.ensure(mtab)) return -3;
+      (void)c->w[k].jkws.ensure(mtab);  // refused (no memory left): the direct form runs
     }
   }
   // adjoint-stage buffers of every worker: PT, Lam, scratch W (a batch each), R_k and the
