@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 CHILD = """
-import sys
+import ctypes, sys
 sys.path.insert(0, "tests")
 import conftest
 import numpy as np, torch
@@ -35,19 +35,21 @@ sheet = strip()
 rwg = setup_rwg(sheet)
 engine.face_integrals(sheet, rwg, 10 * ul, 0.4, 0.2)  # holds the sheet and its integrals, no tables
 engine.release_memory()
+cu = ctypes.CDLL("libcuda.so.1")  # PyTorch's allocator rounds small requests up to 20 MB
+free = lambda: torch.cuda.mem_get_info(0)[0]
 fill = []
 for unit in (1 << 30, 1 << 26, 1 << 22):
-    while torch.cuda.mem_get_info(0)[0] > unit + (4 << 20):
-        fill.append(torch.empty((torch.cuda.mem_get_info(0)[0] - (4 << 20)) // unit * unit, dtype=torch.uint8,
-                                device="cuda:0"))
-print("free MB", torch.cuda.mem_get_info(0)[0] / 1e6)
+    while free() > unit + (4 << 20):
+        p = ctypes.c_uint64()
+        assert cu.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t((free() - (4 << 20)) // unit * unit)) == 0
+        fill.append(p)
 before = engine.lib().pss_kernel_launches()
 got = engine.face_integrals(sheet, rwg, ul, 0.4, 0.2)
 assert engine.lib().pss_kernel_launches() - before == 1
 for k in ("J", "Jxi", "Jeta", "K", "Kxi", "Keta"):
     assert np.max(np.abs(got[k] - want[k])) <= 1e-13 * np.max(np.abs(want[k])), k
-del fill
-torch.cuda.empty_cache()
+for p in fill:
+    assert cu.cuMemFree_v2(p) == 0
 before = engine.lib().pss_kernel_launches()
 again = engine.face_integrals(sheet, rwg, ul, 0.4, 0.2)
 assert engine.lib().pss_kernel_launches() - before == 4
