@@ -71,7 +71,20 @@ print("done")
 """
 
 
-@pytest.mark.parametrize("child", [GIVEN_BACK, MAKES_WAY], ids=["given_back", "makes_way"])
+BOUNDED = HEAD + """
+engine.release_memory()
+before = free()
+big = rectstrip(Lx=8, Ly=8, Px=10, Py=10, Nx=56, Ny=56, units=mm)  # 6272 faces: 4.5 GB to class
+for _ in range(3):
+    unique_face_pairs(big, where="device")
+    kept = before - free()
+    print("kept", kept / MIB)
+    assert 1024 * MIB < kept <= 2048 * MIB + 64 * MIB  # the excess goes, the rest stays
+print("done")
+"""
+
+
+@pytest.mark.parametrize("child", [GIVEN_BACK, MAKES_WAY, BOUNDED], ids=["given_back", "makes_way", "bounded"])
 def test_pool(child):
     r = subprocess.run([sys.executable, "-c", child], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
