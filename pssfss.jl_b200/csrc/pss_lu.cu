@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kPanelRows / RPT) k_panel(Mat<F32> M0, LuBatch
   bool act[RPT];
 #pragma unroll
   for (int k = 0; k < RPT; ++k) act[k] = tid + k * T < nloc;
-  __syncthreads();
+  cluster.sync();  // every CTA of the cluster runs before the first push into its shared memory
 
   for (int j = 0; j < w; ++j) {
     const int par = j & 1;
