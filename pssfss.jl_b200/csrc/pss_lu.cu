@@ -13,9 +13,9 @@
 //     interchange list, and the rows are copied to their final positions.
 //   * k_laswp applies that list to all other columns in one launch.
 //   * k_rowsolve: the block-row solve L11^{-1} X of an outer block (or of one panel inside it).
-//   * the Schur complement A22 -= L21 U12: k_gemm64 (FP64 matrix pipe), and in FP32 mode
-//     k_gemm32 for the skinny updates inside an outer block and the tcgen05 3xTF32 kernel
-//     (pss_gemm_tc.cu) for the trailing update of each outer block.
+//   * the Schur complement A22 -= L21 U12: k_gemm64 (FP64 matrix pipe), and in FP32 mode the
+//     tcgen05 3xTF32 kernel (pss_gemm_tc.cu) for every update of at least 64 x 32, inside an
+//     outer block too, and k_gemm32 for the few smaller ones at the matrix's end.
 // In FP32 mode the matrix is two float planes (real, imaginary).
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kSwpThreads) k_laswp(Mat<F32> M0, long long ms
 // broadcast by a shuffle); then the remaining rows take their rank-32 update from shared memory.
 // One launch per outer block replaces four 32-row solves and three updates of the rows between
 // them (with their operand splits): about 10 ms of launches, each too short to fill the chip, per
-// batch of 12 at N = 3976, now 3.4 ms (143 us at the first outer block).
+// batch of 12 at N = 3976, now 3.5 ms (144 us at the first outer block).
 template <bool F32>
 struct RowSolve {
   static constexpr int NB = F32 ? 128 : 64, COLS = F32 ? 64 : 32, S = 32, LP = S + 1;

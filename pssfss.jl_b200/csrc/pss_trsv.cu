@@ -185,8 +185,10 @@ __device__ __forceinline__ C czero() { return C{0, 0}; }
 //   * the predecessor's tile waits in registers, the diagonal inverse in shared memory.
 // After the flag: x of the predecessor to shared memory, one 64 x 64 product from registers, one
 // with the inverse, the result and the flag.  The release of the flag after the block barrier
-// orders the block's stores; no further fence is needed.  660 -> 300 us per triangle of a batch of factors
-// (N = 3976, four right-hand sides, FP32).  Chains of more right-hand sides run side by side.
+// orders the block's stores; no further fence is needed.  660 -> 390 us per triangle of 12 factors
+// (N = 3976, four right-hand sides, FP32, cold caches).  Chains of more right-hand sides run side
+// by side.  A row's products, the predecessor's among them, are summed on their own and
+// subtracted from its right-hand side once.
 template <bool F32>
 struct TrsvT {
   static constexpr int T = F32 ? 256 : 512;    // threads
